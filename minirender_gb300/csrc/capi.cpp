@@ -587,35 +587,40 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     total += (uint64_t)c->meshes[h].d.n_tri;
   }
   if (total >= ((uint64_t)1 << 31)) return fail(c, MR_E_INVALID, "more than 2^31-1 triangles in one frame");
-  size_t nrs = (size_t)std::max(n, 1);
-  if (c->h_rs_cap < nrs) {
+  // Several renderables go through the staged table; a frame's only one rides
+  // in the kernels' parameters, so its launch waits for no staging block.
+  DevRenderable one;
+  DevRenderable* table = &one;
+  uint32_t one_bases[3 * 2];
+  uint32_t* h_tbase = one_bases;
+  if (n != 1) {
+    const size_t nrs = (size_t)std::max(n, 1);
     CK(cudaEventSynchronize(c->staged), "staging wait");
-    if (c->h_stage) cudaFreeHost(c->h_stage);
-    c->h_stage = nullptr;
-    c->h_rs = nullptr;
-    c->h_tri_base = nullptr;
-    c->h_P = nullptr;
-    c->h_rs_cap = 0;
-    c->off_bases = align256(sizeof(DevRenderable) * nrs);
-    c->off_P = c->off_bases + align256(sizeof(uint32_t) * 3 * (nrs + 1));
-    c->stage_bytes = (c->off_P + sizeof(float) * 16 + 15) & ~(size_t)15;
-    CK(cudaMallocHost(&c->h_stage, c->stage_bytes), "pinned staging");
-    CK(cudaHostGetDevicePointer((void**)&c->d_stage_src, c->h_stage, 0), "mapped staging");
-    CK(c->stage.ensure(c->stage_bytes), "staging buffer");
-    c->h_rs = (DevRenderable*)c->h_stage;
-    c->h_tri_base = (uint32_t*)(c->h_stage + c->off_bases);
-    c->h_P = (float*)(c->h_stage + c->off_P);
-    c->h_rs_cap = nrs;
-  } else {
-    CK(cudaEventSynchronize(c->staged), "staging wait");
+    if (c->h_rs_cap < nrs) {
+      if (c->h_stage) cudaFreeHost(c->h_stage);
+      c->h_stage = nullptr;
+      c->h_rs = nullptr;
+      c->h_tri_base = nullptr;
+      c->h_rs_cap = 0;
+      c->off_bases = align256(sizeof(DevRenderable) * nrs);
+      c->stage_bytes = (c->off_bases + sizeof(uint32_t) * 3 * (nrs + 1) + 15) & ~(size_t)15;
+      CK(cudaMallocHost(&c->h_stage, c->stage_bytes), "pinned staging");
+      CK(cudaHostGetDevicePointer((void**)&c->d_stage_src, c->h_stage, 0), "mapped staging");
+      CK(c->stage.ensure(c->stage_bytes), "staging buffer");
+      c->h_rs = (DevRenderable*)c->h_stage;
+      c->h_tri_base = (uint32_t*)(c->h_stage + c->off_bases);
+      c->h_rs_cap = nrs;
+    }
+    table = c->h_rs;
+    h_tbase = c->h_tri_base;
   }
   uint32_t base = 0;
   uint64_t vbase = 0, nbase = 0;
-  uint32_t* h_vbase = c->h_tri_base + (n + 1);
-  uint32_t* h_nbase = c->h_tri_base + 2 * (n + 1);
+  uint32_t* h_vbase = h_tbase + (n + 1);
+  uint32_t* h_nbase = h_tbase + 2 * (n + 1);
   for (int32_t i = 0; i < n; i++) {
     const MeshRec& m = c->meshes[rs[i].mesh];
-    DevRenderable& R = c->h_rs[i];
+    DevRenderable& R = table[i];
     float mv[16], inv[16], nm[16];
     if (rs[i].flags & MR_RS_MODELVIEW) memcpy(mv, rs[i].transform, sizeof(mv));
     else mat4_mul(f->view, rs[i].transform, mv);
@@ -627,7 +632,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     R.no_clip = (rs[i].flags & MR_RS_NO_CLIP) ? 1 : 0;
     const bool texturing = switches(rs[i].flags, *f, R);
     R.tri_base = base;
-    c->h_tri_base[i] = base;
+    h_tbase[i] = base;
     base += (uint32_t)m.d.n_tri;
     R.vert_base = (uint32_t)vbase;
     R.nrm_base = (uint32_t)nbase;
@@ -655,7 +660,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
       else R.texf = (const float*)T.mem;
     }
   }
-  c->h_tri_base[n] = base;
+  h_tbase[n] = base;
   h_vbase[n] = (uint32_t)vbase;
   h_nbase[n] = (uint32_t)nbase;
 
@@ -669,7 +674,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   if (f->save_normals) CK(c->normals.ensure(3 * npx), "normals buffer");
   CK(c->recs.ensure((size_t)2 * total), "record buffer");
   CK(c->spill.ensure((size_t)2 * total), "spill buffer");
-  if (c->items.cap < ((size_t)1 << 18)) CK(c->items.ensure((size_t)1 << 18), "row-block buffer");
+  if (c->items.cap < ((size_t)1 << 18)) CK(c->items.ensure((size_t)1 << 18), "block list");
   // The per-vertex pass pays off when vertices are shared (each one used by
   // two or more triangle corners on average); for triangle soups every
   // corner is its own vertex and the kernels transform corners themselves.
@@ -679,14 +684,20 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     CK(c->vb.ensure(vbase), "vertex buffer");
     CK(c->vn.ensure(nbase), "normal buffer");
   }
-  memcpy(c->h_P, f->projection, sizeof(float) * 16);
-
   FrameParams& F = c->last;
   memset(&F, 0, sizeof(F));
-  // the clear kernel fetches the staging block from mapped pinned memory
-  F.stage_src = (const uint4*)c->d_stage_src;
-  F.stage_dst = (uint4*)c->stage.p;
-  F.stage_n16 = (uint32_t)(c->stage_bytes / 16);
+  if (n == 1) {
+    F.one = one;
+  } else {  // the clear kernel fetches the staging block from mapped pinned memory
+    F.stage_src = (const uint4*)c->d_stage_src;
+    F.stage_dst = (uint4*)c->stage.p;
+    F.stage_n16 = (uint32_t)(c->stage_bytes / 16);
+    const uint32_t* d_bases = (const uint32_t*)(c->stage.p + c->off_bases);
+    F.g.rs = (const DevRenderable*)c->stage.p;
+    F.g.tri_base = d_bases;
+    F.g.vert_base = d_bases + (n + 1);
+    F.g.nrm_base = d_bases + 2 * (n + 1);
+  }
   F.v.W = W;
   F.v.H = H;
   F.v.w = (float)W;
@@ -703,11 +714,6 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   F.g.n_renderables = n;
   F.g.n_tris = (uint32_t)total;
   F.small_max = c->small_max;
-  const uint32_t* d_bases = (const uint32_t*)(c->stage.p + c->off_bases);
-  F.g.rs = (const DevRenderable*)c->stage.p;
-  F.g.tri_base = d_bases;
-  F.g.vert_base = d_bases + (n + 1);
-  F.g.nrm_base = d_bases + 2 * (n + 1);
   F.g.n_verts = (uint32_t)vbase;
   F.g.n_nrms = (uint32_t)nbase;
   F.g.va = vertex_pass ? c->va.p : nullptr;  // null: kernels transform per corner
@@ -745,6 +751,10 @@ static int queue_reads(mr_ctx* c, const ReadTargets& r) {
   return MR_OK;
 }
 
+// Blocks the large-triangle list grows to at most (512 MB); a frame with more
+// rasterises the rest through the spill list.
+constexpr size_t kMaxItems = (size_t)1 << 26;
+
 // Waits for the last frame and reads its counters.  An outstanding
 // mr_read_async completes here: its counter copy was queued behind the frame
 // and its output copies before the read_done event (work queued on the
@@ -763,8 +773,8 @@ static int settle(mr_ctx* c) {
   c->pending = false;
   const Counters& k = *c->h_cnt;
   if (k.item_count > c->last.item_cap) {
-    size_t want = (size_t)k.item_count + k.item_count / 4 + 1024;
-    CK(c->items.ensure(want), "row-block buffer");
+    const size_t want = std::min<size_t>((size_t)(k.item_count + k.item_count / 4 + 1024), kMaxItems);
+    CK(c->items.ensure(want), "block list");
   }
   return (k.error_flags & 1u) ? fail(c, MR_E_BAD_INDEX, "a mesh index was out of range; those triangles were skipped") : MR_OK;
 }
@@ -837,6 +847,15 @@ MR_API int mr_get_outputs(mr_ctx* c, mr_outputs* o) {
   return MR_OK;
 }
 
+// Triangle statistics over the counters' slots (small: small_direct too).
+static void sum_stats(const Counters& k, mr_stats* s, bool small) {
+  for (const StatSlot& t : k.stat) {
+    s->clipped += (int64_t)t.clipped;
+    s->rasterised += (int64_t)(t.drawn >> 32);
+    if (small) s->small_direct += (int64_t)(t.drawn & 0xFFFFFFFFu);
+  }
+}
+
 MR_API int mr_get_stats(mr_ctx* c, mr_stats* s) {
   if (!c || !s) return MR_E_INVALID;
   std::lock_guard<std::recursive_mutex> g(c->mu);
@@ -846,9 +865,7 @@ MR_API int mr_get_stats(mr_ctx* c, mr_stats* s) {
   memset(s, 0, sizeof(*s));
   const Counters& k = *c->h_cnt;
   s->triangles = c->last.g.n_tris;
-  s->clipped = (int64_t)k.clipped;
-  s->rasterised = (int64_t)k.rasterised;
-  s->small_direct = (int64_t)k.small_direct;
+  sum_stats(k, s, true);
   s->binned = (int64_t)k.rec_count;
   s->bin_entries = (int64_t)k.item_count;
   s->error_flags = k.error_flags;
@@ -868,8 +885,9 @@ MR_API int mr_read_range_image(mr_ctx* c, float* xyz) {
   if (!c->last.depth) return fail(c, MR_E_INVALID, "depth was not requested for this frame");
   size_t npx = (size_t)c->last.v.W * c->last.v.H;
   CK(c->range.ensure(3 * npx), "range buffer");
-  CK(launch_range(c->last.v.W, c->last.v.H, (const float*)(c->stage.p + c->off_P), c->last.depth, c->range.p,
-                  c->stream), "range launch");
+  Mat4 P;
+  memcpy(P.m, c->last.v.P, sizeof(P.m));
+  CK(launch_range(c->last.v.W, c->last.v.H, P, c->last.depth, c->range.p, c->stream), "range launch");
   CK(cudaMemcpyAsync(xyz, c->range.p, 12 * npx, cudaMemcpyDeviceToHost, c->stream), "range read");
   CK(cudaStreamSynchronize(c->stream), "range wait");
   return rc;
@@ -1306,8 +1324,7 @@ MR_API int mr_get_batch_stats(mr_ctx* c, mr_stats* s) {
   memset(s, 0, sizeof(*s));
   const Counters& k = *c->b.h_cnt;
   s->triangles = c->b.P.g.n_tris;
-  s->clipped = (int64_t)k.clipped;
-  s->rasterised = (int64_t)k.rasterised;
+  sum_stats(k, s, false);
   s->binned = (int64_t)k.rec_count;
   s->bin_entries = (int64_t)k.bin_needed;
   s->error_flags = k.error_flags;

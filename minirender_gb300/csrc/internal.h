@@ -16,8 +16,7 @@
 namespace mrg {
 cudaError_t launch_validate(const DevMesh& M, uint32_t* bad, cudaStream_t st);
 cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev, cudaEvent_t staged = nullptr);
-cudaError_t launch_range(int W, int H, const float* dP, const float* depth, float* xyz,
-                         cudaStream_t st);
+cudaError_t launch_range(int W, int H, const Mat4& P, const float* depth, float* xyz, cudaStream_t st);
 cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* block_sums, cudaStream_t st,
                          cudaEvent_t* ev);
 int batch_grid(int tile_w, int tile_h, int chunk, int threads, bool pre);
@@ -150,15 +149,14 @@ struct mr_ctx {
   DevBuf<BigRec> recs;
   DevBuf<LargeItem> items;     // large-triangle row blocks of the last frame
   DevBuf<LargeItem> spill;     // records whose rows did not fit items (one entry each)
-  // Per-frame staging, one block on both sides (one copy per frame):
-  // renderables (cap) | tri, vertex and normal base tables 3 x (cap+1) | projection
+  // Per-frame staging of frames of several renderables, one block on both
+  // sides: renderables (cap) | tri, vertex and normal base tables 3 x (cap+1)
   DevBuf<unsigned char> stage;
   unsigned char* h_stage = nullptr;
   unsigned char* d_stage_src = nullptr;  // h_stage as the device sees it (mapped)
-  size_t h_rs_cap = 0, stage_bytes = 0, off_bases = 0, off_P = 0;
+  size_t h_rs_cap = 0, stage_bytes = 0, off_bases = 0;
   DevRenderable* h_rs = nullptr;
   uint32_t* h_tri_base = nullptr;
-  float* h_P = nullptr;
   DevBuf<float4> va, vn;        // per-frame vertex-pass outputs
   DevBuf<float2> vb;
   Counters* d_cnt = nullptr;

@@ -1,19 +1,21 @@
 // GB300 (sm_103a) kernels of the rasterisation path.
 //
 // One frame per call (launch_frame):
-//   k_clear        vis[] = VIS_EMPTY                 (Renderer::clear, src/Renderer.cpp:113-119)
-//   k_vertex       per-vertex view transform + projection to pixel space and
+//   k_begin        vis[] = VIS_EMPTY                 (Renderer::clear, src/Renderer.cpp:113-119)
+//                  and, for a frame of one renderable, the vertex pass
+//   k_vertex       (frames of several renderables, batches) per-vertex view
+//                  transform + projection to pixel space and
 //                  per-normal transform, once per frame (the PREMULT loops,
 //                  src/Renderer.cpp:344-348, plus htransform :13-20 and the
 //                  pixel mapping :193-197, which depend on the vertex only)
 //   k_setup        triangle assembly + near clip + triangle setup + cull;
 //                  small triangles rasterised by the warp that set them up,
 //                  one (triangle, row) per lane; large ones appended to a
-//                  warp-compacted record list with their row blocks
+//                  warp-compacted record list with their blocks
 //                                                   (src/Renderer.cpp:121-269, 351-379)
-//   k_raster_large one warp per row block of a large sub-triangle (the setup
-//                  kernel lists the blocks), each row walked across the whole
-//                  bounding box with 64-bit atomicMin (src/Renderer.cpp:238-269)
+//   k_raster_large one warp per block (32 rows by a column segment) of a large
+//                  sub-triangle, one row per lane, 64-bit atomicMin
+//                                                   (src/Renderer.cpp:238-269)
 //   k_resolve      deferred pass: re-derives the winning sub-triangle's
 //                  barycentrics exactly, shades once per visible pixel and
 //                  writes RGB8/depth/ids            (src/Renderer.cpp:271-305, src/io.cpp:358-362)
@@ -38,7 +40,8 @@
 // rasteriser and the resolve replay that chain.  Values the vertex pass stores
 // are the same expressions the reference evaluates per triangle corner.
 // Kernels templated on PRE read the vertex-pass buffers; without them
-// (allocation-free entry point) vertices are transformed per triangle.
+// (triangle soups, allocation-free entry point) vertices are transformed per
+// triangle.  ONE: the frame's only renderable is read from the parameters.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -113,39 +116,13 @@ __device__ __forceinline__ Vtx clip_vtx(float z, const Vtx& a, const Vtx& b) {
   return v;
 }
 
-// clipTriangle, src/Renderer.cpp:131-161, for a triangle with at least one
-// corner in front of the near plane.  Returns 0, 1 or 2 sub-triangles.
+// clipTriangle, src/Renderer.cpp:131-161, for a triangle with a corner behind
+// the near plane: the number of its sub-triangles (0, 1 or 2), and sub-triangle
+// `sub` (when there is one of that number) in place of v.
 template <bool ATTR>
-__device__ __forceinline__ int clip_tri(float zn, Vtx (&v)[3], Vtx (&sub)[2][3]) {
+__device__ __forceinline__ int clip_pick(float zn, Vtx (&v)[3], int sub) {
   if (v[0].pos.z > zn && v[1].pos.z > zn && v[2].pos.z > zn) return 0;
   // rotate until v[0] has the largest z (at most two turns for any input)
-  for (int it = 0; it < 3 && (v[0].pos.z < v[1].pos.z || v[0].pos.z < v[2].pos.z); it++) {
-    Vtx t0 = v[0]; v[0] = v[2]; v[2] = v[1]; v[1] = t0;
-  }
-  if (v[1].pos.z > zn) {
-    sub[0][0] = clip_vtx<ATTR>(zn, v[0], v[2]);
-    sub[0][1] = clip_vtx<ATTR>(zn, v[1], v[2]);
-    sub[0][2] = v[2];
-    return 1;
-  }
-  if (v[2].pos.z > zn) {
-    sub[0][0] = clip_vtx<ATTR>(zn, v[0], v[1]);
-    sub[0][1] = v[1];
-    sub[0][2] = clip_vtx<ATTR>(zn, v[1], v[2]);
-    return 1;
-  }
-  Vtx v01 = clip_vtx<ATTR>(zn, v[0], v[1]);
-  Vtx v02 = clip_vtx<ATTR>(zn, v[0], v[2]);
-  sub[0][0] = v01; sub[0][1] = v[1]; sub[0][2] = v[2];
-  sub[1][0] = v01; sub[1][1] = v[2]; sub[1][2] = v02;
-  return 2;
-}
-
-// Sub-triangle s (0 or 1) of clipTriangle's output for a triangle that
-// crosses the near plane and has that sub-triangle, computed in place in v:
-// the same operations as clip_tri, without materialising both halves.
-template <bool ATTR>
-__device__ __forceinline__ void clip_pick(float zn, Vtx (&v)[3], int s) {
   for (int it = 0; it < 3 && (v[0].pos.z < v[1].pos.z || v[0].pos.z < v[2].pos.z); it++) {
     Vtx t0 = v[0]; v[0] = v[2]; v[2] = v[1]; v[1] = t0;
   }
@@ -153,21 +130,22 @@ __device__ __forceinline__ void clip_pick(float zn, Vtx (&v)[3], int s) {
     const Vtx a = clip_vtx<ATTR>(zn, v[0], v[2]);
     v[1] = clip_vtx<ATTR>(zn, v[1], v[2]);
     v[0] = a;
-    return;
+    return 1;
   }
   if (v[2].pos.z > zn) {
     const Vtx a = clip_vtx<ATTR>(zn, v[0], v[1]);
     v[2] = clip_vtx<ATTR>(zn, v[1], v[2]);
     v[0] = a;
-    return;
+    return 1;
   }
   const Vtx v01 = clip_vtx<ATTR>(zn, v[0], v[1]);
-  if (s) {  // (v01, v2, v02)
+  if (sub) {  // (v01, v2, v02)
     const Vtx v02 = clip_vtx<ATTR>(zn, v[0], v[2]);
     v[1] = v[2];
     v[2] = v02;
   }
   v[0] = v01;
+  return 2;
 }
 
 // View-space corners of triangle t (paintMesh, src/Renderer.cpp:344-379).
@@ -326,6 +304,34 @@ __device__ __forceinline__ bool covered(float e1, float e2) {
   return !(e1 < 0 || e2 < 0 || 1 - e1 - e2 < 0);
 }
 
+// Two edge values advanced together: one packed IEEE add per column
+// (add.rn.f32x2 rounds each half as the scalar add does).
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// The edge values n columns on: n running sums, column by column.
+__device__ __forceinline__ unsigned long long advance2(unsigned long long e, unsigned long long d, int n) {
+#pragma unroll 1
+  for (; n >= 8; n -= 8) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) e = add2(e, d);
+  }
+  if (n & 4) e = add2(add2(add2(add2(e, d), d), d), d);
+  if (n & 2) e = add2(add2(e, d), d);
+  if (n & 1) e = add2(e, d);
+  return e;
+}
+
 // Walks columns xs..xe of row y (replaying the running sums from x0) and
 // calls emit(x, packed, e1, e2) for every fragment that would pass z < 1e11f
 // (e1, e2: the running edge values at column x).
@@ -334,39 +340,34 @@ __device__ __forceinline__ void walk_row(const Setup& S, bool persp, uint32_t id
                                          int xe, Emit emit) {
   float e1, e2;
   row_start(S, y, e1, e2);
-  const float d1 = S.n1.x, d2 = S.n2.x;
-  for (int x = S.x0; x < xs; x++) {
-    e1 += d1;
-    e2 += d2;
-  }
+  const unsigned long long d = pack2(S.n1.x, S.n2.x);
+  unsigned long long e = advance2(pack2(e1, e2), d, xs - S.x0);
   for (int x = xs; x <= xe; x++) {
+    unpack2(e, e1, e2);
     if (covered(e1, e2)) {
       float k0, k1, k2;
       float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
       if (z < 1e11f) emit(x, ((unsigned long long)depth_key(z) << 32) | id, e1, e2);
     }
-    e1 += d1;
-    e2 += d2;
+    e = add2(e, d);
   }
 }
 
-// Per-block statistics: warps add into shared counters, one global atomic per
-// counter and block (a single global address updated by every warp would
-// serialise in L2).  Every thread of the block must call block_flush.
-struct BlockCounters {
-  unsigned v[3];
-};
-__device__ __forceinline__ void block_count(BlockCounters& bc, int k, unsigned v) {
-  unsigned s = __reduce_add_sync(0xffffffffu, v);
-  if ((threadIdx.x & 31) == 0 && s) atomicAdd(&bc.v[k], s);
+// Column segments of a large sub-triangle's bounding box (see kLargeCols).
+__device__ __forceinline__ int large_seg_cols(int x0, int x1) {
+  return kLargeCols * ((x1 - x0) / (kLargeCols * kLargeSegs) + 1);
 }
-__device__ __forceinline__ void block_flush(BlockCounters& bc, unsigned long long* d0, unsigned long long* d1,
-                                            unsigned long long* d2) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (bc.v[0]) atomicAdd(d0, (unsigned long long)bc.v[0]);
-    if (bc.v[1] && d1) atomicAdd(d1, (unsigned long long)bc.v[1]);
-    if (bc.v[2]) atomicAdd(d2, (unsigned long long)bc.v[2]);
+__device__ __forceinline__ int large_segs(int x0, int x1) { return (x1 - x0) / large_seg_cols(x0, x1) + 1; }
+
+// Adds a warp's sub-triangles (small: rasterised by the setup kernel) and
+// cut triangles to its statistics slot.  Called by all lanes of the warp.
+__device__ __forceinline__ void count_triangles(Counters* c, bool small, bool big, bool cut) {
+  const unsigned s = __ballot_sync(0xffffffffu, small), l = __ballot_sync(0xffffffffu, big);
+  const unsigned k = __ballot_sync(0xffffffffu, cut);
+  if ((threadIdx.x & 31) == 0 && (s | l | k)) {
+    StatSlot& slot = c->stat[((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kStatSlots];
+    if (s | l) atomicAdd(&slot.drawn, ((unsigned long long)(__popc(s) + __popc(l)) << 32) | (unsigned)__popc(s));
+    if (k) atomicAdd(&slot.clipped, (unsigned long long)__popc(k));
   }
 }
 
@@ -389,73 +390,74 @@ __device__ __forceinline__ Setup rec_setup(const BigRec& B) {
   return S;
 }
 
-// Assembly, near clip and setup of global triangle g (paintMesh + the first
-// half of paintTriangle).  Fills up to two setups in draw order; kind[s] = 1
-// for a sub-triangle with pixels to test.  Returns false for a triangle whose
-// indices failed the upload check.
+// Assembly, near clip and setup of sub-triangle `sub` of triangle t (paintMesh
+// + the first half of paintTriangle).  True: it has pixels to test.  n_sub:
+// the triangle's sub-triangles (1 when the near plane does not cut it).  The
+// setup kernels take a triangle's second half in a round of its own, so only
+// one Setup is live (two cost the vertex-pass instance a third of its
+// registers; the round runs for warps with such a triangle only).
 template <bool PRE>
-__device__ __forceinline__ bool setup_triangle(const View& V, const Geo& G, const DevRenderable& R,
-                                               uint32_t g, Setup (&S)[2], int (&kind)[2],
-                                               unsigned& n_clipped) {
-  const int t = (int)(g - R.tri_base);
-  if ((R.mesh.bad[t >> 5] >> (t & 31)) & 1u) return false;
+__device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const DevRenderable& R, int t, int sub,
+                                          Setup& S, int& n_sub, bool& cut) {
   int ip[3];
 #pragma unroll
   for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
   // no_clip (paintTriangle(..., world=false)): never clipped, so the near
   // test compares against +inf
   const float zn = R.no_clip ? __int_as_float(0x7f800000) : V.znear;
+  V2 p[3];
+  float zt[3];
+  Vtx v[3];
   if (PRE) {
     float4 a[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) a[c] = G.va[R.vert_base + ip[c]];
-    if (!(a[0].w > zn || a[1].w > zn || a[2].w > zn)) {
-      V2 p[3] = {v2(a[0].x, a[0].y), v2(a[1].x, a[1].y), v2(a[2].x, a[2].y)};
-      float zt[3] = {a[0].z, a[1].z, a[2].z};
-      if (setup_from(V, p, zt, S[0])) kind[0] = 1;
-      return true;
+    for (int c = 0; c < 3; c++) {
+      a[c] = G.va[R.vert_base + ip[c]];
+      p[c] = v2(a[c].x, a[c].y);
+      zt[c] = a[c].z;
     }
-  }
-  Vtx v[3], sub[2][3];
-  corners<PRE, false>(G, R, t, ip, v);
-  int n;
-  if (!(v[0].pos.z > zn || v[1].pos.z > zn || v[2].pos.z > zn)) {
-    sub[0][0] = v[0]; sub[0][1] = v[1]; sub[0][2] = v[2];
-    n = 1;
+    cut = a[0].w > zn || a[1].w > zn || a[2].w > zn;
   } else {
-    n = clip_tri<false>(zn, v, sub);
-    n_clipped += n > 0;
+    corners<false, false>(G, R, t, ip, v);
+    cut = v[0].pos.z > zn || v[1].pos.z > zn || v[2].pos.z > zn;
   }
-  for (int s = 0; s < n; s++)
-    if (setup_view(V, sub[s], S[s])) kind[s] = 1;
-  return true;
+  n_sub = 1;
+  if (cut) {
+    if (PRE) corners<true, false>(G, R, t, ip, v);
+    n_sub = clip_pick<false>(zn, v, sub);
+    if (n_sub <= sub) return false;
+  }
+  if (!PRE || cut) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) project(V, v[c].pos, p[c].x, p[c].y, zt[c]);
+  }
+  return setup_from(V, p, zt, S);
 }
 
-// The sub-triangle `id` won by a pixel: its renderable, vertex indices and
+__device__ __forceinline__ long long box_pixels(const Setup& S) {
+  return (long long)(S.x1 - S.x0 + 1) * (S.y1 - S.y0 + 1);
+}
+
+// Whether triangle t's indices failed the upload check.
+__device__ __forceinline__ bool bad_triangle(const DevMesh& M, int t) { return (M.bad[t >> 5] >> (t & 31)) & 1u; }
+
+// The sub-triangle `id` (of R) won by a pixel: its vertex indices and
 // view-space corners with attributes (the clipped sub-triangle when the
 // triangle crosses the near plane), src/Renderer.cpp:334-379, 131-161.
-// Renderables of the pixel's frame are rs_lo..rs_hi-1.
-// s_tb, when given, holds tri_base[rs_lo .. rs_hi) in shared memory.
 template <bool PRE>
-__device__ __forceinline__ const DevRenderable* winner_tri(const View& V, const Geo& G, int rs_lo, int rs_hi,
-                                                         uint32_t id, int (&ip)[3], Vtx (&vc)[3],
-                                                         bool& clipped, const uint32_t* s_tb = nullptr) {
-  const uint32_t g = id >> 1;
-  const int s = (int)(id & 1u);
-  const int k = s_tb ? rs_lo + find_base(s_tb, 0, rs_hi - rs_lo, g) : find_base(G.tri_base, rs_lo, rs_hi, g);
-  const DevRenderable* R = &G.rs[k];
-  const int t = (int)(g - R->tri_base);
-  if (!PRE && R->mesh.rec) {
-    corners_rec(*R, t, vc);  // (ip is not used without the vertex pass)
+__device__ __forceinline__ void winner_tri(const View& V, const Geo& G, const DevRenderable& R, uint32_t id,
+                                           int (&ip)[3], Vtx (&vc)[3], bool& clipped) {
+  const int t = (int)((id >> 1) - R.tri_base);
+  if (!PRE && R.mesh.rec) {
+    corners_rec(R, t, vc);  // (ip is not used without the vertex pass)
   } else {
 #pragma unroll
-    for (int c = 0; c < 3; c++) ip[c] = __ldg(R->mesh.idx + 3 * t + c);
-    corners<PRE, true>(G, *R, t, ip, vc);
+    for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
+    corners<PRE, true>(G, R, t, ip, vc);
   }
-  const float zn = R->no_clip ? __int_as_float(0x7f800000) : V.znear;
+  const float zn = R.no_clip ? __int_as_float(0x7f800000) : V.znear;
   clipped = vc[0].pos.z > zn || vc[1].pos.z > zn || vc[2].pos.z > zn;
-  if (clipped) clip_pick<true>(zn, vc, s);  // sub-triangle s exists: it won this pixel
-  return R;
+  if (clipped) clip_pick<true>(zn, vc, (int)(id & 1u));  // that sub-triangle exists: it won this pixel
 }
 
 // Texture and Blinn-Phong lighting of a fragment with perspective-corrected
@@ -517,59 +519,62 @@ __device__ __forceinline__ void winner_setup(const View& V, const Geo& G, const 
 // from the bounding-box edge (src/Renderer.cpp:240-243).
 __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, float& e2) {
   row_start(S, y, e1, e2);
-  for (int c = S.x0; c < x; c++) {
-    e1 += S.n1.x;
-    e2 += S.n2.x;
-  }
-}
-
-// Shading of the pixel (x, y) whose visibility word is vw, src/Renderer.cpp:
-// 247-305 (FAST_LIGHT): re-derives the winner's setup, replays its edge
-// functions to column x, and evaluates texture and Blinn-Phong lighting.
-// Renderables of the pixel's frame are rs_lo..rs_hi-1.
-template <bool PRE>
-__device__ __forceinline__ void resolve_pixel(const View& V, const Geo& G, int rs_lo, int rs_hi,
-                                              unsigned long long vw, int x, int y, const float* s_dec,
-                                              V3& value, float& depth, uint32_t& id, V3& normal_out) {
-  normal_out = v3(0, 0, 1);
-  if (vw == VIS_EMPTY) {
-    value = v3(V.bg[0], V.bg[1], V.bg[2]);
-    depth = 1e11f;
-    id = MR_NO_TRIANGLE;
-    return;
-  }
-  id = (uint32_t)vw;
-  int ip[3];
-  Vtx vc[3];
-  bool clipped;
-  const DevRenderable& R = *winner_tri<PRE>(V, G, rs_lo, rs_hi, id, ip, vc, clipped);
-  Setup S;
-  winner_setup<PRE>(V, G, R, ip, vc, clipped, S);
-  float e1, e2;
-  replay(S, x, y, e1, e2);
-  float k0, k1, k2;
-  depth = frag_depth(S, V.persp != 0, e1, e2, k0, k1, k2);
-  shade(V, R, vc, k0, k1, k2, s_dec, value, normal_out);
+  unpack2(advance2(pack2(e1, e2), pack2(S.n1.x, S.n2.x), x - S.x0), e1, e2);
 }
 
 // savePPM conversion, src/io.cpp:358-362.
 __device__ __forceinline__ uint8_t to_byte(float v) { return (uint8_t)(int)clampr(v * 255.0f, 0.0f, 255.0f); }
 
 // ------------------------------------------------------------------ kernels
-// vis[0..n) = VIS_EMPTY; also zeroes z[0..nz) (a frame's counters and tile
-// tables, so they need no separate memset before the frame).
-// With src, also copies n16 16-byte units from src (mapped pinned host
-// memory: the frame's staging block) to dst, so a frame never queues behind
-// other streams' transfers on the copy engine.
-__global__ void k_clear(unsigned long long* vis, size_t n, uint32_t* z0, uint32_t nz0, uint32_t* z1, uint32_t nz1,
-                        const uint4* src, uint4* dst, uint32_t n16) {
+// Vertex i of R, at g in the frame's vertex buffers.
+__device__ __forceinline__ void vertex(const Geo& G, const View& V, const DevRenderable& R, uint32_t g, int i) {
+  const V3 v = affine(R.mv, ld3(R.mesh.pos, i));
+  float px, py, zt;
+  project(V, v, px, py, zt);
+  G.va[g] = make_float4(px, py, zt, v.z);
+  G.vb[g] = make_float2(v.x, v.y);
+}
+// Normal i of R, at g in the frame's normal buffer.
+__device__ __forceinline__ void normal(const Geo& G, const DevRenderable& R, uint32_t g, int i) {
+  const V3 n = affine(R.nm, ld3(R.mesh.nrm, i));
+  G.vn[g] = make_float4(n.x, n.y, n.z, 0.f);
+}
+
+// The first kernel of a frame: vis[0..n) = VIS_EMPTY (Renderer::clear), the
+// counters zeroed, and one of
+//   - the staging block of a frame of several renderables copied from mapped
+//     pinned host memory, so a frame never queues behind other streams'
+//     transfers on the copy engine;
+//   - VERT: the vertex pass of a frame of one renderable, which comes in the
+//     kernel's parameters (one launch less, and the stores of the clear fill
+//     the vertex pass's load latency).
+__device__ __forceinline__ void clear_words(unsigned long long* vis, size_t n, size_t i, size_t stride) {
+  // two words per store (vis is 16-byte aligned)
+  ulonglong2* v2 = reinterpret_cast<ulonglong2*>(vis);
+  for (size_t k = i; k < n / 2; k += stride) v2[k] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
+  if (i == 0 && (n & 1)) vis[n - 1] = VIS_EMPTY;
+}
+template <bool VERT>
+__global__ void __launch_bounds__(256) k_begin(FrameParams F) {
   pdl_trigger();
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t k = i; k < n16; k += stride) dst[k] = src[k];
-  for (size_t k = i; k < nz0; k += stride) z0[k] = 0;
-  for (size_t k = i; k < nz1; k += stride) z1[k] = 0;
-  for (; i < n; i += stride) vis[i] = VIS_EMPTY;
+  if (!VERT)
+    for (size_t k = i; k < F.stage_n16; k += stride) F.stage_dst[k] = F.stage_src[k];
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(F.counters);
+  for (size_t k = i; k < sizeof(Counters) / 4; k += stride) cnt[k] = 0;
+  clear_words(F.vis, (size_t)F.v.W * F.v.H, i, stride);
+  if (VERT) {
+    for (size_t g = i; g < (size_t)F.g.n_verts + F.g.n_nrms; g += stride) {
+      if (g < F.g.n_verts) vertex(F.g, F.v, F.one, (uint32_t)g, (int)g);
+      else normal(F.g, F.one, (uint32_t)(g - F.g.n_verts), (int)(g - F.g.n_verts));
+    }
+  }
+}
+
+// vis[0..n) = VIS_EMPTY (batches: every scene's words).
+__global__ void __launch_bounds__(256) k_clear(unsigned long long* vis, size_t n) {
+  clear_words(vis, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
 // Index check of a mesh upload (one bit per triangle), and for meshes with
@@ -630,25 +635,22 @@ __global__ void k_validate(DevMesh M, uint32_t* bad, float4* rec) {
   }
 }
 
-// Vertex pass: threads [0, n_verts) transform and project positions,
-// threads [n_verts, n_verts + n_nrms) transform normals.  The view of a
-// vertex is scenes[R.scene].v for batches, V otherwise.
+// Vertex pass of several renderables: threads [0, n_verts) transform and
+// project positions, threads [n_verts, n_verts + n_nrms) transform normals.
+// BATCH: the view of a vertex is scenes[R.scene].v, else V.
+template <bool BATCH>
 __global__ void __launch_bounds__(256) k_vertex(Geo G, View V, const SceneRec* scenes) {
   pdl_wait();
   pdl_trigger();
-  uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g < G.n_verts) {
     const DevRenderable& R = G.rs[find_base(G.vert_base, 0, G.n_renderables, g)];
-    V3 v = affine(R.mv, ld3(R.mesh.pos, (int)(g - R.vert_base)));
-    float px, py, zt;
-    project(scenes ? scenes[R.scene].v : V, v, px, py, zt);
-    G.va[g] = make_float4(px, py, zt, v.z);
-    G.vb[g] = make_float2(v.x, v.y);
+    if constexpr (BATCH) vertex(G, scenes[R.scene].v, R, g, (int)(g - R.vert_base));
+    else vertex(G, V, R, g, (int)(g - R.vert_base));
   } else if (g - G.n_verts < G.n_nrms) {
-    uint32_t gn = g - G.n_verts;
+    const uint32_t gn = g - G.n_verts;
     const DevRenderable& R = G.rs[find_base(G.nrm_base, 0, G.n_renderables, gn)];
-    V3 n = affine(R.nm, ld3(R.mesh.nrm, (int)(gn - R.nrm_base)));
-    G.vn[gn] = make_float4(n.x, n.y, n.z, 0.f);
+    normal(G, R, gn, (int)(gn - R.nrm_base));
   }
 }
 
@@ -706,8 +708,13 @@ __device__ __forceinline__ Setup rec_get(const Rec& q) {
 }
 constexpr int kStageRecs = 32;  // records staged per warp and round
 
-constexpr int kSetupThreads = 256;
-constexpr int kSetupWarps = kSetupThreads / 32;
+// Threads per block of the setup kernels.  Their warps share nothing in a
+// frame (statistics go to slots, staging is per warp), and a block keeps its
+// place until its slowest warp is done, so frames take small blocks: 1080p
+// mesh setup 48.8 us with 256 threads, 46.6 with 128, 44.6 with 64; 10M-
+// triangle soup 378, 368, 366 us.  Batches reserve records per block, one
+// global atomic each, and take 128 (256 scenes: 428, 417, 420 us).
+constexpr int kSetupThreads = 64, kSetupBatchThreads = 128;
 
 // Where small triangles' fragments go: the frame's visibility buffer...
 struct FrameTarget {
@@ -755,195 +762,195 @@ __device__ __forceinline__ void raster_tiny(const Setup& Q, bool persp, uint32_t
   }
 }
 
-// Raster of the warp's small sub-triangles (kind 1; ids[s] the id of
-// sub-triangle s), whose frame is `tag`, with 64-bit atomicMin into the
-// target (src/Renderer.cpp:
+// Raster of the warp's small sub-triangles (one per lane where `on`), whose
+// frame is `tag`, with 64-bit atomicMin into the target (src/Renderer.cpp:
 // 238-269).  When every one in the warp spans at most 4x4 pixels the lanes
 // rasterise their own (the loops are short and nearly uniform); otherwise
 // they are staged in shared memory and rasterised with one (triangle, row)
 // per lane so every lane has work.  Called by all lanes of the warp.
 template <class Target, class Rec>
-__device__ __forceinline__ void raster_small(const Setup (&S)[2], const int (&kind)[2], const uint32_t (&ids)[2],
-                                             uint32_t tag, const Target& T, Rec* s_rec, int* s_pre) {
+__device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t id, uint32_t tag, const Target& T,
+                                             Rec* s_rec, int* s_pre) {
   const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
-  int span = 0;
-#pragma unroll
-  for (int s = 0; s < 2; s++)
-    if (kind[s] == 1) span = max(span, max(S[s].x1 - S[s].x0, S[s].y1 - S[s].y0) + 1);
+  const unsigned m = __ballot_sync(0xffffffffu, on);
+  if (m == 0) return;
+  const int span = on ? max(S.x1 - S.x0, S.y1 - S.y0) + 1 : 0;
   if (__reduce_max_sync(0xffffffffu, (unsigned)span) <= 4u) {
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-      if (kind[s] == 1)
-        raster_tiny(S[s], T.perspective(tag), ids[s], [&](int y) { return T.row(tag, y); });
+    if (on) raster_tiny(S, T.perspective(tag), id, [&](int y) { return T.row(tag, y); });
     return;
   }
-  // one round per sub-triangle slot (at most 32 records; slot 1 holds the
-  // second half of near-clipped triangles only)
+  const int n = __popc(m);
+  if (on) rec_put(s_rec[__popc(m & lt)], S, id, tag);
+  __syncwarp();
+  const int c = (int)lane < n ? rec_rows(s_rec[lane]) : 0;
+  int inc = c;
 #pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const unsigned m = __ballot_sync(0xffffffffu, kind[s] == 1);
-    if (m == 0) continue;
-    const int n = __popc(m);
-    if (kind[s] == 1) rec_put(s_rec[__popc(m & lt)], S[s], ids[s], tag);
-    __syncwarp();
-    const int c = (int)lane < n ? rec_rows(s_rec[lane]) : 0;
-    int inc = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, inc, o);
-      if ((int)lane >= o) inc += u;
-    }
-    const int total = __shfl_sync(0xffffffffu, inc, 31);
-    s_pre[lane] = inc - c;
-    __syncwarp();
-    for (int b = 0; b < total; b += 32) {
-      const int k = b + (int)lane;
-      if (k < total) {
-        int lo = 0;  // the last record lo < n with s_pre[lo] <= k
-#pragma unroll
-        for (int step = 16; step; step >>= 1)
-          if (lo + step < n && s_pre[lo + step] <= k) lo += step;
-        const Rec& q = s_rec[lo];
-        const Setup U = rec_get(q);
-        const int y = U.y0 + (k - s_pre[lo]);
-        const uint32_t tg = q.tag;
-        unsigned long long* row = T.row(tg, y);
-        walk_row(U, T.perspective(tg), q.id, y, U.x0, U.x1,
-                 [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
-      }
-    }
-    __syncwarp();  // s_rec / s_pre free for the warp's next use
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if ((int)lane >= o) inc += u;
   }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+  s_pre[lane] = inc - c;
+  __syncwarp();
+  for (int b = 0; b < total; b += 32) {
+    const int k = b + (int)lane;
+    if (k < total) {
+      int lo = 0;  // the last record lo < n with s_pre[lo] <= k
+#pragma unroll
+      for (int step = 16; step; step >>= 1)
+        if (lo + step < n && s_pre[lo + step] <= k) lo += step;
+      const Rec& q = s_rec[lo];
+      const Setup U = rec_get(q);
+      const int y = U.y0 + (k - s_pre[lo]);
+      const uint32_t tg = q.tag;
+      unsigned long long* row = T.row(tg, y);
+      walk_row(U, T.perspective(tg), q.id, y, U.x0, U.x1,
+               [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
+    }
+  }
+  __syncwarp();  // s_rec / s_pre free for the warp's next use
 }
 
-// Blocks per SM the register budget of k_setup must allow.  With the vertex
-// pass the kernel waits on index -> vertex gathers and more resident warps
-// hide that: 6 blocks (40 registers, some spilled to L1) with the packed
-// staging records, which leave more L1 to the spills.  Without it (triangle
-// soups) it is bound by instruction issue, spilling costs more than the
-// extra warps hide, and the aligned records' vector copies are cheaper: 4
-// blocks (64 registers).  Measured on 1080p and 4K frames.
+// Appends the warp's large sub-triangles (one per lane where `big`) to the
+// record list, one atomic per warp, and their blocks to the block list.
+// False in a lane whose record found no place (a fixed record store).
+__device__ __forceinline__ bool append_large(const FrameParams& F, const Setup& S, bool big, uint32_t id) {
+  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  const unsigned m = __ballot_sync(0xffffffffu, big);
+  if (m == 0) return true;
+  unsigned base = 0;
+  if (lane == 0) base = atomicAdd(&F.counters->rec_count, (unsigned)__popc(m));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  unsigned n_items = 0;
+  const unsigned slot = base + __popc(m & lt);
+  const bool placed = slot < F.rec_cap;
+  if (big && placed) {
+    F.recs[slot] = to_rec(S, id);
+    n_items = (unsigned)(((S.y1 - S.y0) / kLargeRows + 1) * large_segs(S.x0, S.x1));
+  }
+  // the blocks: one range per warp, each lane's at its exclusive prefix,
+  // written by all lanes (a screen-sized triangle has hundreds)
+  unsigned inc = n_items;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (unsigned)o) inc += u;
+  }
+  const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+  unsigned long long ibase = 0;
+  if (lane == 0 && total) ibase = atomicAdd(&F.counters->item_count, (unsigned long long)total);
+  ibase = __shfl_sync(0xffffffffu, ibase, 0);
+  for (unsigned b = 0; b < total; b += 32) {
+    const unsigned i = b + lane;
+    unsigned own = 0;  // the lane whose record block i belongs to
+#pragma unroll
+    for (unsigned step = 16; step; step >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= i) own += step;
+    const unsigned k = i - __shfl_sync(0xffffffffu, inc - n_items, own);
+    if (i >= total) continue;
+    const LargeItem item{base + __popc(m & ((1u << own) - 1u)), k};
+    // blocks past the end of the list: the record's remaining ones go to the
+    // spill list (one entry per record, so it cannot overflow)
+    if (ibase + i < F.item_cap) F.items[ibase + i] = item;
+    else if (k == 0 || ibase + i == F.item_cap) F.spill[atomicAdd(&F.counters->spill_count, 1u)] = item;
+  }
+  return placed || !big;
+}
+
+// The renderable of global triangle g.  ONE: the frame's only renderable,
+// which the kernels read from their parameters (constant bank) instead of
+// through the staged table: no search, and no pointer to fetch before the
+// first index can be read.
+template <bool ONE>
+__device__ __forceinline__ const DevRenderable& renderable(const FrameParams& F, uint32_t g) {
+  if constexpr (ONE) return F.one;
+  else return F.g.rs[find_base(F.g.tri_base, 0, F.g.n_renderables, g)];
+}
+
+// Blocks of 256 threads per SM the register budget of the setup kernels must
+// allow.  With the vertex pass the kernel waits on index -> vertex gathers
+// and more resident warps hide that: 6 (40 registers, some spilled to L1)
+// with the packed staging records, which leave more L1 to the spills.
+// Without it (triangle soups) it is bound by its strided position loads and
+// by instruction issue, spilling and a smaller L1 cost more than the extra
+// warps hide, and the aligned records' vector copies are cheaper: 4 (64
+// registers).  Measured on 1080p and 4K frames.
 template <bool PRE>
 constexpr int kSetupMinBlocks = PRE ? 6 : 4;
-template <bool PRE>
-__global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE>) k_setup(FrameParams F) {
+template <bool PRE, bool ONE>
+__global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup(FrameParams F) {
   pdl_wait();
   using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;  // see kSetupMinBlocks
-  __shared__ Rec s_rec[kSetupWarps][kStageRecs];
-  __shared__ int s_pre[kSetupWarps][kStageRecs];
-  __shared__ BlockCounters bc;
-  if (threadIdx.x < 3) bc.v[threadIdx.x] = 0;
-  __syncthreads();
+  __shared__ Rec s_rec[kSetupThreads / 32][kStageRecs];
+  __shared__ int s_pre[kSetupThreads / 32][kStageRecs];
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  const bool persp = F.v.persp != 0;
-  Setup S[2];
-  int kind[2] = {0, 0};  // 0 none, 1 small, 2 big
-  unsigned n_clipped = 0, n_raster = 0, n_small = 0;
-  if (g < F.g.n_tris) {
-    const DevRenderable& R = F.g.rs[find_base(F.g.tri_base, 0, F.g.n_renderables, g)];
-    if (!setup_triangle<PRE>(F.v, F.g, R, g, S, kind, n_clipped)) {
-      atomicOr(&F.counters->error_flags, 1u);
-    } else {
-#pragma unroll
-      for (int s = 0; s < 2; s++)
-        if (kind[s]) {
-          n_raster++;
-          long long bw = S[s].x1 - S[s].x0 + 1, bh = S[s].y1 - S[s].y0 + 1;
-          if (bw * bh <= (long long)F.small_max) n_small++;
-          else kind[s] = 2;
-        }
-    }
+  const unsigned w = threadIdx.x >> 5;
+  const bool in = g < F.g.n_tris;
+  const DevRenderable& R = renderable<ONE>(F, in ? g : 0u);
+  const int t = (int)(g - R.tri_base);
+  int n_sub = 0;
+  if (in) {
+    if (bad_triangle(R.mesh, t)) atomicOr(&F.counters->error_flags, 1u);
+    else n_sub = 1;
   }
-  // large records: warp-level compaction, one atomic per warp and slot
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    unsigned m = __ballot_sync(0xffffffffu, kind[s] == 2);
-    if (m == 0) continue;
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(&F.counters->rec_count, (unsigned)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    unsigned n_items = 0, slot = 0;
-    if (kind[s] == 2) {
-      slot = base + __popc(m & lt);
-      if (slot < F.rec_cap) {
-        F.recs[slot] = to_rec(S[s], 2u * g + (uint32_t)s);
-        n_items = (unsigned)(S[s].y1 - S[s].y0 + kLargeRows) / kLargeRows;
-      } else {
-        kind[s] = 1;  // no record left (a fixed record store): rasterised below
-      }
+#pragma unroll 1
+  for (int sub = 0; sub < 2; sub++) {
+    if (sub && !__any_sync(0xffffffffu, n_sub == 2)) break;
+    Setup S;
+    bool small = false, big = false, cut = false;
+    if (n_sub > sub && sub_setup<PRE>(F.v, F.g, R, t, sub, S, n_sub, cut)) {
+      small = box_pixels(S) <= (long long)F.small_max;
+      big = !small;
     }
-    // its row blocks: one range per warp, each lane's at its exclusive prefix
-    unsigned inc = n_items;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
-      if ((int)lane >= o) inc += u;
-    }
-    const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
-    unsigned ibase = 0;
-    if (lane == 0 && total) ibase = atomicAdd(&F.counters->item_count, total);
-    ibase = __shfl_sync(0xffffffffu, ibase, 0) + inc - n_items;
-    // blocks past the end of the list: the record's remaining rows go to the
-    // spill list (at most one entry per record, so it cannot overflow)
-    for (unsigned k = 0; k < n_items; k++) {
-      const uint32_t row = (uint32_t)(S[s].y0 + (int)k * kLargeRows);
-      if (ibase + k < F.item_cap) {
-        F.items[ibase + k] = LargeItem{slot, row};
-      } else {
-        F.spill[atomicAdd(&F.counters->spill_count, 1u)] = LargeItem{slot, row};
-        break;
-      }
-    }
+    count_triangles(F.counters, small, big, sub == 0 && cut && n_sub > 0);
+    const uint32_t id = 2u * g + (uint32_t)sub;
+    if (!append_large(F, S, big, id)) small = true;  // rasterised here, as small ones are
+    raster_small(S, small, id, 0u, FrameTarget{F.vis, F.v.W, F.v.persp != 0}, s_rec[w], s_pre[w]);
   }
-  const uint32_t ids[2] = {2u * g, 2u * g + 1u};
-  raster_small(S, kind, ids, 0u, FrameTarget{F.vis, F.v.W, persp}, s_rec[w], s_pre[w]);
-  block_count(bc, 0, n_raster);
-  block_count(bc, 1, n_small);
-  block_count(bc, 2, n_clipped);
-  block_flush(bc, &F.counters->rasterised, &F.counters->small_direct, &F.counters->clipped);
 }
 
-// Large sub-triangles, one warp per row block of kLargeRows rows of a record,
-// one row per lane: each row is walked across the record's whole bounding
-// box (no replay beyond the reference's own) with 64-bit atomicMin into
-// vis[] (src/Renderer.cpp:238-269).  Then the spill list: one warp per
-// record, its remaining rows kLargeRows at a time.  An ordinary launch: with
-// no large record every warp leaves at once.
-__device__ __forceinline__ void raster_rec_row(const FrameParams& F, bool persp, const BigRec& R, int y) {
+// Large sub-triangles, one warp per block of kLargeRows rows by one column
+// segment of a record's bounding box, one row per lane: the lane replays its
+// row to the segment and walks it with 64-bit atomicMin into vis[]
+// (src/Renderer.cpp:238-269).  Then the spill list: one warp per record, its
+// remaining blocks.  An ordinary launch: with no large record every warp
+// leaves at once.
+// Bound by the serial walk of a row, which is why rows are cut into segments
+// (large_segs): 64 primitives at 1280x720, 30.4 -> 10.9 us.
+__device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, uint32_t rec, uint32_t k) {
+  const BigRec& R = F.recs[rec];
   const Setup S = rec_setup(R);
+  const int segs = large_segs(S.x0, S.x1), w = large_seg_cols(S.x0, S.x1);
+  const int b = (int)k / segs, c = (int)k - b * segs;
+  const int y = S.y0 + b * kLargeRows + (int)(threadIdx.x & 31);
+  if (y > S.y1) return;
+  const int xs = S.x0 + c * w;
   unsigned long long* row = F.vis + (size_t)y * F.v.W;
-  walk_row(S, persp, R.id, y, S.x0, S.x1,
+  walk_row(S, persp, R.id, y, xs, min(xs + w - 1, S.x1),
            [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
 }
 
 __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
   pdl_wait();
   pdl_trigger();
-  const uint32_t n = min(F.counters->item_count, F.item_cap);
+  const uint32_t n = (uint32_t)min(F.counters->item_count, (unsigned long long)F.item_cap);
   const uint32_t n_spill = F.counters->spill_count;
   const bool persp = F.v.persp != 0;
-  const int lane = (int)(threadIdx.x & 31);
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (uint32_t it = w0; it < n; it += nw) {
-    const LargeItem item = F.items[it];
-    const BigRec& R = F.recs[item.rec];
-    const int y = (int)item.row + lane;
-    if (y <= R.y1) raster_rec_row(F, persp, R, y);
-  }
+  for (uint32_t it = w0; it < n; it += nw) raster_block(F, persp, F.items[it].rec, F.items[it].k);
   for (uint32_t it = w0; it < n_spill; it += nw) {
     const LargeItem item = F.spill[it];
     const BigRec& R = F.recs[item.rec];
-    for (int y = (int)item.row + lane; y <= R.y1; y += kLargeRows) raster_rec_row(F, persp, R, y);
+    const uint32_t blocks = (uint32_t)(((R.y1 - R.y0) / kLargeRows + 1) * large_segs(R.x0, R.x1));
+    for (uint32_t k = item.k; k < blocks; k++) raster_block(F, persp, item.rec, k);
   }
 }
 
 // Deferred resolve + shade: one thread per pixel, 256-thread blocks over
 // 32x8-pixel tiles.
 constexpr int kResolveTileW = 32, kResolveTileH = 8;
-template <bool PRE>
+template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
   pdl_wait();
   // loadPPM's texel decode b/255.0f (src/io.cpp:410), one division per byte value
@@ -958,10 +965,26 @@ __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
   const int x = bx * kResolveTileW + (lane & 15) + 16 * (w & 1), y = by * kResolveTileH + (lane >> 4) + 2 * (w >> 1);
   if (x >= F.v.W || y >= F.v.H) return;
   const size_t px = (size_t)y * F.v.W + x;
-  V3 value, normal;
-  float depth;
-  uint32_t id;
-  resolve_pixel<PRE>(F.v, F.g, 0, F.g.n_renderables, F.vis[px], x, y, s_dec, value, depth, id, normal);
+  // the winner's setup is re-derived and its edge functions replayed to
+  // column x, then texture and lighting (src/Renderer.cpp:247-305, FAST_LIGHT)
+  const unsigned long long vw = F.vis[px];
+  V3 value = v3(F.v.bg[0], F.v.bg[1], F.v.bg[2]), normal = v3(0, 0, 1);
+  float depth = 1e11f;
+  uint32_t id = MR_NO_TRIANGLE;
+  if (vw != VIS_EMPTY) {
+    id = (uint32_t)vw;
+    const DevRenderable& R = renderable<ONE>(F, id >> 1);
+    int ip[3];
+    Vtx vc[3];
+    bool clipped;
+    winner_tri<PRE>(F.v, F.g, R, id, ip, vc, clipped);
+    Setup S;
+    winner_setup<PRE>(F.v, F.g, R, ip, vc, clipped, S);
+    float e1, e2, k0, k1, k2;
+    replay(S, x, y, e1, e2);
+    depth = frag_depth(S, F.v.persp != 0, e1, e2, k0, k1, k2);
+    shade(F.v, R, vc, k0, k1, k2, s_dec, value, normal);
+  }
   if (F.rgb8) {
     F.rgb8[3 * px + 0] = to_byte(value.x);
     F.rgb8[3 * px + 1] = to_byte(value.y);
@@ -987,70 +1010,66 @@ __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
 // (the register budget and staging layout of k_setup, for the same reasons;
 // on the 256-scene batch: 0.665 -> 0.453 ms)
 template <bool PRE>
-__global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE>) k_setup_batch(BatchParams B) {
+__global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256 / kSetupBatchThreads) k_setup_batch(BatchParams B) {
   using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;
-  __shared__ Rec s_rec[kSetupWarps][kStageRecs];
-  __shared__ int s_pre[kSetupWarps][kStageRecs];
-  __shared__ BlockCounters bc;
+  __shared__ Rec s_rec[kSetupBatchThreads / 32][kStageRecs];
+  __shared__ int s_pre[kSetupBatchThreads / 32][kStageRecs];
   __shared__ unsigned s_fill, s_base;
-  if (threadIdx.x < 3) bc.v[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_fill = 0;
   __syncthreads();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
-  Setup S[2];
-  int kind[2] = {0, 0};  // 0 none, 1 small (rasterised here), 2 record
-  unsigned n_clipped = 0, n_raster = 0, n_small = 0;
   uint32_t scene = 0;
+  const DevRenderable* R = nullptr;
   if (g < B.g.n_tris) {
-    const DevRenderable& R = B.g.rs[find_base(B.g.tri_base, 0, B.g.n_renderables, g)];
-    scene = R.scene;
-    if (!setup_triangle<PRE>(B.scenes[scene].v, B.g, R, g, S, kind, n_clipped))
+    R = &B.g.rs[find_base(B.g.tri_base, 0, B.g.n_renderables, g)];
+    scene = R->scene;
+    if (bad_triangle(R->mesh, (int)(g - R->tri_base))) {
       atomicOr(&B.counters->error_flags, 1u);
-#pragma unroll
-    for (int s = 0; s < 2; s++)
-      if (kind[s]) {
-        n_raster++;
-        long long bw = S[s].x1 - S[s].x0 + 1, bh = S[s].y1 - S[s].y0 + 1;
-        if (bw * bh <= (long long)B.small_max) n_small++;
-        else kind[s] = 2;
-      }
+      R = nullptr;
+    }
   }
-  // record slots: each warp reserves within the block, the block once globally
-  unsigned m2[2], wbase = 0;
-#pragma unroll
-  for (int s = 0; s < 2; s++) m2[s] = __ballot_sync(0xffffffffu, kind[s] == 2);
-  const unsigned wn = __popc(m2[0]) + __popc(m2[1]);
-  if (lane == 0 && wn) wbase = atomicAdd(&s_fill, wn);
-  wbase = __shfl_sync(0xffffffffu, wbase, 0);
-  __syncthreads();
-  if (threadIdx.x == 0) s_base = s_fill ? atomicAdd(&B.counters->rec_count, s_fill) : 0;
-  __syncthreads();
-  unsigned base = s_base + wbase;
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const unsigned m = m2[s];
-    if (m == 0) continue;
-    if (kind[s] == 2) {
-      unsigned slot = base + __popc(m & lt);
+  int n_sub = R ? 1 : 0;
+#pragma unroll 1
+  for (int sub = 0; sub < 2; sub++) {
+    // (the second round, of triangles cut in two, is rare and a warp's own)
+    if (sub && !__any_sync(0xffffffffu, n_sub == 2)) break;
+    Setup S;
+    bool small = false, big = false, cut = false;
+    if (n_sub > sub && sub_setup<PRE>(B.scenes[scene].v, B.g, *R, (int)(g - R->tri_base), sub, S, n_sub, cut)) {
+      small = box_pixels(S) <= (long long)B.small_max;
+      big = !small;
+    }
+    count_triangles(B.counters, small, big, sub == 0 && cut && n_sub > 0);
+    // record slots: in the first round each warp reserves within the block
+    // and the block once globally
+    const unsigned m = __ballot_sync(0xffffffffu, big);
+    unsigned base = 0;
+    if (sub == 0) {
+      if (lane == 0 && m) base = atomicAdd(&s_fill, (unsigned)__popc(m));
+      __syncthreads();
+      if (threadIdx.x == 0) s_base = s_fill ? atomicAdd(&B.counters->rec_count, s_fill) : 0;
+      __syncthreads();
+      base += s_base;
+    } else if (lane == 0 && m) {
+      base = atomicAdd(&B.counters->rec_count, (unsigned)__popc(m));
+    }
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const uint32_t id = 2u * g + (uint32_t)sub;
+    if (big) {
+      const unsigned slot = base + __popc(m & lt);
       if (slot < B.rec_cap) {
-        B.recs[slot] = to_rec(S[s], 2u * g + (uint32_t)s);
+        B.recs[slot] = to_rec(S, id);
         B.rec_scene[slot] = scene;
         const SceneRec& SR = B.scenes[scene];
-        int tx0 = S[s].x0 / B.tile_w, tx1 = S[s].x1 / B.tile_w, ty0 = S[s].y0 / B.tile_h, ty1 = S[s].y1 / B.tile_h;
+        const int tx0 = S.x0 / B.tile_w, tx1 = S.x1 / B.tile_w, ty0 = S.y0 / B.tile_h, ty1 = S.y1 / B.tile_h;
         for (int ty = ty0; ty <= ty1; ty++)
           for (int tx = tx0; tx <= tx1; tx++)
             atomicAdd(B.tile_count + SR.tile_base + ty * SR.tiles_x + tx, 1u);
       }
     }
-    base += __popc(m);
+    if (B.small_max > 0) raster_small(S, small, id, scene, BatchTarget{B.scenes}, s_rec[w], s_pre[w]);
   }
-  const uint32_t ids[2] = {2u * g, 2u * g + 1u};
-  if (B.small_max > 0) raster_small(S, kind, ids, scene, BatchTarget{B.scenes}, s_rec[w], s_pre[w]);
-  block_count(bc, 0, n_raster);
-  block_count(bc, 1, n_small);
-  block_count(bc, 2, n_clipped);
-  block_flush(bc, &B.counters->rasterised, &B.counters->small_direct, &B.counters->clipped);
 }
 
 // Renderables per scene whose triangle bases k_batch keeps in shared memory
@@ -1239,7 +1258,6 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B, uint32_t* bl
     if (threadIdx.x == 0) {
       B.tile_start[B.n_tiles] = run;
       B.counters->bin_needed = run;
-      B.counters->bin_entries += run;
     }
   }
   grid.sync();
@@ -1367,8 +1385,9 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B, uint32_t* bl
         int ip[3];
         Vtx vc[3];
         bool clipped;
-        const DevRenderable& R = *winner_tri<PRE>(s_view, B.g, s_meta[3], s_meta[4], id, ip, vc, clipped,
-                                                   tb_shared ? s_tb : nullptr);
+        const DevRenderable& R = B.g.rs[tb_shared ? s_meta[3] + find_base(s_tb, 0, n_rs, id >> 1)
+                                                  : find_base(B.g.tri_base, s_meta[3], s_meta[4], id >> 1)];
+        winner_tri<PRE>(s_view, B.g, R, id, ip, vc, clipped);
         Setup S;
         float e1, e2;
         const float2 ee = captured ? s_e[i] : make_float2(__int_as_float(0x7fc00000), 0.f);
@@ -1395,7 +1414,8 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B, uint32_t* bl
   }
 }
 
-__global__ void k_range(int W, int H, const float* P, const float* depth, float* xyz) {
+__global__ void k_range(int W, int H, Mat4 M, const float* depth, float* xyz) {
+  const float* P = M.m;
   size_t px = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (px >= (size_t)W * H) return;
   int i = (int)(px / W), j = (int)(px - (size_t)i * W);
@@ -1469,29 +1489,32 @@ static cudaError_t launch_coop(const void* fn, int grid, int block, void** args,
 }
 
 // Launch sequence of one frame.  With F.g.va set, the vertex pass runs first
-// and the setup/resolve kernels read its buffers.  ev (optional, 6 events)
-// brackets the stages: clear+vertex, setup, large-triangle raster, -, resolve.
-cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev, cudaEvent_t staged) {
-  size_t npx = (size_t)F.v.W * F.v.H;
-  const bool pre = F.g.va != nullptr;
+// and the setup/resolve kernels read its buffers.  staged (frames of several
+// renderables) is recorded once the staging block has been read.  ev
+// (optional, 6 events) brackets the stages: clear+vertex, setup,
+// large-triangle raster, -, resolve.
+template <bool PRE, bool ONE>
+static cudaError_t launch_stages(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev, cudaEvent_t staged) {
+  const size_t npx = (size_t)F.v.W * F.v.H;
+  const size_t n_verts = PRE ? (size_t)F.g.n_verts + F.g.n_nrms : 0;
   if (ev) cudaEventRecord(ev[0], st);
   // The clear also brings vis[] into L2 (write-allocate), so the setup
   // kernel's atomics hit L2.
-  const int cgrid = std::min(grid_for(npx, 256), sm_count() * 16);
-  k_clear<<<cgrid, 256, 0, st>>>(
-      F.vis, npx, reinterpret_cast<uint32_t*>(F.counters), (uint32_t)(sizeof(Counters) / 4), nullptr, 0,
-      F.stage_src, F.stage_dst, F.stage_n16);
-  if (staged) cudaEventRecord(staged, st);  // the staging block has been read
-  // vertex pass, setup and resolve may be scheduled while their predecessor
-  // finishes (they wait for it before reading its output)
+  const int cgrid = std::min(grid_for((npx + 1) / 2, 256), sm_count() * 16);
   cudaError_t le = cudaSuccess;
-  if (pre && (F.g.n_verts + F.g.n_nrms) > 0)
-    le = launch_after(k_vertex, grid_for((size_t)F.g.n_verts + F.g.n_nrms, 256), 256, st, F.g, F.v,
-                      (const SceneRec*)nullptr);
-  if (le != cudaSuccess) return le;
+  if (PRE && ONE) {
+    k_begin<true><<<std::max(cgrid, grid_for(n_verts, 256)), 256, 0, st>>>(F);
+  } else {
+    k_begin<false><<<cgrid, 256, 0, st>>>(F);
+    if (staged && !ONE) cudaEventRecord(staged, st);
+    // vertex pass, setup and resolve may be scheduled while their predecessor
+    // finishes (they wait for it before reading its output)
+    if (n_verts) le = launch_after(k_vertex<false>, grid_for(n_verts, 256), 256, st, F.g, F.v, (const SceneRec*)nullptr);
+    if (le != cudaSuccess) return le;
+  }
   if (ev) cudaEventRecord(ev[1], st);
   if (F.g.n_tris) {
-    le = launch_after(pre ? k_setup<true> : k_setup<false>, grid_for(F.g.n_tris, kSetupThreads), kSetupThreads, st, F);
+    le = launch_after(k_setup<PRE, ONE>, grid_for(F.g.n_tris, kSetupThreads), kSetupThreads, st, F);
     if (le != cudaSuccess) return le;
   }
   if (ev) cudaEventRecord(ev[2], st);
@@ -1500,10 +1523,17 @@ cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev,
   if (ev) cudaEventRecord(ev[3], st);
   if (ev) cudaEventRecord(ev[4], st);
   const int rgrid = ((F.v.W + kResolveTileW - 1) / kResolveTileW) * ((F.v.H + kResolveTileH - 1) / kResolveTileH);
-  le = launch_after(pre ? k_resolve<true> : k_resolve<false>, rgrid, 256, st, F);
+  le = launch_after(k_resolve<PRE, ONE>, rgrid, 256, st, F);
   if (le != cudaSuccess) return le;
   if (ev) cudaEventRecord(ev[5], st);
   return cudaGetLastError();
+}
+
+cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev, cudaEvent_t staged) {
+  const bool pre = F.g.va != nullptr;
+  if (F.g.n_renderables == 1)
+    return pre ? launch_stages<true, true>(F, st, ev, staged) : launch_stages<false, true>(F, st, ev, staged);
+  return pre ? launch_stages<true, false>(F, st, ev, staged) : launch_stages<false, false>(F, st, ev, staged);
 }
 
 size_t batch_smem(int tile_w, int tile_h, int chunk) {
@@ -1534,16 +1564,15 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* 
   if (ev) cudaEventRecord(ev[0], st);
   if (pre && B.g.n_verts + B.g.n_nrms > 0) {
     View none = {};
-    k_vertex<<<grid_for((size_t)B.g.n_verts + B.g.n_nrms, 256), 256, 0, st>>>(B.g, none, B.scenes);
+    k_vertex<true><<<grid_for((size_t)B.g.n_verts + B.g.n_nrms, 256), 256, 0, st>>>(B.g, none, B.scenes);
   }
   if (B.small_max > 0 && B.n_px) {  // small triangles' visibility words of every scene
-    const int cgrid = std::min(grid_for(B.n_px, 256), sm_count() * 16);
-    k_clear<<<cgrid, 256, 0, st>>>(B.vis, B.n_px, nullptr, 0, nullptr, 0, nullptr, nullptr, 0);
+    k_clear<<<std::min(grid_for((B.n_px + 1) / 2, 256), sm_count() * 16), 256, 0, st>>>(B.vis, B.n_px);
   }
   if (ev) cudaEventRecord(ev[1], st);
   if (B.g.n_tris) {
-    if (pre) k_setup_batch<true><<<grid_for(B.g.n_tris, kSetupThreads), kSetupThreads, 0, st>>>(B);
-    else k_setup_batch<false><<<grid_for(B.g.n_tris, kSetupThreads), kSetupThreads, 0, st>>>(B);
+    if (pre) k_setup_batch<true><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
+    else k_setup_batch<false><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
   }
   if (ev) cudaEventRecord(ev[2], st);
   BatchParams Bc = B;
@@ -1555,9 +1584,9 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* 
   return cudaGetLastError();
 }
 
-cudaError_t launch_range(int W, int H, const float* dP, const float* depth, float* xyz, cudaStream_t st) {
+cudaError_t launch_range(int W, int H, const Mat4& P, const float* depth, float* xyz, cudaStream_t st) {
   size_t npx = (size_t)W * H;
-  k_range<<<grid_for(npx, 256), 256, 0, st>>>(W, H, dP, depth, xyz);
+  k_range<<<grid_for(npx, 256), 256, 0, st>>>(W, H, P, depth, xyz);
   return cudaGetLastError();
 }
 

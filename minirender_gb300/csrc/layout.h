@@ -71,6 +71,10 @@ struct View {
   float bg[3];
 };
 
+struct Mat4 {
+  float m[16];
+};
+
 // Geometry of a launch: renderable table, base tables and the per-vertex
 // buffers of the vertex pass (va null: kernels transform per triangle).
 struct Geo {
@@ -94,29 +98,44 @@ struct __align__(16) BigRec {
   int32_t x0, y0, x1, y1;     // inclusive clamped pixel bounding box
 };
 
+// Triangle statistics, one slot per group of warps (a single counter updated
+// by every warp would serialise in L2), each on a sector of its own.
+constexpr int kStatSlots = 64;
+struct alignas(32) StatSlot {
+  unsigned long long drawn;    // rasterised sub-triangles << 32 | of these, in the setup kernel
+  unsigned long long clipped;  // triangles cut by the near plane
+};
+
 struct Counters {
-  unsigned long long triangles, clipped, rasterised, small_direct, binned, bin_entries;
+  StatSlot stat[kStatSlots];
   unsigned int error_flags;
   unsigned int rec_count;      // records written
   unsigned int bin_needed;     // total (tile, record) pairs requested
   unsigned int bin_overflow;
   unsigned int work_next;      // persistent-kernel work counter
-  unsigned int item_count;     // large-triangle row blocks requested (single frames)
-  unsigned int spill_count;    // records whose remaining rows did not fit the row-block list
-  unsigned int pad;
+  unsigned int spill_count;    // records whose remaining blocks did not fit the block list
+  unsigned long long item_count;  // large-triangle blocks requested (single frames; 64 bits: a
+                                  // frame of many screen-sized triangles passes 2^32)
 };
 
 // One-frame launch.
-// Row block of a large sub-triangle: kLargeRows rows from `row` of record
-// `rec`; in the spill list, every row from `row` to the record's last.
+// Block `k` of the bounding box of large sub-triangle `rec`: kLargeRows rows
+// by one column segment, blocks numbered along the rows first; in the spill
+// list, every block from `k` to the record's last.
 struct LargeItem {
-  uint32_t rec, row;
+  uint32_t rec, k;
 };
 constexpr int kLargeRows = 32;
+// Columns per segment: 32 columns up to a width of 512, then a 16th of the
+// width (in whole 32s).  A segment starts with the replay of the columns left
+// of it (one add per column); at most 16 segments keep those adds below a
+// sixth of the walk's work.
+constexpr int kLargeCols = 32, kLargeSegs = 16;
 
 struct FrameParams {
   View v;
   Geo g;
+  DevRenderable one;          // the renderable of a frame that has one (no table is staged for it)
   int small_max;
   unsigned long long* vis;    // W*H
   BigRec* recs;               // large sub-triangles
@@ -124,8 +143,8 @@ struct FrameParams {
   LargeItem* items;           // their row blocks
   uint32_t item_cap;
   LargeItem* spill;           // rec_cap entries: records past the end of items[]
-  const uint4* stage_src;     // the frame's staging block in mapped pinned host memory,
-  uint4* stage_dst;           // fetched by the clear kernel (no copy-engine transfer)
+  const uint4* stage_src;     // the frame's staging block in mapped pinned host memory (several
+  uint4* stage_dst;           // renderables), fetched by the clear kernel (no copy-engine transfer)
   uint32_t stage_n16;         // its size in 16-byte units
   uint8_t* rgb8;
   float* depth;

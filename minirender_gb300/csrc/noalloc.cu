@@ -33,11 +33,9 @@ constexpr size_t kVisBytes = (size_t)MR_NOALLOC_MAX_PIXELS * sizeof(unsigned lon
 constexpr size_t kBadOff = al(kVisOff + kVisBytes);
 constexpr size_t kBadBytes = ((size_t)MR_NOALLOC_MAX_TRIANGLES / 32 + 1) * sizeof(uint32_t);
 constexpr size_t kCntOff = al(kBadOff + kBadBytes);
-constexpr size_t kRsOff = al(kCntOff + sizeof(Counters));
-constexpr size_t kBaseOff = al(kRsOff + sizeof(DevRenderable));
 constexpr uint32_t kRecCap = 1u << 15;   // large sub-triangles with a record
-constexpr uint32_t kItemCap = 1u << 16;  // their 32-row blocks (more: the spill list)
-constexpr size_t kRecOff = al(kBaseOff + 2 * sizeof(uint32_t));
+constexpr uint32_t kItemCap = 1u << 17;  // their blocks (more: the spill list)
+constexpr size_t kRecOff = al(kCntOff + sizeof(Counters));
 constexpr size_t kItemOff = al(kRecOff + (size_t)kRecCap * sizeof(BigRec));
 constexpr size_t kSpillOff = al(kItemOff + (size_t)kItemCap * sizeof(LargeItem));
 constexpr size_t kEnd = al(kSpillOff + (size_t)kRecCap * sizeof(LargeItem));  // one entry per record at most
@@ -126,8 +124,6 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
     if (tex_is_rgb8) R.tex8 = (const uint8_t*)texture;
     else R.texf = (const float*)texture;
   }
-  const uint32_t base[2] = {0, (uint32_t)M.n_tri};
-
   const int W = f->width, H = f->height;
   FrameParams F;
   memset(&F, 0, sizeof(F));
@@ -150,8 +146,7 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
   // kernel; larger ones take records and row blocks from the fixed store
   // (the spill list holds one entry per record, so it cannot overflow).
   F.small_max = 64;
-  F.g.rs = (const DevRenderable*)(S + kRsOff);
-  F.g.tri_base = (const uint32_t*)(S + kBaseOff);
+  F.one = R;
   F.vis = (unsigned long long*)(S + kVisOff);
   F.recs = (BigRec*)(S + kRecOff);
   F.rec_cap = kRecCap;
@@ -163,10 +158,7 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
   F.ids = tri_id;
   F.counters = (Counters*)(S + kCntOff);
 
-  cudaError_t e = cudaMemcpyAsync(S + kRsOff, &R, sizeof(R), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(S + kBaseOff, base, sizeof(base), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(S + kCntOff, 0, sizeof(Counters), st);
-  if (e == cudaSuccess) e = launch_validate(M, (uint32_t*)(S + kBadOff), st);
+  cudaError_t e = launch_validate(M, (uint32_t*)(S + kBadOff), st);
   if (e == cudaSuccess) e = launch_frame(F, st, nullptr);
   Counters c;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&c, S + kCntOff, sizeof(c), cudaMemcpyDeviceToHost, st);
