@@ -702,11 +702,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   F.v.H = H;
   F.v.w = (float)W;
   F.v.h = (float)H;
-  memcpy(F.v.P, f->projection, sizeof(F.v.P));
-  // Renderer::render, src/Renderer.cpp:317-326.
-  F.v.persp = f->projection[15] == 0;
-  float zn = F.v.persp ? f->projection[11] / (f->projection[10] - 1) : (f->projection[11] + 1) / f->projection[10];
-  F.v.znear = -zn;
+  set_projection(F.v, f->projection);
   if (f->light_is_point) affine(f->view, f->light, F.v.lightdir);
   else normalized(f->light, F.v.lightdir);
   F.v.ambient = f->ambient;
@@ -901,10 +897,7 @@ static void make_view(const mr_frame* f, View& V) {
   V.H = f->height;
   V.w = (float)f->width;
   V.h = (float)f->height;
-  memcpy(V.P, f->projection, sizeof(V.P));
-  V.persp = f->projection[15] == 0;
-  float zn = V.persp ? f->projection[11] / (f->projection[10] - 1) : (f->projection[11] + 1) / f->projection[10];
-  V.znear = -zn;
+  set_projection(V, f->projection);
   if (f->light_is_point) affine(f->view, f->light, V.lightdir);
   else normalized(f->light, V.lightdir);
   V.ambient = f->ambient;

@@ -75,6 +75,16 @@ struct DevBuf {
   }
 };
 
+// Projection state of a frame as Renderer::render() prepares it
+// (src/Renderer.cpp:317-326).
+inline void set_projection(View& V, const float* P) {
+  memcpy(V.P, P, sizeof(V.P));
+  V.persp = P[15] == 0;
+  V.simple = V.persp && P[1] == 0 && P[3] == 0 && P[4] == 0 && P[7] == 0 && P[12] == 0 && P[13] == 0 && P[14] == -1;
+  const float zn = V.persp ? P[11] / (P[10] - 1) : (P[11] + 1) / P[10];
+  V.znear = -zn;
+}
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace mrgi

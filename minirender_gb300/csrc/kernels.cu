@@ -86,6 +86,23 @@ __device__ __forceinline__ V2 ld2(const float* p, int i) {
   return v2(__ldg(p + 2 * i), __ldg(p + 2 * i + 1));
 }
 
+// Two IEEE binary32 additions in one instruction (each half is rounded as the
+// scalar addition rounds); the setup and resolve kernels are bound by
+// instruction issue.  Products stay scalar: a packed multiply feeding a packed
+// add came out one unit in the last place off, as a fused one does.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 // htransform, src/Renderer.cpp:13-20
 __device__ __forceinline__ V3 htransform(const float* m, V3 p) {
   float iw = rcp(m[12] * p.x + m[13] * p.y + m[14] * p.z + m[15]);
@@ -100,6 +117,32 @@ __device__ __forceinline__ void project(const View& V, V3 v, float& px, float& p
   px = (1 + ndc.x) * (V.w / 2);
   py = (1 - ndc.y) * (V.h / 2);
   zt = V.persp ? -rcp(v.z) : ndc.z;
+}
+
+// project() of a triangle's three corners.  For V.simple matrices and finite
+// corners off the z = 0 plane the products with zero entries are +-0, which
+// change no sum that reaches a pixel coordinate, w is exactly -z, and the
+// perspective z term -1/z is the 1/w already taken: 10 operations and a
+// reciprocal a corner instead of 35 and two.
+__device__ __forceinline__ void project3(const View& V, const Vtx (&v)[3], V2 (&p)[3], float (&zt)[3]) {
+  const float size = ((fabsf(v[0].pos.x) + fabsf(v[0].pos.y)) + (fabsf(v[1].pos.x) + fabsf(v[1].pos.y))) +
+                     ((fabsf(v[2].pos.x) + fabsf(v[2].pos.y)) +
+                      (fabsf(v[0].pos.z) + (fabsf(v[1].pos.z) + fabsf(v[2].pos.z))));  // NaN or inf: not finite
+  const float zmin = fminf(fminf(fabsf(v[0].pos.z), fabsf(v[1].pos.z)), fabsf(v[2].pos.z));
+  if (V.simple && size < __int_as_float(0x7f800000) && zmin > 0) {
+    const float hw = V.w / 2, hh = V.h / 2;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const V3 q = v[c].pos;
+      const float iw = rcp(-q.z);
+      p[c].x = (1 + (V.P[0] * q.x + V.P[2] * q.z) * iw) * hw;
+      p[c].y = (1 - (V.P[5] * q.y + V.P[6] * q.z) * iw) * hh;
+      zt[c] = iw;
+    }
+  } else {
+#pragma unroll
+    for (int c = 0; c < 3; c++) project(V, v[c].pos, p[c].x, p[c].y, zt[c]);
+  }
 }
 
 // clip(), src/Renderer.cpp:121-129
@@ -228,60 +271,55 @@ struct Setup {
   int x0, y0, x1, y1;
 };
 
-// paintTriangle setup from projected corners, src/Renderer.cpp:198-224.
-// False = nothing to draw (off screen or culled).
-__device__ __forceinline__ bool setup_from(const View& V, const V2 (&p)[3], const float (&zt)[3], Setup& S) {
-  V2 pmin = v2(1e30f, 1e30f), pmax = v2(-1e30f, -1e30f);
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    pmin = v2(minr(pmin.x, p[i].x), minr(pmin.y, p[i].y));
-    pmax = v2(maxr(pmax.x, p[i].x), maxr(pmax.y, p[i].y));
-  }
-  if (pmax.x < 0 || pmax.y < 0 || pmin.x > V.w || pmin.y > V.h) return false;
-  float d0x = p[0].x - p[1].x, d0y = p[0].y - p[1].y;
-  float d2x = p[2].x - p[1].x, d2y = p[2].y - p[1].y;
-  float a = d0x * d2y - d0y * d2x;
-  if (a <= 0) return false;  // back-face cull, :207-210
-  float i2a = (a == 0) ? 0.0f : -rcp(a);
+// The edge functions of paintTriangle's setup, src/Renderer.cpp:204-224, of a
+// triangle with signed area a > 0 (or NaN).
+__device__ __forceinline__ void setup_edges(const V2 (&p)[3], const float (&zt)[3], float a, Setup& S) {
+  const float i2a = -rcp(a);
   float ex = p[0].x - p[2].x, ey = p[0].y - p[2].y;
   S.n1 = v2(-ey * i2a, ex * i2a);
   ex = p[1].x - p[0].x;
   ey = p[1].y - p[0].y;
   S.n2 = v2(-ey * i2a, ex * i2a);
-  pmin.x = clampr(pmin.x, 0.f, V.w - 1);
-  pmax.x = clampr(pmax.x, 0.f, V.w - 1);
-  pmin.y = clampr(pmin.y, 0.f, V.h - 1);
-  pmax.y = clampr(pmax.y, 0.f, V.h - 1);
-  S.x0 = (int)floorf(pmin.x);
-  S.y0 = (int)floorf(pmin.y);
-  S.x1 = (int)floorf(pmax.x);
-  S.y1 = (int)floorf(pmax.y);
   S.p0 = p[0];
   S.p2 = p[2];
   S.z[0] = zt[0];
   S.z[1] = zt[1];
   S.z[2] = zt[2];
+}
+__device__ __forceinline__ float area2(const V2 (&p)[3]) {
+  const float d0x = p[0].x - p[1].x, d0y = p[0].y - p[1].y;
+  const float d2x = p[2].x - p[1].x, d2y = p[2].y - p[1].y;
+  return d0x * d2y - d0y * d2x;
+}
+// Least and greatest of three coordinates, a NaN among them ignored as the
+// reference's running comparisons from +-1e30 ignore it (src/Renderer.cpp:
+// 198-203; the sign of a zero, which min and max may choose differently, is
+// lost in the clamp and floor that follow).
+__device__ __forceinline__ float least(float a, float b, float c) { return fminf(fminf(fminf(a, b), c), 1e30f); }
+__device__ __forceinline__ float greatest(float a, float b, float c) { return fmaxf(fmaxf(fmaxf(a, b), c), -1e30f); }
+// Pixel of a coordinate clamped to 0..n-1.
+__device__ __forceinline__ int pixel_of(float x, float n) { return __float2int_rd(fminf(fmaxf(x, 0.f), n - 1)); }
+
+// paintTriangle setup from projected corners, src/Renderer.cpp:198-224.
+// False = nothing to draw (off screen or culled).
+__device__ __forceinline__ bool setup_from(const View& V, const V2 (&p)[3], const float (&zt)[3], Setup& S) {
+  const float xmin = least(p[0].x, p[1].x, p[2].x), ymin = least(p[0].y, p[1].y, p[2].y);
+  const float xmax = greatest(p[0].x, p[1].x, p[2].x), ymax = greatest(p[0].y, p[1].y, p[2].y);
+  if (xmax < 0 || ymax < 0 || xmin > V.w || ymin > V.h) return false;
+  const float a = area2(p);
+  if (a <= 0) return false;  // back-face cull, :207-210
+  setup_edges(p, zt, a, S);
+  S.x0 = pixel_of(xmin, V.w);
+  S.y0 = pixel_of(ymin, V.h);
+  S.x1 = pixel_of(xmax, V.w);
+  S.y1 = pixel_of(ymax, V.h);
   return true;
 }
 
-// Setup of a sub-triangle given by view-space corners (the clipped path).
-__device__ __forceinline__ bool setup_view(const View& V, const Vtx (&s)[3], Setup& S) {
-  V2 p[3];
-  float zt[3];
-#pragma unroll
-  for (int i = 0; i < 3; i++) project(V, s[i].pos, p[i].x, p[i].y, zt[i]);
-  return setup_from(V, p, zt, S);
-}
-
 // Edge functions at the start of row y (pixel centre x0+0.5), :240-242.
-__device__ __forceinline__ void row_start(const Setup& S, int y, float& e1, float& e2) {
-  float yf = (float)y + 0.5f;
-  float ptx = (float)S.x0 + 0.5f;
-  float qx = ptx - S.p2.x, qy = yf - S.p2.y;
-  e1 = S.n1.x * qx + S.n1.y * qy;
-  qx = ptx - S.p0.x;
-  qy = yf - S.p0.y;
-  e2 = S.n2.x * qx + S.n2.y * qy;
+__device__ __forceinline__ unsigned long long row_start2(const Setup& S, int y) {
+  const float yf = (float)y + 0.5f, ptx = (float)S.x0 + 0.5f;
+  return pack2(S.n1.x * (ptx - S.p2.x) + S.n1.y * (yf - S.p2.y), S.n2.x * (ptx - S.p0.x) + S.n2.y * (yf - S.p0.y));
 }
 
 // Depth of a covered fragment and its perspective-corrected weights, :247-261.
@@ -300,25 +338,10 @@ __device__ __forceinline__ float frag_depth(const Setup& S, bool persp, float e1
   return k0 * S.z[0] + k1 * S.z[1] + k2 * S.z[2] + 0.0f * 1.0f;
 }
 
-__device__ __forceinline__ bool covered(float e1, float e2) {
-  return !(e1 < 0 || e2 < 0 || 1 - e1 - e2 < 0);
-}
+// !(e1 < 0 || e2 < 0 || 1 - e1 - e2 < 0): a NaN is not below zero, and min
+// ignores it.
+__device__ __forceinline__ bool covered(float e1, float e2) { return !(fminf(fminf(e1, e2), 1 - e1 - e2) < 0); }
 
-// Two edge values advanced together: one packed IEEE add per column
-// (add.rn.f32x2 rounds each half as the scalar add does).
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
 // The edge values n columns on: n running sums, column by column.
 __device__ __forceinline__ unsigned long long advance2(unsigned long long e, unsigned long long d, int n) {
 #pragma unroll 1
@@ -339,9 +362,8 @@ template <typename Emit>
 __device__ __forceinline__ void walk_row(const Setup& S, bool persp, uint32_t id, int y, int xs,
                                          int xe, Emit emit) {
   float e1, e2;
-  row_start(S, y, e1, e2);
   const unsigned long long d = pack2(S.n1.x, S.n2.x);
-  unsigned long long e = advance2(pack2(e1, e2), d, xs - S.x0);
+  unsigned long long e = advance2(row_start2(S, y), d, xs - S.x0);
   for (int x = xs; x <= xe; x++) {
     unpack2(e, e1, e2);
     if (covered(e1, e2)) {
@@ -390,26 +412,34 @@ __device__ __forceinline__ Setup rec_setup(const BigRec& B) {
   return S;
 }
 
+// Whether triangle t's indices failed the upload check.
+__device__ __forceinline__ bool bad_triangle(const DevMesh& M, int t) { return (M.bad[t >> 5] >> (t & 31)) & 1u; }
+
 // Assembly, near clip and setup of sub-triangle `sub` of triangle t (paintMesh
 // + the first half of paintTriangle).  True: it has pixels to test.  n_sub:
-// the triangle's sub-triangles (1 when the near plane does not cut it).  The
-// setup kernels take a triangle's second half in a round of its own, so only
-// one Setup is live (two cost the vertex-pass instance a third of its
-// registers; the round runs for warps with such a triangle only).
+// the triangle's sub-triangles (1 when the near plane does not cut it), -1
+// when its indices failed the upload check.  The setup kernels take a
+// triangle's second half in a round of its own, so only one Setup is live
+// (two cost the vertex-pass instance a third of its registers; the round runs
+// for warps with such a triangle only).
 template <bool PRE>
 __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const DevRenderable& R, int t, int sub,
                                           Setup& S, int& n_sub, bool& cut) {
-  int ip[3];
-#pragma unroll
-  for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
   // no_clip (paintTriangle(..., world=false)): never clipped, so the near
   // test compares against +inf
   const float zn = R.no_clip ? __int_as_float(0x7f800000) : V.znear;
   V2 p[3];
   float zt[3];
   Vtx v[3];
+  int ip[3];
   if (PRE) {
+    if (bad_triangle(R.mesh, t)) {
+      n_sub = -1;
+      return false;
+    }
     float4 a[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       a[c] = G.va[R.vert_base + ip[c]];
@@ -418,6 +448,14 @@ __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const Dev
     }
     cut = a[0].w > zn || a[1].w > zn || a[2].w > zn;
   } else {
+    // (indices and index check in flight together; with the vertex pass the
+    // three registers cost more than the latency)
+#pragma unroll
+    for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
+    if (bad_triangle(R.mesh, t)) {
+      n_sub = -1;
+      return false;
+    }
     corners<false, false>(G, R, t, ip, v);
     cut = v[0].pos.z > zn || v[1].pos.z > zn || v[2].pos.z > zn;
   }
@@ -427,19 +465,13 @@ __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const Dev
     n_sub = clip_pick<false>(zn, v, sub);
     if (n_sub <= sub) return false;
   }
-  if (!PRE || cut) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) project(V, v[c].pos, p[c].x, p[c].y, zt[c]);
-  }
+  if (!PRE || cut) project3(V, v, p, zt);
   return setup_from(V, p, zt, S);
 }
 
 __device__ __forceinline__ long long box_pixels(const Setup& S) {
   return (long long)(S.x1 - S.x0 + 1) * (S.y1 - S.y0 + 1);
 }
-
-// Whether triangle t's indices failed the upload check.
-__device__ __forceinline__ bool bad_triangle(const DevMesh& M, int t) { return (M.bad[t >> 5] >> (t & 31)) & 1u; }
 
 // The sub-triangle `id` (of R) won by a pixel: its vertex indices and
 // view-space corners with attributes (the clipped sub-triangle when the
@@ -496,30 +528,31 @@ __device__ __forceinline__ void shade(const View& V, const DevRenderable& R, con
 }
 
 // The setup (src/Renderer.cpp:198-224) of the winning sub-triangle, the same
-// values its raster used.
+// values its raster used; of the bounding box only the column x0 that a
+// replay starts from.
 template <bool PRE>
 __device__ __forceinline__ void winner_setup(const View& V, const Geo& G, const DevRenderable& R,
                                              const int (&ip)[3], const Vtx (&vc)[3], bool clipped, Setup& S) {
+  V2 p[3];
+  float zt[3];
   if (PRE && !clipped) {
-    V2 p[3];
-    float zt[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       float4 a = G.va[R.vert_base + ip[c]];
       p[c] = v2(a.x, a.y);
       zt[c] = a.z;
     }
-    setup_from(V, p, zt, S);
   } else {
-    setup_view(V, vc, S);
+    project3(V, vc, p, zt);
   }
+  setup_edges(p, zt, area2(p), S);
+  S.x0 = pixel_of(least(p[0].x, p[1].x, p[2].x), V.w);
 }
 
 // The running edge values at pixel (x, y): row start, then column by column
 // from the bounding-box edge (src/Renderer.cpp:240-243).
 __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, float& e2) {
-  row_start(S, y, e1, e2);
-  unpack2(advance2(pack2(e1, e2), pack2(S.n1.x, S.n2.x), x - S.x0), e1, e2);
+  unpack2(advance2(row_start2(S, y), pack2(S.n1.x, S.n2.x), x - S.x0), e1, e2);
 }
 
 // savePPM conversion, src/io.cpp:358-362.
@@ -721,7 +754,8 @@ struct FrameTarget {
   unsigned long long* vis;
   int W;
   bool persp;
-  __device__ unsigned long long* row(uint32_t, int y) const { return vis + (size_t)y * W; }
+  // (a frame has at most 2^28 pixels)
+  __device__ unsigned long long* row(uint32_t, int y) const { return vis + (uint32_t)y * (uint32_t)W; }
   __device__ bool perspective(uint32_t) const { return persp; }
 };
 // ...or, in a batch, the visibility buffer of the triangle's scene (tag).
@@ -734,31 +768,53 @@ struct BatchTarget {
 };
 
 // Raster of a sub-triangle whose bounding box spans at most 4x4 pixels by
-// one thread (src/Renderer.cpp:238-269): the row and column loops have
-// constant bounds and unroll, so the rows' independent edge evaluations
-// interleave (each row still starts from its bounding-box edge and steps
-// column by column).  row(y) gives the visibility words of row y.
-template <typename RowFn>
+// one thread (src/Renderer.cpp:238-269); each row starts from its
+// bounding-box edge and steps column by column.  row(y) gives the visibility
+// words of row y.
+// LIST: the covered cells first (bit 4 * row + column), then one covered pixel
+// per turn of a loop, whose depth and atomic a warp issues as often as its
+// fullest lane has pixels (5-6 for triangles of 1-4 square pixels) instead of
+// once for each of the 16 cells that any lane covers: 10M-triangle soup setup
+// 348 -> 329 us, 16 soups 100 -> 92 us.  The vertex-pass kernels take the
+// plain walk: the list's registers are spilled there (1080p mesh 46.7 ->
+// 50.8 us).
+template <bool LIST, typename RowFn>
 __device__ __forceinline__ void raster_tiny(const Setup& Q, bool persp, uint32_t id, RowFn row_of) {
+  const unsigned long long d = pack2(Q.n1.x, Q.n2.x);
+  unsigned cov = 0;
 #pragma unroll
   for (int r = 0; r < 4; r++) {
     const int y = Q.y0 + r;
-    if (y <= Q.y1) {
-      unsigned long long* row = row_of(y);
-      float e1, e2;
-      row_start(Q, y, e1, e2);
+    if (!LIST && y > Q.y1) break;
+    unsigned long long e = row_start2(Q, y);
 #pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const int x = Q.x0 + c;
-        if (x <= Q.x1 && covered(e1, e2)) {
-          float k0, k1, k2;
-          const float z = frag_depth(Q, persp, e1, e2, k0, k1, k2);
-          if (z < 1e11f) atomicMin(row + x, ((unsigned long long)depth_key(z) << 32) | id);
-        }
-        e1 += Q.n1.x;
-        e2 += Q.n2.x;
+    for (int c = 0; c < 4; c++) {
+      float e1, e2;
+      unpack2(e, e1, e2);
+      if (LIST) {
+        if (covered(e1, e2)) cov |= 1u << (4 * r + c);
+      } else if (Q.x0 + c <= Q.x1 && covered(e1, e2)) {
+        float k0, k1, k2;
+        const float z = frag_depth(Q, persp, e1, e2, k0, k1, k2);
+        if (z < 1e11f) atomicMin(row_of(y) + Q.x0 + c, ((unsigned long long)depth_key(z) << 32) | id);
       }
+      if (c < 3) e = add2(e, d);
     }
+  }
+  if (!LIST) return;
+  cov &= (0x1111u * ((2u << (Q.x1 - Q.x0)) - 1u)) & ((1u << (4 * (Q.y1 - Q.y0 + 1))) - 1u);
+  while (cov) {
+    const int b = __ffs((int)cov) - 1, r = b >> 2, c = b & 3;
+    cov &= cov - 1;
+    const int y = Q.y0 + r;
+    float e1, e2, k0, k1, k2;
+    unsigned long long e = row_start2(Q, y);
+    if (c > 0) e = add2(e, d);
+    if (c > 1) e = add2(e, d);
+    if (c > 2) e = add2(e, d);
+    unpack2(e, e1, e2);
+    const float z = frag_depth(Q, persp, e1, e2, k0, k1, k2);
+    if (z < 1e11f) atomicMin(row_of(y) + Q.x0 + c, ((unsigned long long)depth_key(z) << 32) | id);
   }
 }
 
@@ -776,7 +832,8 @@ __device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t i
   if (m == 0) return;
   const int span = on ? max(S.x1 - S.x0, S.y1 - S.y0) + 1 : 0;
   if (__reduce_max_sync(0xffffffffu, (unsigned)span) <= 4u) {
-    if (on) raster_tiny(S, T.perspective(tag), id, [&](int y) { return T.row(tag, y); });
+    constexpr bool list = std::is_same_v<Rec, SmallRec>;
+    if (on) raster_tiny<list>(S, T.perspective(tag), id, [&](int y) { return T.row(tag, y); });
     return;
   }
   const int n = __popc(m);
@@ -888,11 +945,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
   const bool in = g < F.g.n_tris;
   const DevRenderable& R = renderable<ONE>(F, in ? g : 0u);
   const int t = (int)(g - R.tri_base);
-  int n_sub = 0;
-  if (in) {
-    if (bad_triangle(R.mesh, t)) atomicOr(&F.counters->error_flags, 1u);
-    else n_sub = 1;
-  }
+  int n_sub = in ? 1 : 0;
 #pragma unroll 1
   for (int sub = 0; sub < 2; sub++) {
     if (sub && !__any_sync(0xffffffffu, n_sub == 2)) break;
@@ -902,6 +955,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
       small = box_pixels(S) <= (long long)F.small_max;
       big = !small;
     }
+    if (sub == 0 && n_sub < 0) atomicOr(&F.counters->error_flags, 1u);
     count_triangles(F.counters, small, big, sub == 0 && cut && n_sub > 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
     if (!append_large(F, S, big, id)) small = true;  // rasterised here, as small ones are
@@ -1024,10 +1078,6 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256
   if (g < B.g.n_tris) {
     R = &B.g.rs[find_base(B.g.tri_base, 0, B.g.n_renderables, g)];
     scene = R->scene;
-    if (bad_triangle(R->mesh, (int)(g - R->tri_base))) {
-      atomicOr(&B.counters->error_flags, 1u);
-      R = nullptr;
-    }
   }
   int n_sub = R ? 1 : 0;
 #pragma unroll 1
@@ -1040,6 +1090,7 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256
       small = box_pixels(S) <= (long long)B.small_max;
       big = !small;
     }
+    if (sub == 0 && n_sub < 0) atomicOr(&B.counters->error_flags, 1u);
     count_triangles(B.counters, small, big, sub == 0 && cut && n_sub > 0);
     // record slots: in the first round each warp reserves within the block
     // and the block once globally
@@ -1175,12 +1226,8 @@ __device__ __forceinline__ void raster_items(const BigRec* s_recs, const uint32_
       // the fragment that won a pixel is the one whose id the pixel holds
       // (it was covered and passed the depth test in the first pass)
       float e1, e2;
-      row_start(S, y, e1, e2);
       const float d1 = S.n1.x, d2 = S.n2.x;
-      for (int x = S.x0; x < xs; x++) {
-        e1 += d1;
-        e2 += d2;
-      }
+      unpack2(advance2(row_start2(S, y), pack2(d1, d2), xs - S.x0), e1, e2);
       const uint32_t* row = reinterpret_cast<const uint32_t*>(svis + (y - py0) * TW);  // low words: ids
       for (int x = xs; x <= xe; x++) {
         if (row[2 * (x - px0)] == R.id) s_e[(y - py0) * TW + (x - px0)] = make_float2(e1, e2);

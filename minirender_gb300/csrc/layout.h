@@ -65,6 +65,8 @@ struct View {
   float w, h;
   float P[16];
   int persp;
+  int simple;         // P is a perspective matrix with only the entries [0][0], [0][2], [1][1], [1][2]
+                      // and the z row, and w = -z: see project3
   float znear;
   float lightdir[3];  // placed as render() places it (src/Renderer.cpp:317-320)
   float ambient;

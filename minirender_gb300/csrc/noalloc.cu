@@ -131,11 +131,7 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
   F.v.H = H;
   F.v.w = (float)W;
   F.v.h = (float)H;
-  memcpy(F.v.P, f->projection, sizeof(F.v.P));
-  // Renderer::render, src/Renderer.cpp:317-326.
-  F.v.persp = f->projection[15] == 0;
-  float zn = F.v.persp ? f->projection[11] / (f->projection[10] - 1) : (f->projection[11] + 1) / f->projection[10];
-  F.v.znear = -zn;
+  set_projection(F.v, f->projection);
   if (f->light_is_point) affine(f->view, f->light, F.v.lightdir);
   else normalized(f->light, F.v.lightdir);
   F.v.ambient = f->ambient;

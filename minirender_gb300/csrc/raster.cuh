@@ -42,9 +42,8 @@ __device__ __forceinline__ V3 affine(const float* m, V3 p) {
 // Order-preserving map of a non-NaN float to u32 (-0 and +0 map alike,
 // because the reference's strict z < depth treats them as equal).
 __device__ __forceinline__ uint32_t depth_key(float z) {
-  uint32_t b = __float_as_uint(z);
-  if ((b << 1) == 0) b = 0;
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  const uint32_t b = __float_as_uint(z + 0.0f);  // -0 + 0 is +0
+  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
 }
 
 }  // namespace mrg

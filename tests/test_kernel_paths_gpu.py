@@ -61,3 +61,53 @@ def test_large_triangle_column_segments(product_lib, meshes):
     to a width of 512, then 64, 96, ...) and row blocks of large triangles."""
     st, sc = _boxes((9, 31, 32, 33, 64, 65, 511, 512, 513, 545, 1025, 1300), (8, 31, 32, 33, 65, 90), 1400, 100, meshes)
     _same(_render(st, sc), O.render(st, sc), "boxes")
+
+
+def _skewed():
+    m = np.array(pj.projection_perspective(-0.5, 0.5, -0.4, 0.4, 1, 50), np.float32).reshape(4, 4)
+    m[0, 1] = 0.2
+    return m
+
+
+_PROJECTIONS = {
+    "symmetric": lambda: pj.projection_perspective(-0.5, 0.5, -0.4, 0.4, 1, 50),
+    "off_axis": lambda: pj.projection_perspective(-0.3, 0.6, -0.5, 0.2, 1, 50),
+    "skewed": _skewed,
+    "ortho": lambda: pj.projection_ortho(-4, 5, -3, 4, 1, 50),
+}
+
+
+def _awkward(shared: bool):
+    """Triangles of 1 to 30 pixels, some through the near plane, some with a
+    corner at z = 0, infinite, NaN or near the largest float."""
+    rng = np.random.default_rng(12 + shared)
+    n = 400
+    c = np.stack([rng.uniform(-6, 6, n), rng.uniform(-5, 5, n), -rng.uniform(0.5, 40, n)], 1)
+    v = (c[:, None] + rng.normal(0, 0.4, (n, 3, 3)) * [1, 1, 0.6]).astype(np.float32)
+    for k, bad in enumerate((0.0, -0.0, np.inf, -np.inf, np.nan, 3e38, -3e38, 1e-40)):
+        for axis in range(3):
+            v[3 * k + axis + 40, rng.integers(0, 3), axis] = bad
+    v[100, :, 2] = 0.0
+    v = v.reshape(-1, 3)
+    idx = np.arange(3 * n, dtype=np.int32)
+    if shared:  # neighbouring triangles use each other's corners
+        idx = np.concatenate([idx, np.roll(idx, 1), np.roll(idx, 2)]).astype(np.int32)
+    nrm = rng.normal(size=(3 * n, 3)).astype(np.float32)
+    sc = S.Scene()
+    sc.add(S.TriMesh(v, nrm, idx, normalsI=idx, material=S.Material(shininess=8)))
+    return sc
+
+
+@pytest.mark.parametrize("shared", [False, True], ids=["soup", "shared"])
+@pytest.mark.parametrize("projection", sorted(_PROJECTIONS))
+def test_projection_forms(product_lib, projection, shared):
+    """The short projection of perspective matrices without skew, its general
+    form, and the corners that must take the general form."""
+    st = FrameState(width=120, height=90, projection=_PROJECTIONS[projection](),
+                    light=np.array([0.2, 0.4, 1], np.float32))
+    sc = _awkward(shared)
+    ref = O.render(st, sc)
+    assert (ref["ids"] != 0xFFFFFFFF).sum() > 500
+    got = _render(st, sc)
+    assert np.array_equal(got["ids"], ref["ids"])
+    assert np.array_equal(got["depth"].view(np.uint32), ref["depth"].view(np.uint32))
