@@ -166,7 +166,7 @@ typedef struct mr_stats {
     int64_t rasterised;       /* sub-triangles past cull and reject */
     int64_t small_direct;     /* rasterised in the setup kernel */
     int64_t binned;           /* large sub-triangles (records) */
-    int64_t bin_entries;      /* their work items: 32-row blocks (mr_render),
+    int64_t bin_entries;      /* their work items: blocks of 32 rows by a column segment (mr_render),
                                  (tile, sub-triangle) pairs (mr_render_batch) */
     int64_t error_flags;      /* nonzero: MR_E_BAD_INDEX seen */
     float stage_ms[8];        /* when profiling: clear+vertex, setup, large raster, -, resolve */
@@ -253,8 +253,9 @@ typedef struct mr_batch_scene {
     int32_t n_renderables;
 } mr_batch_scene;
 
-/* Tile edge (8/16/32), threads per tile block (64/128/256) and records
- * staged per pass in shared memory (16..256) for mr_render_batch. */
+/* Tile edge (8/16/32) and threads per block (64/128/256) for
+ * mr_render_batch.  `chunk` (16..256) is validated and kept for source
+ * compatibility; records are no longer staged in shared memory. */
 MR_API int mr_set_batch_tuning(mr_ctx* ctx, int tile, int threads, int chunk);
 /* As mr_set_batch_tuning with a rectangular screen tile: power-of-two sides,
  * width 4..256, height 2..64, 64..4096 pixels.  Wide tiles shorten the

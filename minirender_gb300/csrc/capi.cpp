@@ -970,7 +970,7 @@ static int enqueue_batch(mr_ctx* c, BatchSlot& B, cudaStream_t st, cudaEvent_t* 
     CK(cudaEventRecord(B.staged, st), "staging event");
   CK(cudaMemsetAsync(B.d_cnt, 0, sizeof(Counters), st), "counter reset");
   CK(cudaMemsetAsync(B.tiles.p, 0, sizeof(uint32_t) * (3 * (size_t)B.P.n_tiles + 1), st), "tile reset");
-  CK(launch_batch(B.P, B.threads, B.grid, B.block_sums.p, st, ev), "batch launch");
+  CK(launch_batch(B.P, B.threads, B.grid, st, ev), "batch launch");
   return MR_OK;
 }
 
@@ -1027,7 +1027,7 @@ int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEven
 void BatchSlot::release() {
   rs.release(); bases.release(); scenes.release(); stb.release(); va.release(); vn.release();
   vb.release(); recs.release(); rec_scene.release(); tiles.release(); bins.release();
-  block_sums.release(); out8.release(); outd.release(); outi.release(); vis.release();
+  out8.release(); outd.release(); outi.release(); vis.release();
   if (h_rs) cudaFreeHost(h_rs);
   if (h_u32) cudaFreeHost(h_u32);
   if (h_scenes) cudaFreeHost(h_scenes);
@@ -1121,9 +1121,8 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   if (B.small_max > 0) CK(B.vis.ensure(pixels), "batch visibility");
   if (B.bins.cap < std::max<size_t>((size_t)1 << 20, 2 * tris))
     CK(B.bins.ensure(std::max<size_t>((size_t)1 << 20, 2 * tris)), "batch bins");
-  int grid = batch_grid(TW, TH, B.chunk, B.threads, vertex_pass);
+  int grid = batch_grid(TW, TH, B.threads, vertex_pass);
   if (grid <= 0) return fail(c, MR_E_INVALID, "batch tuning does not fit on the device");
-  CK(B.block_sums.ensure((size_t)grid + 1), "batch scan");
   uint32_t tri = 0, vb = 0, nb = 0, tile_base = 0;
   for (int32_t s = 0; s < n_scenes; s++) {
     const mr_frame* f = &sc[s].frame;
@@ -1213,7 +1212,6 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   P.n_tiles = tile_base;
   P.tile_w = TW;
   P.tile_h = TH;
-  P.chunk = B.chunk;
   P.small_max = B.small_max;
   P.vis = B.small_max > 0 ? B.vis.p : nullptr;
   P.n_px = (size_t)pixels;

@@ -17,9 +17,8 @@ namespace mrg {
 cudaError_t launch_validate(const DevMesh& M, uint32_t* bad, cudaStream_t st);
 cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev, cudaEvent_t staged = nullptr);
 cudaError_t launch_range(int W, int H, const Mat4& P, const float* depth, float* xyz, cudaStream_t st);
-cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* block_sums, cudaStream_t st,
-                         cudaEvent_t* ev);
-int batch_grid(int tile_w, int tile_h, int chunk, int threads, bool pre);
+cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream_t st, cudaEvent_t* ev);
+int batch_grid(int tile_w, int tile_h, int threads, bool pre);
 // Tile shapes k_batch takes: power-of-two sides, 64..4096 pixels (whole warps).
 inline bool batch_tile_ok(int tw, int th) {
   auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
@@ -105,7 +104,7 @@ struct BatchSlot {
   DevBuf<float4> va, vn;
   DevBuf<float2> vb;
   DevBuf<BigRec> recs;
-  DevBuf<uint32_t> rec_scene, tiles, bins, block_sums;
+  DevBuf<uint32_t> rec_scene, tiles, bins;
   DevBuf<unsigned long long> vis;
   DevBuf<uint8_t> out8;
   DevBuf<float> outd;

@@ -25,12 +25,12 @@
 //   k_setup_batch (sub-triangles with a bounding box of at most small_max
 //   pixels rasterised into their scene's visibility words, larger ones
 //   become records counted into the scene's tiles), then k_batch: one
-//   cooperative, persistent launch -- scan, scatter, and a dynamically
-//   scheduled loop over all tiles of all scenes that rasterises each tile's
-//   records into shared memory (seeded with the small triangles' words),
-//   captures the winners' edge values and resolves + shades its pixels in
-//   place.  The PRE template flag is false for triangle soups: no vertex
-//   pass, kernels transform corners themselves.
+//   cooperative, persistent launch -- list ranges, scatter, and a dynamically
+//   scheduled loop over strips of all tiles of all scenes, one warp each, that
+//   rasterises the tile's records into shared memory (seeded with the small
+//   triangles' words) and resolves + shades the strip's pixels in place.  The
+//   PRE template flag is false for triangle soups: no vertex pass, kernels
+//   transform corners themselves.
 // Also: k_validate (index checks at upload), k_range (getRangeImage,
 // src/Renderer.cpp:388-415).
 //
@@ -371,6 +371,54 @@ __device__ __forceinline__ void walk_row(const Setup& S, bool persp, uint32_t id
       float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
       if (z < 1e11f) emit(x, ((unsigned long long)depth_key(z) << 32) | id, e1, e2);
     }
+    e = add2(e, d);
+  }
+}
+
+// Columns S.x0 + lo .. S.x0 + hi outside of which the row that starts with
+// edge values (e1, e2) covers nothing: each edge function is a line whose
+// crossing of zero bounds the covered run, give or take the rounding of the
+// running sums.  err bounds that rounding (a column's sum is off by at most
+// half a unit in the last place of the largest edge value per column, taken
+// four times over), so the walk may start and stop there and still visits
+// every pixel the reference covers.  Values that are not finite bound nothing.
+__device__ __forceinline__ void edge_bound(float e, float g, float err, float& lo, float& hi) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(g));
+  const float q = -e * r, m = err * fabsf(r) + (fabsf(q) * 2e-6f + 1e-3f);
+  if (g > 0) lo = fmaxf(lo, q - m);
+  if (g < 0) hi = fminf(hi, q + m);
+}
+__device__ __forceinline__ void covered_run(const Setup& S, unsigned long long e, int cols, int& lo, int& hi) {
+  float e1, e2;
+  unpack2(e, e1, e2);
+  const float d1 = S.n1.x, d2 = S.n2.x, w = (float)cols;
+  const float size = (fabsf(e1) + fabsf(e2) + 1.f) + w * (fabsf(d1) + fabsf(d2));
+  const float err = (w + 8.f) * size * 2.4e-7f;
+  float a = 0.f, b = w;
+  edge_bound(e1, d1, err, a, b);
+  edge_bound(e2, d2, err, a, b);
+  edge_bound(1.f - e1 - e2, -(d1 + d2), err, a, b);
+  lo = (int)ceilf(fminf(a, w));
+  hi = (int)floorf(fmaxf(b, -1.f));
+}
+
+// The columns of xs..xe of row y that the row may cover, in order, with their
+// running edge values (which step column by column from S.x0).
+template <typename Visit>
+__device__ __forceinline__ void walk_span(const Setup& S, int y, int xs, int xe, Visit visit) {
+  const unsigned long long d = pack2(S.n1.x, S.n2.x);
+  unsigned long long e = row_start2(S, y);
+  int lo, hi;
+  covered_run(S, e, xe - S.x0 + 1, lo, hi);
+  xs = max(xs, S.x0 + lo);
+  xe = min(xe, S.x0 + hi);
+  if (xs > xe) return;
+  e = advance2(e, d, xs - S.x0);
+  for (int x = xs; x <= xe; x++) {
+    float e1, e2;
+    unpack2(e, e1, e2);
+    visit(x, e1, e2);
     e = add2(e, d);
   }
 }
@@ -980,8 +1028,14 @@ __device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, u
   if (y > S.y1) return;
   const int xs = S.x0 + c * w;
   unsigned long long* row = F.vis + (size_t)y * F.v.W;
-  walk_row(S, persp, R.id, y, xs, min(xs + w - 1, S.x1),
-           [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
+  const uint32_t id = R.id;
+  walk_span(S, y, xs, min(xs + w - 1, S.x1), [&](int x, float e1, float e2) {
+    if (covered(e1, e2)) {
+      float k0, k1, k2;
+      const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
+      if (z < 1e11f) atomicMin(row + x, ((unsigned long long)depth_key(z) << 32) | id);
+    }
+  });
 }
 
 __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
@@ -1123,201 +1177,107 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256
   }
 }
 
-// Renderables per scene whose triangle bases k_batch keeps in shared memory
-// (larger scenes search the global table).
-constexpr int kBatchTbMax = 256;
+// Rows of a tile that one warp of k_batch takes at a time: the strip holds at
+// most 256 pixels (8 a lane).
+__host__ __device__ inline int strip_rows(int tw, int th) { return th < 256 / tw ? th : 256 / tw; }
+// Words of shared memory between a strip's rows: rows of 16 pixels and more
+// are skewed so the same column of several rows falls in different banks.
+__host__ __device__ inline int strip_pitch(int tw) { return tw >= 16 ? tw + 4 : tw; }
 
-// Exclusive prefix sum of v over the threads of the block (blockDim.x a
-// multiple of 32, at most 1024); tot = the block's sum.  Every thread of the
-// block must call it; s_part holds 33 words.
-__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_part, uint32_t& tot) {
-  const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
-  uint32_t inc = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += u;
-  }
-  __syncthreads();  // s_part free from a previous call
-  if (lane == 31) s_part[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    const uint32_t p = lane < nw ? s_part[lane] : 0u;
-    uint32_t pi = p;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, pi, o);
-      if (lane >= o) pi += u;
+// The records bins[s..e) of a tile, rasterised by one warp into its strip
+// (px0..px1, py0..py1): 32 records at a time, the (record, row) pairs inside
+// the strip enumerated by a prefix sum and taken one per lane.
+// The fragments are merged into the strip's visibility words.
+__device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, uint32_t e, int px0, int py0, int px1,
+                                             int py1, bool persp, int pitch, unsigned long long* svis) {
+  const int lane = (int)(threadIdx.x & 31);
+#pragma unroll 1
+  for (uint32_t c0 = s; c0 < e; c0 += 32) {
+    uint32_t rec = 0;
+    int rows = 0;
+    if (c0 + lane < e) {
+      rec = B.bins[c0 + lane];
+      const int4 box = *reinterpret_cast<const int4*>(&B.recs[rec].x0);  // x0, y0, x1, y1
+      if (max(box.x, px0) <= min(box.z, px1)) rows = max(0, min(box.w, py1) - max(box.y, py0) + 1);
     }
-    if (lane < nw) s_part[lane] = pi - p;
-    if (lane == 31) s_part[32] = pi;
-  }
-  __syncthreads();
-  tot = s_part[32];
-  return s_part[w] + inc - v;
-}
-
-// Stages the tile's records bins[c0 .. c0+cn) in shared memory with the
-// exclusive prefix of the rows each covers inside the tile (px0..px1,
-// py0..py1): s_off[cn] is the number of (record, row) items.  Block-wide.
-__device__ __forceinline__ void stage_chunk(const BigRec* recs, const uint32_t* bins, uint32_t c0, uint32_t cn,
-                                            int px0, int py0, int px1, int py1, BigRec* s_recs,
-                                            uint32_t* s_off, int* s_run = nullptr) {
-  __syncthreads();  // the previous pass over s_recs / s_off is done
-  int run = 0;
-  for (uint32_t i = threadIdx.x; i < cn; i += blockDim.x) {
-    const BigRec r = recs[bins[c0 + i]];
-    s_recs[i] = r;
-    const int ys = max(r.y0, py0), ye = min(r.y1, py1);
-    const bool hit = ys <= ye && max(r.x0, px0) <= min(r.x1, px1);
-    s_off[i] = hit ? (uint32_t)(ye - ys + 1) : 0u;
-    if (hit) run = max(run, min(r.x1, px1) - r.x0);
-  }
-  if (s_run && run) atomicMax(s_run, run);
-  __syncthreads();
-  if (threadIdx.x < 32) {  // one warp scans: each lane a contiguous run
-    const int lane = (int)threadIdx.x;
-    const uint32_t per = (cn + 31) / 32;
-    const uint32_t b = min(cn, (uint32_t)lane * per), e = min(cn, b + per);
-    uint32_t sum = 0;
-    for (uint32_t i = b; i < e; i++) sum += s_off[i];
-    uint32_t inc = sum;
+    int inc = rows;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += u;
     }
-    uint32_t run = inc - sum;
-    for (uint32_t i = b; i < e; i++) {
-      const uint32_t c = s_off[i];
-      s_off[i] = run;
-      run += c;
-    }
-    if (lane == 31) s_off[cn] = inc;
-  }
-  __syncthreads();
-}
-
-// The (record, row) items of a staged chunk, one per thread: CAPTURE=false
-// merges the fragments into the shared visibility tile; CAPTURE=true (after
-// every record of the tile has been merged) stores, for each pixel, the
-// running edge values of the fragment that won it, so the resolve needs no
-// replay.  A pixel's winning word is unique (it holds the sub-triangle id).
-// Tiles whose records could make a pixel replay its winner's edge functions
-// over more columns than this capture the winners' edge values (pass 2).
-constexpr int kReplayMax = 256;
-
-template <bool CAPTURE>
-__device__ __forceinline__ void raster_items(const BigRec* s_recs, const uint32_t* s_off, uint32_t cn, int TW,
-                                             int px0, int py0, int px1, int py1, bool persp,
-                                             unsigned long long* svis, float2* s_e) {
-  const uint32_t total = s_off[cn];
-  for (uint32_t it = threadIdx.x; it < total; it += blockDim.x) {
-    int lo = 0, hi = (int)cn;  // s_off[lo] <= it < s_off[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (s_off[mid] <= it) lo = mid; else hi = mid;
-    }
-    const BigRec& R = s_recs[lo];
-    const int y = max(R.y0, py0) + (int)(it - s_off[lo]);
-    const int xs = max(R.x0, px0), xe = min(R.x1, px1);
-    const Setup S = rec_setup(R);
-    if (CAPTURE) {
-      // the fragment that won a pixel is the one whose id the pixel holds
-      // (it was covered and passed the depth test in the first pass)
-      float e1, e2;
-      const float d1 = S.n1.x, d2 = S.n2.x;
-      unpack2(advance2(row_start2(S, y), pack2(d1, d2), xs - S.x0), e1, e2);
-      const uint32_t* row = reinterpret_cast<const uint32_t*>(svis + (y - py0) * TW);  // low words: ids
-      for (int x = xs; x <= xe; x++) {
-        if (row[2 * (x - px0)] == R.id) s_e[(y - py0) * TW + (x - px0)] = make_float2(e1, e2);
-        e1 += d1;
-        e2 += d2;
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll 1
+    for (int b = 0; b < total; b += 32) {
+      const int i = b + lane;
+      int own = 0;  // the lane whose record row i belongs to
+#pragma unroll
+      for (int step = 16; step; step >>= 1)
+        if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= i) own += step;
+      const int k = i - __shfl_sync(0xffffffffu, inc - rows, own);
+      const uint32_t r = __shfl_sync(0xffffffffu, rec, own);
+      if (i < total) {
+        const BigRec& R = B.recs[r];
+        const Setup S = rec_setup(R);
+        const int y = max(S.y0, py0) + k;
+        const uint32_t id = R.id;
+        unsigned long long* row = svis + (y - py0) * pitch - px0;
+        walk_span(S, y, max(S.x0, px0), min(S.x1, px1), [&](int x, float e1, float e2) {
+          if (covered(e1, e2)) {
+            float k0, k1, k2;
+            const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
+            if (z < 1e11f) atomicMin(row + x, ((unsigned long long)depth_key(z) << 32) | id);
+          }
+        });
       }
-    } else {
-      walk_row(S, persp, R.id, y, xs, xe, [&](int x, unsigned long long v, float, float) {
-        atomicMin(svis + (y - py0) * TW + (x - px0), v);
-      });
     }
+    __syncwarp();
   }
 }
 
 // The batch's persistent kernel (cooperative launch, grid-wide barriers):
-//   1. exclusive scan of the per-tile counts (per-block segments, then one
-//      block scanning the block sums), 2. scatter record indices into tile
-//      lists, 3. tiles of all scenes taken from a work counter: the tile's
-//      visibility words start from the scene's small-triangle words; its
-//      records are staged in shared memory `chunk` at a time and rasterised
-//      (pass 1), walked again to capture each winner's edge values (pass 2),
-//      then every pixel of the tile is resolved, shaded and written to its
-//      scene's outputs.
-// MINB: blocks of 256 threads per SM the register allocation must allow
-// (2: up to 128 registers per thread, for 64-thread blocks; 4: up to 64, so
-// that 128- and 256-thread blocks keep enough warps resident).  At 64
-// registers the vertex-pass instance spills 216 bytes per thread; an 80-
-// register instance (3 blocks) that spills 36 was measured slower on the
-// 256-scene batch (fused stage 3.62 vs 3.37 ms), so the warps win.
+//   1. a range of the list for each tile's records, 2. record indices
+//   scattered into the ranges, 3. the tiles of all scenes, in strips of at
+//   most 256 pixels, one warp each: the strip's visibility words start from
+//   the scene's small-triangle words; its records are rasterised into shared
+//   memory, then every pixel is resolved, shaded and written to its scene's
+//   outputs.
+// A strip is one warp's alone, so nothing in it waits for other warps; a block
+// takes groups of strips from a work counter and its warps share a group
+// through a counter in shared memory (neighbouring strips read the same
+// records and vertices).  With a block per tile, block barriers between the
+// phases were 38 % of the warps' time: 256 scenes 2934 -> 2670 us, 16 soups 260
+// -> 240, eight 3840x2160 scenes in 16x16 tiles 5037 -> 3558.  (The old form
+// also captured the winners' edge values where a replay could pass 256
+// columns; with packed adds the replay is the cheaper.)  Groups of two strips
+// a warp: one gives up the shared reads (2822 us), four leave a tail (2723).
+// MINB: blocks of 256 threads per SM the register allocation must allow.
 template <int MINB, bool PRE>
-__global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B, uint32_t* block_sums) {
+__global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int TW = B.tile_w, TH = B.tile_h, TP = TW * TH;
-  unsigned long long* svis = (unsigned long long*)smem;
-  float2* s_e = (float2*)(smem + (size_t)TP * sizeof(unsigned long long));
-  BigRec* s_recs = (BigRec*)(smem + (size_t)TP * (sizeof(unsigned long long) + sizeof(float2)));
-  uint32_t* s_off = (uint32_t*)(s_recs + B.chunk);  // chunk + 1 entries
   __shared__ float s_dec[256];
-  __shared__ uint32_t s_part[33];
-  __shared__ uint32_t s_tile;
-  __shared__ int s_run;  // longest column replay a pixel of the tile could need
-  __shared__ View s_view;
-  __shared__ int s_meta[8];
-  __shared__ uint32_t s_tb[kBatchTbMax];
-  __shared__ int s_tb_scene;
-  __shared__ uint8_t* s_out8;
-  __shared__ float* s_outd;
-  __shared__ uint32_t* s_outi;
-  __shared__ const unsigned long long* s_invis;  // small triangles' visibility words of the scene
+  __shared__ unsigned long long s_first;
+  __shared__ uint32_t s_next;
+  __shared__ SceneRec s_scene[8];
   cg::grid_group grid = cg::this_grid();
   const uint32_t nb = gridDim.x, nt = blockDim.x;
+  const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
+  const int TW = B.tile_w, TH = B.tile_h, SH = strip_rows(TW, TH), pitch = strip_pitch(TW), lw = __ffs(TW) - 1;
+  unsigned long long* svis = reinterpret_cast<unsigned long long*>(smem) + (size_t)w * SH * pitch;
   for (uint32_t i = threadIdx.x; i < 256; i += nt) s_dec[i] = (float)i / 255.0f;
-  if (threadIdx.x == 0) s_tb_scene = -1;
-  // 1. scan: block b owns tiles [b*seg, (b+1)*seg)
-  const uint32_t seg = (B.n_tiles + nb - 1) / nb;
-  const uint32_t t0 = min(B.n_tiles, blockIdx.x * seg), t1 = min(B.n_tiles, t0 + seg);
-  {
-    uint32_t sum = 0;
-    for (uint32_t i = t0 + threadIdx.x; i < t1; i += nt) sum += B.tile_count[i];
-    uint32_t tot;
-    block_scan(sum, s_part, tot);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
-  }
-  grid.sync();
-  if (blockIdx.x == 0) {  // exclusive scan of the block sums, by the whole block
-    uint32_t run = 0;
-    for (uint32_t b0 = 0; b0 < nb; b0 += nt) {
-      const uint32_t i = b0 + threadIdx.x;
-      const uint32_t v = i < nb ? block_sums[i] : 0u;
-      uint32_t tot;
-      const uint32_t ex = block_scan(v, s_part, tot);
-      if (i < nb) block_sums[i] = run + ex;
-      run += tot;
+  // 1. the tiles' ranges, in any order: one atomic per warp of tiles
+  for (uint32_t t0 = (blockIdx.x * nt + threadIdx.x) & ~31u; t0 < B.n_tiles; t0 += nb * nt) {
+    const uint32_t t = t0 + lane, v = t < B.n_tiles ? B.tile_count[t] : 0u;
+    uint32_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
     }
-    if (threadIdx.x == 0) {
-      B.tile_start[B.n_tiles] = run;
-      B.counters->bin_needed = run;
-    }
-  }
-  grid.sync();
-  {
-    uint32_t run = block_sums[blockIdx.x];
-    for (uint32_t b0 = t0; b0 < t1; b0 += nt) {
-      const uint32_t i = b0 + threadIdx.x;
-      const uint32_t v = i < t1 ? B.tile_count[i] : 0u;
-      uint32_t tot;
-      const uint32_t ex = block_scan(v, s_part, tot);
-      if (i < t1) B.tile_start[i] = run + ex;
-      run += tot;
-    }
+    uint32_t base = 0;
+    if (lane == 31 && inc) base = atomicAdd(&B.counters->bin_needed, inc);
+    base = __shfl_sync(0xffffffffu, base, 31);
+    if (t < B.n_tiles) B.tile_start[t] = base + inc - v;
   }
   grid.sync();
   // 2. scatter
@@ -1335,128 +1295,102 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B, uint32_t* bl
       }
   }
   grid.sync();
-  // 3. tiles
+  // 3. strips, in groups of two per warp of the block
+  const uint32_t strips = (uint32_t)(TH / SH), warps = nt >> 5;
+  const unsigned long long units = (unsigned long long)B.n_tiles * strips;
+  const uint32_t group = 2u * warps;
   for (;;) {
     __syncthreads();
-    if (threadIdx.x < 32) {  // warp 0 takes the next tile and loads its scene
-      const int lane = (int)threadIdx.x;
-      uint32_t t = 0;
-      if (lane == 0) t = atomicAdd(&B.counters->work_next, 1u);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      if (t < B.n_tiles) {
-        // the scene: the last j with scene_tile_base[j] <= t (bases ascending)
-        unsigned cnt = 0;
-        for (int j = 1 + lane; j < B.n_scenes; j += 32) cnt += B.scene_tile_base[j] <= t;
-        const int sc = (int)__reduce_add_sync(0xffffffffu, cnt);
-        const SceneRec& SR = B.scenes[sc];
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&SR.v);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(&s_view);
-        for (int k = lane; k < (int)(sizeof(View) / 4); k += 32) dst[k] = src[k];
-        if (lane == 0) {
-          s_meta[0] = sc;
-          s_meta[1] = (int)(t - SR.tile_base);
-          s_meta[2] = SR.tiles_x;
-          s_meta[3] = (int)SR.rs_begin;
-          s_meta[4] = (int)SR.rs_end;
-          s_meta[5] = (int)(2u * B.g.tri_base[SR.rs_begin]);  // ids are reported per scene
-          // the tile's list (bins truncated at capacity on overflow)
-          s_meta[6] = (int)min(B.tile_start[t], B.bin_cap);
-          s_meta[7] = (int)min(B.tile_start[t + 1], B.bin_cap);
-          s_out8 = SR.rgb8;
-          s_outd = SR.depth;
-          s_outi = SR.ids;
-          s_invis = SR.vis;
+    if (threadIdx.x == 0) {
+      s_first = (unsigned long long)atomicAdd(&B.counters->work_next, 1u) * group;
+      s_next = 0;
+    }
+    __syncthreads();
+    const unsigned long long first = s_first;
+    if (first >= units) break;
+    const uint32_t n_units = (uint32_t)min((unsigned long long)group, units - first);
+    for (;;) {
+      uint32_t k = 0;
+      if (lane == 0) k = atomicAdd(&s_next, 1u);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= n_units) break;
+      const uint32_t t = (uint32_t)((first + k) / strips), strip = (uint32_t)((first + k) % strips);
+      // the scene: the last j with scene_tile_base[j] <= t (bases ascending,
+      // the first 0), 32 candidates at a time
+      int sc = 0;
+      for (int n = B.n_scenes; n > 1;) {
+        const int step = (n + 31) >> 5, j = sc + lane * step;
+        const unsigned m = __ballot_sync(0xffffffffu, lane * step < n && B.scene_tile_base[j] <= t);
+        const int at = (31 - __clz((int)m)) * step;
+        sc += at;
+        n = min(step, n - at);
+      }
+      __syncwarp();
+      {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(&B.scenes[sc]);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(&s_scene[w]);
+        for (int i = lane; i < (int)(sizeof(SceneRec) / 4); i += 32) dst[i] = src[i];
+      }
+      __syncwarp();
+      const SceneRec& C = s_scene[w];
+      const int lt = (int)(t - C.tile_base), ty = lt / C.tiles_x, tx = lt - ty * C.tiles_x;
+      const int px0 = tx * TW, py0 = ty * TH + (int)strip * SH;
+      const int px1 = min(px0 + TW, C.v.W) - 1, py1 = min(py0 + SH, C.v.H) - 1;
+      if (py0 > py1) continue;
+      const bool persp = C.v.persp != 0;
+      // the tile's list (truncated at capacity on overflow)
+      const uint32_t ls = min(B.tile_start[t], B.bin_cap), le = min(B.tile_start[t] + B.tile_count[t], B.bin_cap);
+      if (ls < le) {
+        // the strip starts from the small triangles' words (or empty), copied
+        // with cp.async so all of a lane's loads are in flight at once
+        for (int i = lane; i < SH * TW; i += 32) {
+          const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
+          if (C.vis && x <= px1 && y <= py1) cp_async8(&svis[cy * pitch + cx], &C.vis[(uint32_t)y * (uint32_t)C.v.W + x]);
+          else svis[cy * pitch + cx] = VIS_EMPTY;
         }
+        cp_async_wait_all();
+        __syncwarp();
+        raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
+        __syncwarp();
       }
-      if (lane == 0) s_tile = t;
-    }
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    if (tile >= B.n_tiles) break;
-    const int n_rs = s_meta[4] - s_meta[3];
-    const bool tb_shared = n_rs <= kBatchTbMax;
-    if (tb_shared && s_tb_scene != s_meta[0]) {  // uniform: read after the barrier above
-      for (int i = threadIdx.x; i < n_rs; i += nt) s_tb[i] = B.g.tri_base[s_meta[3] + i];
-      __syncthreads();
-      if (threadIdx.x == 0) s_tb_scene = s_meta[0];
-    }
-    const int lt = s_meta[1], tx = lt % s_meta[2], ty = lt / s_meta[2];
-    const int px0 = tx * TW, py0 = ty * TH;
-    const int px1 = min(px0 + TW, s_view.W) - 1, py1 = min(py0 + TH, s_view.H) - 1;
-    // the tile starts from the small triangles' words (or empty), copied
-    // with cp.async so all of a thread's loads are in flight at once (made
-    // visible to the block by the barrier that opens pass 1)
-    for (int i = threadIdx.x; i < TP; i += nt) {
-      const int x = px0 + i % TW, y = py0 + i / TW;
-      if (s_invis && x <= px1 && y <= py1) cp_async8(&svis[i], &s_invis[(size_t)y * s_view.W + x]);
-      else svis[i] = VIS_EMPTY;
-    }
-    cp_async_wait_all();
-    const uint32_t s = (uint32_t)s_meta[6], e = (uint32_t)s_meta[7];
-    const bool persp = s_view.persp != 0;
-    const uint32_t nck = (e - s + (uint32_t)B.chunk - 1) / (uint32_t)B.chunk;
-    if (threadIdx.x == 0) s_run = 0;  // (ordered by stage_chunk's first barrier)
-    for (uint32_t c = 0; c < nck; c++) {  // pass 1: depth test
-      const uint32_t c0 = s + c * (uint32_t)B.chunk, cn = min((uint32_t)B.chunk, e - c0);
-      stage_chunk(B.recs, B.bins, c0, cn, px0, py0, px1, py1, s_recs, s_off, &s_run);
-      raster_items<false>(s_recs, s_off, cn, TW, px0, py0, px1, py1, persp, svis, s_e);
-    }
-    // pass 2, the winners' edge values, only where a replay from the
-    // bounding-box edge could be long: otherwise the resolve replays (cheaper
-    // than walking every record of the tile a second time)
-    const bool captured = nck > 0 && s_run > kReplayMax;
-    if (captured) {
-      // captured edge values start as NaN (no fragment with a NaN edge value
-      // is ever written: its depth is NaN and fails z < 1e11f); ordered
-      // before the capture by the barrier that opens each pass-2 chunk
-      for (int i = threadIdx.x; i < TP; i += nt) s_e[i] = make_float2(__int_as_float(0x7fc00000), 0.f);
-      for (uint32_t c = 0; c < nck; c++) {
-        const uint32_t c0 = s + c * (uint32_t)B.chunk, cn = min((uint32_t)B.chunk, e - c0);
-        if (nck > 1) stage_chunk(B.recs, B.bins, c0, cn, px0, py0, px1, py1, s_recs, s_off);
-        else __syncthreads();
-        raster_items<true>(s_recs, s_off, cn, TW, px0, py0, px1, py1, persp, svis, s_e);
-      }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < TP; i += nt) {
-      const int x = px0 + i % TW, y = py0 + i / TW;
-      if (x > px1 || y > py1) continue;
-      const unsigned long long vw = svis[i];
-      V3 value, normal;
-      float depth;
-      const uint32_t id = (uint32_t)vw;
-      if (vw == VIS_EMPTY) {
-        value = v3(s_view.bg[0], s_view.bg[1], s_view.bg[2]);
-        depth = 1e11f;
-      } else {
-        int ip[3];
-        Vtx vc[3];
-        bool clipped;
-        const DevRenderable& R = B.g.rs[tb_shared ? s_meta[3] + find_base(s_tb, 0, n_rs, id >> 1)
-                                                  : find_base(B.g.tri_base, s_meta[3], s_meta[4], id >> 1)];
-        winner_tri<PRE>(s_view, B.g, R, id, ip, vc, clipped);
-        Setup S;
-        float e1, e2;
-        const float2 ee = captured ? s_e[i] : make_float2(__int_as_float(0x7fc00000), 0.f);
-        winner_setup<PRE>(s_view, B.g, R, ip, vc, clipped, S);
-        if (ee.x == ee.x) {  // won by a record of this tile: edge values captured
-          e1 = ee.x;
-          e2 = ee.y;
-        } else {  // won by a small triangle rasterised in the setup kernel
+      const bool direct = ls >= le;
+      const uint32_t id0 = 2u * B.g.tri_base[C.rs_begin];  // ids are reported per scene
+#pragma unroll 1
+      for (int i = lane; i < SH * TW; i += 32) {
+        const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
+        if (x > px1 || y > py1) continue;
+        const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)x;
+        const unsigned long long vw = !direct ? svis[cy * pitch + cx] : C.vis ? C.vis[px] : VIS_EMPTY;
+        V3 value, normal;
+        float depth;
+        const uint32_t id = (uint32_t)vw;
+        if (vw == VIS_EMPTY) {
+          value = v3(C.v.bg[0], C.v.bg[1], C.v.bg[2]);
+          depth = 1e11f;
+        } else {
+          int ip[3];
+          Vtx vc[3];
+          bool clipped;
+          const DevRenderable& R = B.g.rs[find_base(B.g.tri_base, (int)C.rs_begin, (int)C.rs_end, id >> 1)];
+          winner_tri<PRE>(C.v, B.g, R, id, ip, vc, clipped);
+          Setup S;
+          winner_setup<PRE>(C.v, B.g, R, ip, vc, clipped, S);
+          float e1, e2;
           replay(S, x, y, e1, e2);
+          float k0, k1, k2;
+          depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
+          shade(C.v, R, vc, k0, k1, k2, s_dec, value, normal);
         }
-        float k0, k1, k2;
-        depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
-        shade(s_view, R, vc, k0, k1, k2, s_dec, value, normal);
+        if (C.rgb8) {
+          uint8_t* o8 = C.rgb8 + 3 * (size_t)px;
+          o8[0] = to_byte(value.x);
+          o8[1] = to_byte(value.y);
+          o8[2] = to_byte(value.z);
+        }
+        if (C.depth) C.depth[px] = depth;
+        if (C.ids) C.ids[px] = vw == VIS_EMPTY ? MR_NO_TRIANGLE : id - id0;
       }
-      const size_t px = (size_t)y * s_view.W + x;
-      if (uint8_t* o8 = s_out8) {
-        o8[3 * px + 0] = to_byte(value.x);
-        o8[3 * px + 1] = to_byte(value.y);
-        o8[3 * px + 2] = to_byte(value.z);
-      }
-      if (s_outd) s_outd[px] = depth;
-      if (s_outi) s_outi[px] = vw == VIS_EMPTY ? MR_NO_TRIANGLE : id - (uint32_t)s_meta[5];
+      __syncwarp();  // the strip's words may be overwritten
     }
   }
 }
@@ -1583,10 +1517,9 @@ cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev,
   return pre ? launch_stages<true, false>(F, st, ev, staged) : launch_stages<false, false>(F, st, ev, staged);
 }
 
-size_t batch_smem(int tile_w, int tile_h, int chunk) {
-  // visibility words + captured edge values per pixel, staged records, row prefix
-  return (size_t)tile_w * tile_h * (sizeof(unsigned long long) + sizeof(float2)) + (size_t)chunk * sizeof(BigRec) +
-         (size_t)(chunk + 1) * sizeof(uint32_t);
+size_t batch_smem(int tile_w, int tile_h, int threads) {
+  // visibility words of one strip per warp
+  return (size_t)(threads / 32) * strip_rows(tile_w, tile_h) * strip_pitch(tile_w) * sizeof(unsigned long long);
 }
 static const void* batch_kernel(int threads, bool pre) {
   if (pre)
@@ -1596,17 +1529,16 @@ static const void* batch_kernel(int threads, bool pre) {
                        : (const void*)k_batch<4, false>;
 }
 // Co-resident blocks of k_batch for the given shape (its cooperative grid).
-int batch_grid(int tile_w, int tile_h, int chunk, int threads, bool pre) {
+int batch_grid(int tile_w, int tile_h, int threads, bool pre) {
   int per = 0;
-  size_t smem = batch_smem(tile_w, tile_h, chunk);
+  size_t smem = batch_smem(tile_w, tile_h, threads);
   const void* k = batch_kernel(threads, pre);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, smem);
   if (per <= 0) return 0;
   return sm_count() * per;
 }
-cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* block_sums, cudaStream_t st,
-                         cudaEvent_t* ev) {
+cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream_t st, cudaEvent_t* ev) {
   const bool pre = B.g.va != nullptr;  // null: kernels transform corners themselves
   if (ev) cudaEventRecord(ev[0], st);
   if (pre && B.g.n_verts + B.g.n_nrms > 0) {
@@ -1623,9 +1555,9 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, uint32_t* 
   }
   if (ev) cudaEventRecord(ev[2], st);
   BatchParams Bc = B;
-  void* args[] = {&Bc, &block_sums};
-  cudaError_t e = launch_coop(batch_kernel(threads, pre), grid, threads, args, batch_smem(B.tile_w, B.tile_h, B.chunk),
-                              st);
+  void* args[] = {&Bc};
+  cudaError_t e = launch_coop(batch_kernel(threads, pre), grid, threads, args,
+                              batch_smem(B.tile_w, B.tile_h, threads), st);
   if (ev) cudaEventRecord(ev[3], st);
   if (e != cudaSuccess) return e;
   return cudaGetLastError();

@@ -175,7 +175,7 @@ struct BatchParams {
   const uint32_t* scene_tile_base;  // n_scenes + 1 prefix of tile counts
   int n_scenes;
   uint32_t n_tiles;
-  int tile_w, tile_h, chunk;        // tile width and height (pixels), records staged per pass
+  int tile_w, tile_h;               // tile width and height (pixels)
   int small_max;                    // bbox pixels up to which the setup kernel rasterises (0: none)
   unsigned long long* vis;          // all scenes' visibility words (small_max > 0)
   size_t n_px;                      // pixels of all scenes

@@ -111,3 +111,25 @@ def test_projection_forms(product_lib, projection, shared):
     got = _render(st, sc)
     assert np.array_equal(got["ids"], ref["ids"])
     assert np.array_equal(got["depth"].view(np.uint32), ref["depth"].view(np.uint32))
+
+
+@pytest.mark.parametrize("small_max", [0, 64])
+@pytest.mark.parametrize("tiling", [(4, 16, 64), (8, 8, 128), (16, 16, 256), (32, 2, 64), (64, 32, 256), (128, 8, 128),
+                                    (256, 16, 256), (64, 64, 64)])
+def test_batch_strips(product_lib, tiling, small_max):
+    """The strips a tile is cut into (at most 256 pixels, rows of 4 to 256
+    columns), at frame edges that cut tiles, strips and rows, for records
+    narrower and wider than a strip."""
+    from minirender_gb300 import workloads as W
+    from minirender_gb300.batch import BatchRenderer
+    items = [_boxes((9, 33, 257, 700), (8, 33, 90), 771, 101), W.config4_scene(3, 16, (131, 77)),
+             _boxes((3, 12), (5, 17), 33, 31, 2), W.config1(64, 47)]
+    br = BatchRenderer(0)
+    try:
+        br.ctx.set_batch_tiling(tiling[0], tiling[1], tiling[2], 64)
+        br.ctx.set_batch_small_max(small_max)
+        br.render(items)
+        for k, (st, sc) in enumerate(items):
+            _same(br.read(k), O.render(st, sc), f"scene {k}")
+    finally:
+        br.close()
