@@ -180,7 +180,7 @@ MR_API int mr_destroy(mr_ctx* c) {
     c->vis.release(); c->rgb8.release(); c->depth.release(); c->rgbf.release();
     c->normals.release(); c->range.release(); c->ids.release(); c->recs.release();
     c->items.release(); c->spill.release(); c->stage.release();
-    c->va.release(); c->vb.release(); c->vn.release();
+    c->va.release(); c->vc.release(); c->vn.release(); c->tri.release();
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->d_cnt) cudaFree(c->d_cnt);
     if (c->h_cnt) cudaFreeHost(c->h_cnt);
@@ -639,8 +639,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     h_vbase[i] = (uint32_t)vbase;
     h_nbase[i] = (uint32_t)nbase;
     vbase += (uint64_t)m.d.n_pos;
-    nbase += (uint64_t)m.d.n_nrm;
-    if (vbase >= ((uint64_t)1 << 32) || nbase >= ((uint64_t)1 << 32))
+    if (vbase >= ((uint64_t)1 << 32))
       return fail(c, MR_E_INVALID, "more than 2^32-1 vertices or normals in one frame");
     const mr_material& M = rs[i].material;
     memcpy(R.diffuse, M.diffuse, sizeof(R.diffuse));
@@ -659,6 +658,9 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
       if (T.rgb8) R.tex8 = (const uint8_t*)T.mem;
       else R.texf = (const float*)T.mem;
     }
+    set_reads(R);
+    if (!R.unified) nbase += (uint64_t)m.d.n_nrm;
+    if (nbase >= ((uint64_t)1 << 32)) return fail(c, MR_E_INVALID, "more than 2^32-1 vertices or normals in one frame");
   }
   h_tbase[n] = base;
   h_vbase[n] = (uint32_t)vbase;
@@ -681,7 +683,8 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   const bool vertex_pass = 3 * (uint64_t)total >= 2 * (uint64_t)vbase;
   if (vertex_pass) {
     CK(c->va.ensure(vbase), "vertex buffer");
-    CK(c->vb.ensure(vbase), "vertex buffer");
+    CK(c->vc.ensure(2 * vbase), "vertex buffer");
+    if (n != 1) CK(c->tri.ensure(total), "triangle table");
     CK(c->vn.ensure(nbase), "normal buffer");
   }
   FrameParams& F = c->last;
@@ -713,7 +716,8 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   F.g.n_verts = (uint32_t)vbase;
   F.g.n_nrms = (uint32_t)nbase;
   F.g.va = vertex_pass ? c->va.p : nullptr;  // null: kernels transform per corner
-  F.g.vb = vertex_pass ? c->vb.p : nullptr;
+  F.g.vc = vertex_pass ? c->vc.p : nullptr;
+  F.g.tri = vertex_pass && n != 1 ? c->tri.p : nullptr;
   F.g.vn = vertex_pass ? c->vn.p : nullptr;
   F.vis = c->vis.p;
   F.recs = c->recs.p;
@@ -984,7 +988,8 @@ int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEven
                                (uint64_t)(uintptr_t)B.h_rs, (uint64_t)(uintptr_t)B.h_u32,
                                (uint64_t)(uintptr_t)B.h_scenes, (uint64_t)(uintptr_t)B.rs.p,
                                (uint64_t)(uintptr_t)B.bases.p, (uint64_t)(uintptr_t)B.scenes.p,
-                               (uint64_t)(uintptr_t)B.va.p, (uint64_t)(uintptr_t)B.vn.p, (uint64_t)(uintptr_t)B.vb.p,
+                               (uint64_t)(uintptr_t)B.va.p, (uint64_t)(uintptr_t)B.vn.p, (uint64_t)(uintptr_t)B.vc.p,
+                               (uint64_t)(uintptr_t)B.tri.p,
                                (uint64_t)(uintptr_t)B.recs.p, (uint64_t)B.P.rec_cap, (uint64_t)(uintptr_t)B.bins.p,
                                (uint64_t)B.P.bin_cap, (uint64_t)(uintptr_t)B.tiles.p, B.P.n_tiles};
   for (int s = 0; s < B.n_scenes; s++) {
@@ -1026,7 +1031,7 @@ int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEven
 
 void BatchSlot::release() {
   rs.release(); bases.release(); scenes.release(); stb.release(); va.release(); vn.release();
-  vb.release(); recs.release(); rec_scene.release(); tiles.release(); bins.release();
+  vc.release(); tri.release(); recs.release(); rec_scene.release(); tiles.release(); bins.release();
   out8.release(); outd.release(); outi.release(); vis.release();
   if (h_rs) cudaFreeHost(h_rs);
   if (h_u32) cudaFreeHost(h_u32);
@@ -1078,7 +1083,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
     if (rs[i].flags & ~kRenderableFlags) return fail(c, MR_E_INVALID, "unknown renderable flags");
     tris += (uint64_t)c->meshes[h].d.n_tri;
     verts += (uint64_t)c->meshes[h].d.n_pos;
-    nrms += (uint64_t)c->meshes[h].d.n_nrm;
+    nrms += mesh_unified(c->meshes[h].d) ? 0 : (uint64_t)c->meshes[h].d.n_nrm;
   }
   if (tris >= ((uint64_t)1 << 31) || verts >= ((uint64_t)1 << 32) || nrms >= ((uint64_t)1 << 32) ||
       tiles >= ((uint64_t)1 << 31))
@@ -1112,7 +1117,8 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   const bool vertex_pass = 3 * tris >= 2 * verts;
   if (vertex_pass) {
     CK(B.va.ensure(verts), "batch vertex buffer");
-    CK(B.vb.ensure(verts), "batch vertex buffer");
+    CK(B.vc.ensure(2 * verts), "batch vertex buffer");
+    CK(B.tri.ensure(tris), "batch triangle table");
     CK(B.vn.ensure(nrms), "batch normal buffer");
   }
   CK(B.recs.ensure(2 * tris), "batch records");
@@ -1148,7 +1154,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
       nbase[i] = nb;
       tri += (uint32_t)m.d.n_tri;
       vb += (uint32_t)m.d.n_pos;
-      nb += (uint32_t)m.d.n_nrm;
+      nb += mesh_unified(m.d) ? 0u : (uint32_t)m.d.n_nrm;
     }
   }
   // per-renderable matrices and materials (Renderer::paintMesh,
@@ -1187,6 +1193,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
         if (T.rgb8) R.tex8 = (const uint8_t*)T.mem;
         else R.texf = (const float*)T.mem;
       }
+      set_reads(R);
     }
   });
   tb[n_rs] = tri;
@@ -1204,7 +1211,8 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   P.g.n_verts = vb;
   P.g.n_nrms = nb;
   P.g.va = vertex_pass ? B.va.p : nullptr;
-  P.g.vb = vertex_pass ? B.vb.p : nullptr;
+  P.g.vc = vertex_pass ? B.vc.p : nullptr;
+  P.g.tri = vertex_pass ? B.tri.p : nullptr;
   P.g.vn = vertex_pass ? B.vn.p : nullptr;
   P.scenes = B.scenes.p;
   P.scene_tile_base = B.bases.p + 3 * (n_rs + 1);

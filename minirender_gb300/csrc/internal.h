@@ -84,6 +84,16 @@ inline void set_projection(View& V, const float* P) {
   V.znear = -zn;
 }
 
+// Whether a mesh has one index per corner for every attribute.
+inline bool mesh_unified(const DevMesh& M) { return M.nidx == M.idx && (!M.has_uv || M.tidx == M.idx); }
+
+// The derived fields of a renderable whose mesh, switches and material are set.
+inline void set_reads(DevRenderable& R) {
+  R.unified = mesh_unified(R.mesh);
+  R.need = (R.lit ? kNeedNormal : 0) | (R.has_tex ? kNeedTexcoord : 0) |
+           (R.lit && (R.point || R.shininess != 0) ? kNeedPosition : 0);
+}
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace mrgi
@@ -101,8 +111,8 @@ struct BatchSlot {
   DevBuf<uint32_t> bases;
   DevBuf<SceneRec> scenes;
   DevBuf<uint32_t> stb;
-  DevBuf<float4> va, vn;
-  DevBuf<float2> vb;
+  DevBuf<float4> va, vc, vn;
+  DevBuf<uint4> tri;
   DevBuf<BigRec> recs;
   DevBuf<uint32_t> rec_scene, tiles, bins;
   DevBuf<unsigned long long> vis;
@@ -166,8 +176,8 @@ struct mr_ctx {
   size_t h_rs_cap = 0, stage_bytes = 0, off_bases = 0;
   DevRenderable* h_rs = nullptr;
   uint32_t* h_tri_base = nullptr;
-  DevBuf<float4> va, vn;        // per-frame vertex-pass outputs
-  DevBuf<float2> vb;
+  DevBuf<float4> va, vc, vn;    // per-frame vertex-pass outputs
+  DevBuf<uint4> tri;            // per-triangle vertices and renderable
   Counters* d_cnt = nullptr;
   Counters* h_cnt = nullptr;
   cudaEvent_t ev[8] = {};

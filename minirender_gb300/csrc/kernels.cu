@@ -191,32 +191,54 @@ __device__ __forceinline__ int clip_pick(float zn, Vtx (&v)[3], int sub) {
   return 2;
 }
 
-// View-space corners of triangle t (paintMesh, src/Renderer.cpp:344-379).
-template <bool PRE, bool ATTR>
-__device__ __forceinline__ void corners(const Geo& G, const DevRenderable& R, int t, const int (&ip)[3],
-                                        Vtx (&v)[3]) {
+// Attributes of a corner that the fragments of a renderable read
+// (DevRenderable::need; a corner cut by the near plane takes all).
+__device__ __forceinline__ bool needs(const DevRenderable& R, int what, bool cut) { return cut || (R.need & what); }
+
+// View-space corners of triangle t without the vertex pass (paintMesh,
+// src/Renderer.cpp:344-379).
+template <bool ATTR>
+__device__ __forceinline__ void corners(const DevRenderable& R, int t, const int (&ip)[3], Vtx (&v)[3]) {
   const DevMesh& M = R.mesh;
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    if (PRE) {
-      float4 a = G.va[R.vert_base + ip[c]];
-      float2 b = G.vb[R.vert_base + ip[c]];
-      v[c].pos = v3(b.x, b.y, a.w);
-    } else {
-      v[c].pos = affine(R.mv, ld3(M.pos, ip[c]));
-    }
+    v[c].pos = affine(R.mv, ld3(M.pos, ip[c]));
     if (ATTR) {
-      // normalsI / texcoordsI shared with the indices: reuse the corner's index
-      // (PRE only: without the vertex pass the extra live registers spill,
-      // and the shared words are L1-hot anyway)
-      const int in = (PRE && M.nidx == M.idx) ? ip[c] : __ldg(M.nidx + 3 * t + c);
-      if (PRE) {
-        float4 n = G.vn[R.nrm_base + in];
+      v[c].nrm = affine(R.nm, ld3(M.nrm, __ldg(M.nidx + 3 * t + c)));
+      v[c].uv = M.has_uv ? ld2(M.uv, __ldg(M.tidx + 3 * t + c)) : v2(0, 0);
+    }
+  }
+}
+
+// The attributes of vertices gv (in the frame's vertex buffers; the corners
+// of triangle t) that R's fragments read.  A unified mesh has them all in
+// vc: normal and view x, view y and texcoord -- two sectors at most a corner
+// where positions, normals and texcoords were three scattered ones.
+__device__ __forceinline__ void vertex_attributes(const Geo& G, const DevRenderable& R, int t, const uint32_t (&gv)[3],
+                                                  bool cut, Vtx (&v)[3]) {
+  const bool nrm = needs(R, kNeedNormal, cut), uv = needs(R, kNeedTexcoord, cut), pos = needs(R, kNeedPosition, cut);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    if (nrm || pos) {
+      const float4 a = G.vc[2 * (size_t)gv[c]];
+      v[c].nrm = v3(a.x, a.y, a.z);
+      v[c].pos.x = a.w;
+    }
+    if (uv || pos) {
+      const float4 b = G.vc[2 * (size_t)gv[c] + 1];
+      v[c].pos.y = b.x;
+      v[c].uv = v2(b.y, b.z);
+    }
+  }
+  if (!R.unified) {
+    const DevMesh& M = R.mesh;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (nrm) {
+        const float4 n = G.vn[R.nrm_base + __ldg(M.nidx + 3 * t + c)];
         v[c].nrm = v3(n.x, n.y, n.z);
-      } else {
-        v[c].nrm = affine(R.nm, ld3(M.nrm, in));
       }
-      v[c].uv = M.has_uv ? ld2(M.uv, (PRE && M.tidx == M.idx) ? ip[c] : __ldg(M.tidx + 3 * t + c)) : v2(0, 0);
+      if (uv) v[c].uv = M.has_uv ? ld2(M.uv, __ldg(M.tidx + 3 * t + c)) : v2(0, 0);
     }
   }
 }
@@ -233,7 +255,7 @@ __device__ __forceinline__ void corners(const Geo& G, const DevRenderable& R, in
 constexpr uint32_t kRecPerFace = 1u;
 
 // The view-space corners with attributes of triangle t from its corner
-// record: the same values corners<false, true> gathers (src/Renderer.cpp:
+// record: the same values corners<true> gathers (src/Renderer.cpp:
 // 344-348, 356-373).  A per-face record needs its first 64 bytes only.
 __device__ __forceinline__ void corners_rec(const DevRenderable& R, int t, Vtx (&v)[3]) {
   const float4* r = R.mesh.rec + (size_t)8 * t;
@@ -460,6 +482,14 @@ __device__ __forceinline__ Setup rec_setup(const BigRec& B) {
   return S;
 }
 
+// Leaves a drawn triangle's vertices and renderable k for the resolve.
+__device__ __forceinline__ void note_triangle(const Geo& G, const DevRenderable& R, uint32_t k, int t) {
+  if (!G.tri) return;
+  const int* i = R.mesh.idx + 3 * (size_t)t;
+  G.tri[R.tri_base + (uint32_t)t] = make_uint4(R.vert_base + (uint32_t)__ldg(i), R.vert_base + (uint32_t)__ldg(i + 1),
+                                               R.vert_base + (uint32_t)__ldg(i + 2), k);
+}
+
 // Whether triangle t's indices failed the upload check.
 __device__ __forceinline__ bool bad_triangle(const DevMesh& M, int t) { return (M.bad[t >> 5] >> (t & 31)) & 1u; }
 
@@ -487,10 +517,10 @@ __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const Dev
     }
     float4 a[3];
 #pragma unroll
-    for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
+    for (int c = 0; c < 3; c++) ip[c] = (int)R.vert_base + __ldg(R.mesh.idx + 3 * t + c);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      a[c] = G.va[R.vert_base + ip[c]];
+      a[c] = G.va[(uint32_t)ip[c]];
       p[c] = v2(a[c].x, a[c].y);
       zt[c] = a[c].z;
     }
@@ -504,12 +534,17 @@ __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const Dev
       n_sub = -1;
       return false;
     }
-    corners<false, false>(G, R, t, ip, v);
+    corners<false>(R, t, ip, v);
     cut = v[0].pos.z > zn || v[1].pos.z > zn || v[2].pos.z > zn;
   }
   n_sub = 1;
   if (cut) {
-    if (PRE) corners<true, false>(G, R, t, ip, v);
+    if (PRE) {
+#pragma unroll
+      for (int c = 0; c < 3; c++)
+        v[c].pos = v3(G.vc[2 * (size_t)(uint32_t)ip[c]].w, G.vc[2 * (size_t)(uint32_t)ip[c] + 1].x,
+                      G.va[(uint32_t)ip[c]].w);
+    }
     n_sub = clip_pick<false>(zn, v, sub);
     if (n_sub <= sub) return false;
   }
@@ -521,23 +556,61 @@ __device__ __forceinline__ long long box_pixels(const Setup& S) {
   return (long long)(S.x1 - S.x0 + 1) * (S.y1 - S.y0 + 1);
 }
 
-// The sub-triangle `id` (of R) won by a pixel: its vertex indices and
-// view-space corners with attributes (the clipped sub-triangle when the
-// triangle crosses the near plane), src/Renderer.cpp:334-379, 131-161.
+// The renderable (of lo..hi-1) of global triangle g; with the vertex pass also
+// its vertices in the frame's buffers, both from the record the setup kernel
+// left: one load where the search, the mesh's index pointer and the indices
+// were a chain of eight.
 template <bool PRE>
-__device__ __forceinline__ void winner_tri(const View& V, const Geo& G, const DevRenderable& R, uint32_t id,
-                                           int (&ip)[3], Vtx (&vc)[3], bool& clipped) {
+__device__ __forceinline__ uint32_t find_triangle(const Geo& G, int lo, int hi, uint32_t g, uint32_t (&gv)[3]) {
+  if (PRE) {
+    const uint4 q = G.tri[g];
+    gv[0] = q.x;
+    gv[1] = q.y;
+    gv[2] = q.z;
+    return q.w;
+  }
+  return (uint32_t)find_base(G.tri_base, lo, hi, g);
+}
+
+// A pixel's winning sub-triangle: its corners with the attributes its
+// fragments read (the sub-triangle's own when the near plane cuts the
+// triangle), their pixel coordinates and depth terms.
+struct Winner {
+  Vtx v[3];
+  V2 p[3];
+  float zt[3];
+};
+
+// Sub-triangle `id` of R (src/Renderer.cpp:334-379, 131-161); with the vertex
+// pass, gv are the triangle's vertices in the frame's buffers.
+template <bool PRE>
+__device__ __forceinline__ void winner(const View& V, const Geo& G, const DevRenderable& R, uint32_t id,
+                                       const uint32_t (&gv)[3], Winner& N) {
   const int t = (int)((id >> 1) - R.tri_base);
-  if (!PRE && R.mesh.rec) {
-    corners_rec(R, t, vc);  // (ip is not used without the vertex pass)
+  const float zn = R.no_clip ? __int_as_float(0x7f800000) : V.znear;
+  bool cut;
+  if (PRE) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float4 a = G.va[gv[c]];
+      N.p[c] = v2(a.x, a.y);
+      N.zt[c] = a.z;
+      N.v[c].pos = v3(0, 0, a.w);
+      N.v[c].nrm = v3(0, 0, 0);
+      N.v[c].uv = v2(0, 0);
+    }
+  } else if (R.mesh.rec) {
+    corners_rec(R, t, N.v);
   } else {
+    int ip[3];
 #pragma unroll
     for (int c = 0; c < 3; c++) ip[c] = __ldg(R.mesh.idx + 3 * t + c);
-    corners<PRE, true>(G, R, t, ip, vc);
+    corners<true>(R, t, ip, N.v);
   }
-  const float zn = R.no_clip ? __int_as_float(0x7f800000) : V.znear;
-  clipped = vc[0].pos.z > zn || vc[1].pos.z > zn || vc[2].pos.z > zn;
-  if (clipped) clip_pick<true>(zn, vc, (int)(id & 1u));  // that sub-triangle exists: it won this pixel
+  cut = N.v[0].pos.z > zn || N.v[1].pos.z > zn || N.v[2].pos.z > zn;
+  if (PRE) vertex_attributes(G, R, t, gv, cut, N.v);
+  if (cut) clip_pick<true>(zn, N.v, (int)(id & 1u));  // that sub-triangle exists: it won this pixel
+  if (!PRE || cut) project3(V, N.v, N.p, N.zt);
 }
 
 // Texture and Blinn-Phong lighting of a fragment with perspective-corrected
@@ -578,23 +651,9 @@ __device__ __forceinline__ void shade(const View& V, const DevRenderable& R, con
 // The setup (src/Renderer.cpp:198-224) of the winning sub-triangle, the same
 // values its raster used; of the bounding box only the column x0 that a
 // replay starts from.
-template <bool PRE>
-__device__ __forceinline__ void winner_setup(const View& V, const Geo& G, const DevRenderable& R,
-                                             const int (&ip)[3], const Vtx (&vc)[3], bool clipped, Setup& S) {
-  V2 p[3];
-  float zt[3];
-  if (PRE && !clipped) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float4 a = G.va[R.vert_base + ip[c]];
-      p[c] = v2(a.x, a.y);
-      zt[c] = a.z;
-    }
-  } else {
-    project3(V, vc, p, zt);
-  }
-  setup_edges(p, zt, area2(p), S);
-  S.x0 = pixel_of(least(p[0].x, p[1].x, p[2].x), V.w);
+__device__ __forceinline__ void winner_setup(const View& V, const Winner& N, Setup& S) {
+  setup_edges(N.p, N.zt, area2(N.p), S);
+  S.x0 = pixel_of(least(N.p[0].x, N.p[1].x, N.p[2].x), V.w);
 }
 
 // The running edge values at pixel (x, y): row start, then column by column
@@ -613,7 +672,15 @@ __device__ __forceinline__ void vertex(const Geo& G, const View& V, const DevRen
   float px, py, zt;
   project(V, v, px, py, zt);
   G.va[g] = make_float4(px, py, zt, v.z);
-  G.vb[g] = make_float2(v.x, v.y);
+  // a mesh of one index per corner for every attribute carries them all here
+  V3 n = v3(0, 0, 0);
+  V2 uv = v2(0, 0);
+  if (R.unified) {
+    if (i < R.mesh.n_nrm) n = affine(R.nm, ld3(R.mesh.nrm, i));
+    if (i < R.mesh.n_uv) uv = ld2(R.mesh.uv, i);
+  }
+  G.vc[2 * (size_t)g] = make_float4(n.x, n.y, n.z, v.x);
+  G.vc[2 * (size_t)g + 1] = make_float4(v.y, uv.x, uv.y, 0.f);
 }
 // Normal i of R, at g in the frame's normal buffer.
 __device__ __forceinline__ void normal(const Geo& G, const DevRenderable& R, uint32_t g, int i) {
@@ -962,26 +1029,28 @@ __device__ __forceinline__ bool append_large(const FrameParams& F, const Setup& 
   return placed || !big;
 }
 
-// The renderable of global triangle g.  ONE: the frame's only renderable,
-// which the kernels read from their parameters (constant bank) instead of
-// through the staged table: no search, and no pointer to fetch before the
-// first index can be read.
+// Renderable k.  ONE: the frame's only renderable, which the kernels read
+// from their parameters (constant bank) instead of through the staged table:
+// no search, and no pointer to fetch before the first index can be read.
 template <bool ONE>
-__device__ __forceinline__ const DevRenderable& renderable(const FrameParams& F, uint32_t g) {
+__device__ __forceinline__ const DevRenderable& renderable(const FrameParams& F, uint32_t k) {
   if constexpr (ONE) return F.one;
-  else return F.g.rs[find_base(F.g.tri_base, 0, F.g.n_renderables, g)];
+  else return F.g.rs[k];
 }
 
 // Blocks of 256 threads per SM the register budget of the setup kernels must
 // allow.  With the vertex pass the kernel waits on index -> vertex gathers
-// and more resident warps hide that: 6 (40 registers, some spilled to L1)
-// with the packed staging records, which leave more L1 to the spills.
-// Without it (triangle soups) it is bound by its strided position loads and
-// by instruction issue, spilling and a smaller L1 cost more than the extra
-// warps hide, and the aligned records' vector copies are cheaper: 4 (64
-// registers).  Measured on 1080p and 4K frames.
+// and more resident warps hide that, at the price of spills: 5 in frames
+// (1080p mesh: 42.5 us, 44.6 with 6), 6 in batches, which spill more either
+// way (256 scenes: 420 us, 446 with 5); with the packed staging records, which
+// leave more L1 to the spills.  Without it (triangle soups) it is bound by its
+// strided position loads and by instruction issue, spilling and a smaller L1
+// cost more than the extra warps hide, and the aligned records' vector copies
+// are cheaper: 4 (64 registers).
 template <bool PRE>
-constexpr int kSetupMinBlocks = PRE ? 6 : 4;
+constexpr int kSetupMinBlocks = PRE ? 5 : 4;
+template <bool PRE>
+constexpr int kSetupBatchMinBlocks = PRE ? 6 : 4;
 template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup(FrameParams F) {
   pdl_wait();
@@ -991,7 +1060,8 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned w = threadIdx.x >> 5;
   const bool in = g < F.g.n_tris;
-  const DevRenderable& R = renderable<ONE>(F, in ? g : 0u);
+  const uint32_t k = ONE ? 0u : (uint32_t)find_base(F.g.tri_base, 0, F.g.n_renderables, in ? g : 0u);
+  const DevRenderable& R = renderable<ONE>(F, k);
   const int t = (int)(g - R.tri_base);
   int n_sub = in ? 1 : 0;
 #pragma unroll 1
@@ -1003,6 +1073,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
       small = box_pixels(S) <= (long long)F.small_max;
       big = !small;
     }
+    if (PRE && !ONE && (small || big)) note_triangle(F.g, R, k, t);
     if (sub == 0 && n_sub < 0) atomicOr(&F.counters->error_flags, 1u);
     count_triangles(F.counters, small, big, sub == 0 && cut && n_sub > 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
@@ -1081,17 +1152,21 @@ __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
   uint32_t id = MR_NO_TRIANGLE;
   if (vw != VIS_EMPTY) {
     id = (uint32_t)vw;
-    const DevRenderable& R = renderable<ONE>(F, id >> 1);
-    int ip[3];
-    Vtx vc[3];
-    bool clipped;
-    winner_tri<PRE>(F.v, F.g, R, id, ip, vc, clipped);
+    uint32_t k = 0, gv[3] = {0, 0, 0};
+    if constexpr (!ONE) k = find_triangle<PRE>(F.g, 0, F.g.n_renderables, id >> 1, gv);
+    const DevRenderable& R = renderable<ONE>(F, k);
+    if constexpr (ONE && PRE) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) gv[c] = (uint32_t)__ldg(R.mesh.idx + 3 * (size_t)(id >> 1) + c);
+    }
+    Winner N;
+    winner<PRE>(F.v, F.g, R, id, gv, N);
     Setup S;
-    winner_setup<PRE>(F.v, F.g, R, ip, vc, clipped, S);
+    winner_setup(F.v, N, S);
     float e1, e2, k0, k1, k2;
     replay(S, x, y, e1, e2);
     depth = frag_depth(S, F.v.persp != 0, e1, e2, k0, k1, k2);
-    shade(F.v, R, vc, k0, k1, k2, s_dec, value, normal);
+    shade(F.v, R, N.v, k0, k1, k2, s_dec, value, normal);
   }
   if (F.rgb8) {
     F.rgb8[3 * px + 0] = to_byte(value.x);
@@ -1118,7 +1193,7 @@ __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
 // (the register budget and staging layout of k_setup, for the same reasons;
 // on the 256-scene batch: 0.665 -> 0.453 ms)
 template <bool PRE>
-__global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256 / kSetupBatchThreads) k_setup_batch(BatchParams B) {
+__global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> * 256 / kSetupBatchThreads) k_setup_batch(BatchParams B) {
   using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;
   __shared__ Rec s_rec[kSetupBatchThreads / 32][kStageRecs];
   __shared__ int s_pre[kSetupBatchThreads / 32][kStageRecs];
@@ -1127,10 +1202,11 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256
   __syncthreads();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
-  uint32_t scene = 0;
+  uint32_t scene = 0, rk = 0;
   const DevRenderable* R = nullptr;
   if (g < B.g.n_tris) {
-    R = &B.g.rs[find_base(B.g.tri_base, 0, B.g.n_renderables, g)];
+    rk = (uint32_t)find_base(B.g.tri_base, 0, B.g.n_renderables, g);
+    R = &B.g.rs[rk];
     scene = R->scene;
   }
   int n_sub = R ? 1 : 0;
@@ -1144,6 +1220,7 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupMinBlocks<PRE> * 256
       small = box_pixels(S) <= (long long)B.small_max;
       big = !small;
     }
+    if (PRE && (small || big)) note_triangle(B.g, *R, rk, (int)(g - R->tri_base));
     if (sub == 0 && n_sub < 0) atomicOr(&B.counters->error_flags, 1u);
     count_triangles(B.counters, small, big, sub == 0 && cut && n_sub > 0);
     // record slots: in the first round each warp reserves within the block
@@ -1368,18 +1445,17 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
           value = v3(C.v.bg[0], C.v.bg[1], C.v.bg[2]);
           depth = 1e11f;
         } else {
-          int ip[3];
-          Vtx vc[3];
-          bool clipped;
-          const DevRenderable& R = B.g.rs[find_base(B.g.tri_base, (int)C.rs_begin, (int)C.rs_end, id >> 1)];
-          winner_tri<PRE>(C.v, B.g, R, id, ip, vc, clipped);
+          uint32_t gv[3];
+          const DevRenderable& R = B.g.rs[find_triangle<PRE>(B.g, (int)C.rs_begin, (int)C.rs_end, id >> 1, gv)];
+          Winner N;
+          winner<PRE>(C.v, B.g, R, id, gv, N);
           Setup S;
-          winner_setup<PRE>(C.v, B.g, R, ip, vc, clipped, S);
+          winner_setup(C.v, N, S);
           float e1, e2;
           replay(S, x, y, e1, e2);
           float k0, k1, k2;
           depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
-          shade(C.v, R, vc, k0, k1, k2, s_dec, value, normal);
+          shade(C.v, R, N.v, k0, k1, k2, s_dec, value, normal);
         }
         if (C.rgb8) {
           uint8_t* o8 = C.rgb8 + 3 * (size_t)px;

@@ -53,11 +53,15 @@ struct DevRenderable {
   int32_t no_clip;      // MR_RS_NO_CLIP: no near-plane clipping
   int32_t lit;          // lighting on for its fragments (the frame's or its paint call's)
   int32_t point;        // point light for its fragments (the frame's or its paint call's)
+  int32_t unified;      // one index per corner for every attribute: see Geo::vc
+  int32_t need;         // corner attributes its fragments read (kNeed*)
   float diffuse[3], specular[3], emissive[3], shininess;
   const uint8_t* tex8;  // rows x cols x 3 bytes (decoded b/255), or
   const float* texf;    // rows x cols x 3 floats
   int32_t tex_rows, tex_cols;
 };
+
+constexpr int kNeedNormal = 1, kNeedTexcoord = 2, kNeedPosition = 4;
 
 // Renderer state of one frame that the kernels read (src/Renderer.cpp:311-326).
 struct View {
@@ -87,8 +91,11 @@ struct Geo {
   int n_renderables;
   uint32_t n_tris, n_verts, n_nrms;
   float4* va;                 // (pixel x, pixel y, z term, view z) per vertex
-  float2* vb;                 // (view x, view y) per vertex
-  float4* vn;                 // view-space normal per normal
+  float4* vc;                 // two per vertex: (view-space normal, view x), (view y, texcoord, 0);
+                              // normal and texcoord of unified renderables only
+  float4* vn;                 // view-space normal per normal (renderables that are not unified)
+  uint4* tri;                 // frames of several renderables with the vertex pass: (vertices, renderable)
+                              // per triangle, left by the setup kernel for the resolve
 };
 
 // Setup record of a rasterised sub-triangle (64 bytes).

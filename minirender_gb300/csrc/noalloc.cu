@@ -124,6 +124,7 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
     if (tex_is_rgb8) R.tex8 = (const uint8_t*)texture;
     else R.texf = (const float*)texture;
   }
+  set_reads(R);
   const int W = f->width, H = f->height;
   FrameParams F;
   memset(&F, 0, sizeof(F));

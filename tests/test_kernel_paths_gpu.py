@@ -133,3 +133,26 @@ def test_batch_strips(product_lib, tiling, small_max):
             _same(br.read(k), O.render(st, sc), f"scene {k}")
     finally:
         br.close()
+
+
+@pytest.mark.parametrize("meshes", [1, 3])
+def test_shared_indices_with_unused_tail(product_lib, meshes):
+    """One index per corner for all attributes, with more vertices than
+    normals and texcoords (the rest unused), under every set of attributes
+    that the fragments read."""
+    from minirender_gb300 import workloads as W
+    st, sc = W.config2(level=3, width=150, height=110, tex_size=32)
+    m = sc.children[0]
+    extra = np.full((7, 3), np.nan, np.float32)
+    verts = np.concatenate([m.vertices, extra])
+    sc.children = []
+    for k in range(meshes):
+        xf = np.eye(4, dtype=np.float32)
+        xf[0, 3] = 0.8 * (k - (meshes - 1) / 2)
+        mat = S.Material(diffuse=(0.2 + 0.2 * k, 0.6, 0.5), shininess=0 if k == 1 else 9,
+                         texture=m.material.texture if k != 2 else None)
+        sc.add(S.TriMesh(verts, m.normals, m.indices, normalsI=m.indices, texcoords=m.texcoords,
+                         texcoordsI=m.indices, material=mat, transform=xf))
+    for lighting, texturing, point in ((True, True, False), (True, False, True), (False, True, False), (False, False, False)):
+        st.lighting, st.texturing, st.light_is_point = lighting, texturing, point
+        _same(_render(st, sc), O.render(st, sc), f"lighting {lighting}, texturing {texturing}, point {point}")
