@@ -980,7 +980,7 @@ static int enqueue_batch(mr_ctx* c, BatchSlot& B, cudaStream_t st, cudaEvent_t* 
 
 // Runs the staged batch of slot B on st; with profiling, ev[6]/ev[7] bracket
 // the whole batch and (outside graphs) ev[0..3] its stages.
-int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
+static int batch_launch(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
   std::vector<uint64_t> key = {(uint64_t)B.n_scenes, (uint64_t)B.n_rs, B.P.g.n_tris, B.P.g.n_verts, B.P.g.n_nrms,
                                (uint64_t)B.tile_w, (uint64_t)B.tile_h, (uint64_t)B.threads, (uint64_t)B.chunk,
                                (uint64_t)B.grid, (uint64_t)B.P.small_max, (uint64_t)(uintptr_t)B.P.vis,
@@ -1027,6 +1027,19 @@ int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEven
   CK(cudaGraphLaunch(B.exec, st), "graph launch");
   if (profiling) CK(cudaEventRecord(ev[7], st), "profiling event");
   return MR_OK;
+}
+
+// batch_launch with the visibility words it starts from empty: a batch leaves
+// them so (a separate clear of every scene's words was 110 us of a 256-scene
+// batch), unless the buffer is new or a launch failed.
+int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
+  if (B.small_max > 0 && !B.vis_empty) {  // a new buffer, or a batch that was not completed
+    CK(cudaMemsetAsync(B.vis.p, 0xFF, B.vis.cap * sizeof(unsigned long long), st), "visibility clear");
+  }
+  B.vis_empty = false;
+  const int rc = batch_launch(c, B, st, profiling, ev);
+  B.vis_empty = rc == MR_OK;
+  return rc;
 }
 
 void BatchSlot::release() {
@@ -1124,7 +1137,11 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   CK(B.recs.ensure(2 * tris), "batch records");
   CK(B.rec_scene.ensure(2 * tris), "batch records");
   CK(B.tiles.ensure(3 * tiles + 1), "batch tiles");
-  if (B.small_max > 0) CK(B.vis.ensure(pixels), "batch visibility");
+  if (B.small_max > 0) {
+    const void* before = B.vis.p;
+    CK(B.vis.ensure(pixels), "batch visibility");
+    if (B.vis.p != before) B.vis_empty = false;
+  }
   if (B.bins.cap < std::max<size_t>((size_t)1 << 20, 2 * tris))
     CK(B.bins.ensure(std::max<size_t>((size_t)1 << 20, 2 * tris)), "batch bins");
   int grid = batch_grid(TW, TH, B.threads, vertex_pass);
@@ -1222,7 +1239,6 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   P.tile_h = TH;
   P.small_max = B.small_max;
   P.vis = B.small_max > 0 ? B.vis.p : nullptr;
-  P.n_px = (size_t)pixels;
   P.recs = B.recs.p;
   P.rec_cap = (uint32_t)std::min<size_t>(B.recs.cap, 0xFFFFFFFFu);
   P.rec_scene = B.rec_scene.p;

@@ -139,6 +139,7 @@ struct BatchSlot {
   cudaEvent_t done = nullptr;
   cudaEvent_t staged = nullptr;   // the batch's host staging has been copied
   bool have = false;
+  bool vis_empty = false;  // every word of vis is VIS_EMPTY between batches (k_batch restores what it reads)
   cudaStream_t stream = nullptr;  // null: the context stream
   cudaEvent_t ev[8] = {};         // profiling events (slots other than the context's)
   bool profiling = false;

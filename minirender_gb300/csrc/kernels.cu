@@ -581,9 +581,17 @@ struct Winner {
   float zt[3];
 };
 
+// The winner of a triangle that the near plane cuts: the sub-triangle's
+// corners, projected.  Out of line: few pixels take it, and the batch kernel's
+// warps, each in a phase of its own, wait for instructions as it is.
+__device__ __noinline__ void cut_winner(const View& V, float zn, int sub, Winner& N) {
+  clip_pick<true>(zn, N.v, sub);
+#pragma unroll 1
+  for (int c = 0; c < 3; c++) project(V, N.v[c].pos, N.p[c].x, N.p[c].y, N.zt[c]);
+}
 // Sub-triangle `id` of R (src/Renderer.cpp:334-379, 131-161); with the vertex
 // pass, gv are the triangle's vertices in the frame's buffers.
-template <bool PRE>
+template <bool PRE, bool CALL = false>
 __device__ __forceinline__ void winner(const View& V, const Geo& G, const DevRenderable& R, uint32_t id,
                                        const uint32_t (&gv)[3], Winner& N) {
   const int t = (int)((id >> 1) - R.tri_base);
@@ -609,6 +617,16 @@ __device__ __forceinline__ void winner(const View& V, const Geo& G, const DevRen
   }
   cut = N.v[0].pos.z > zn || N.v[1].pos.z > zn || N.v[2].pos.z > zn;
   if (PRE) vertex_attributes(G, R, t, gv, cut, N.v);
+  if (CALL) {
+    if (cut) {
+      Winner T = N;
+      cut_winner(V, zn, (int)(id & 1u), T);
+      N = T;
+    } else if (!PRE) {
+      project3(V, N.v, N.p, N.zt);
+    }
+    return;
+  }
   if (cut) clip_pick<true>(zn, N.v, (int)(id & 1u));  // that sub-triangle exists: it won this pixel
   if (!PRE || cut) project3(V, N.v, N.p, N.zt);
 }
@@ -663,7 +681,10 @@ __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, 
 }
 
 // savePPM conversion, src/io.cpp:358-362.
-__device__ __forceinline__ uint8_t to_byte(float v) { return (uint8_t)(int)clampr(v * 255.0f, 0.0f, 255.0f); }
+// (a NaN gives 0 here as there)
+__device__ __forceinline__ uint32_t to_byte(float v) {
+  return (uint32_t)__float2int_rz(fminf(fmaxf(v * 255.0f, 0.0f), 255.0f));
+}
 
 // ------------------------------------------------------------------ kernels
 // Vertex i of R, at g in the frame's vertex buffers.
@@ -718,11 +739,6 @@ __global__ void __launch_bounds__(256) k_begin(FrameParams F) {
       else normal(F.g, F.one, (uint32_t)(g - F.g.n_verts), (int)(g - F.g.n_verts));
     }
   }
-}
-
-// vis[0..n) = VIS_EMPTY (batches: every scene's words).
-__global__ void __launch_bounds__(256) k_clear(unsigned long long* vis, size_t n) {
-  clear_words(vis, n, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x);
 }
 
 // Index check of a mesh upload (one bit per triangle), and for meshes with
@@ -1254,9 +1270,13 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> 
   }
 }
 
+constexpr int kStripMax = 256;
 // Rows of a tile that one warp of k_batch takes at a time: the strip holds at
-// most 256 pixels (8 a lane).
-__host__ __device__ inline int strip_rows(int tw, int th) { return th < 256 / tw ? th : 256 / tw; }
+// most strip_px pixels (or one row).
+__host__ __device__ inline int strip_rows(int tw, int th, int strip_px) {
+  const int r = tw < strip_px ? strip_px / tw : 1;
+  return th < r ? th : r;
+}
 // Words of shared memory between a strip's rows: rows of 16 pixels and more
 // are skewed so the same column of several rows falls in different banks.
 __host__ __device__ inline int strip_pitch(int tw) { return tw >= 16 ? tw + 4 : tw; }
@@ -1339,7 +1359,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
   cg::grid_group grid = cg::this_grid();
   const uint32_t nb = gridDim.x, nt = blockDim.x;
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
-  const int TW = B.tile_w, TH = B.tile_h, SH = strip_rows(TW, TH), pitch = strip_pitch(TW), lw = __ffs(TW) - 1;
+  const int TW = B.tile_w, TH = B.tile_h, SH = strip_rows(TW, TH, B.strip_px), pitch = strip_pitch(TW), lw = __ffs(TW) - 1;
   unsigned long long* svis = reinterpret_cast<unsigned long long*>(smem) + (size_t)w * SH * pitch;
   for (uint32_t i = threadIdx.x; i < 256; i += nt) s_dec[i] = (float)i / 255.0f;
   // 1. the tiles' ranges, in any order: one atomic per warp of tiles
@@ -1373,8 +1393,9 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
   }
   grid.sync();
   // 3. strips, in groups of two per warp of the block
-  const uint32_t strips = (uint32_t)(TH / SH), warps = nt >> 5;
-  const unsigned long long units = (unsigned long long)B.n_tiles * strips;
+  const uint32_t warps = nt >> 5;
+  const int ls2 = __ffs(TH / SH) - 1;  // strips per tile, a power of two
+  const unsigned long long units = (unsigned long long)B.n_tiles << ls2;
   const uint32_t group = 2u * warps;
   for (;;) {
     __syncthreads();
@@ -1391,7 +1412,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
       if (lane == 0) k = atomicAdd(&s_next, 1u);
       k = __shfl_sync(0xffffffffu, k, 0);
       if (k >= n_units) break;
-      const uint32_t t = (uint32_t)((first + k) / strips), strip = (uint32_t)((first + k) % strips);
+      const uint32_t t = (uint32_t)((first + k) >> ls2), strip = (uint32_t)(first + k) & ((1u << ls2) - 1u);
       // the scene: the last j with scene_tile_base[j] <= t (bases ascending,
       // the first 0), 32 candidates at a time
       int sc = 0;
@@ -1426,6 +1447,12 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
           else svis[cy * pitch + cx] = VIS_EMPTY;
         }
         cp_async_wait_all();
+        if (C.vis) {  // the frame's words are left empty for the next batch
+          for (int i = lane; i < SH * TW; i += 32) {
+            const int cy = i >> lw, cx = i & (TW - 1);
+            if (svis[cy * pitch + cx] != VIS_EMPTY) C.vis[(uint32_t)(py0 + cy) * (uint32_t)C.v.W + (uint32_t)(px0 + cx)] = VIS_EMPTY;
+          }
+        }
         __syncwarp();
         raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
         __syncwarp();
@@ -1438,6 +1465,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
         if (x > px1 || y > py1) continue;
         const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)x;
         const unsigned long long vw = !direct ? svis[cy * pitch + cx] : C.vis ? C.vis[px] : VIS_EMPTY;
+        if (direct && vw != VIS_EMPTY) C.vis[px] = VIS_EMPTY;
         V3 value, normal;
         float depth;
         const uint32_t id = (uint32_t)vw;
@@ -1448,7 +1476,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
           uint32_t gv[3];
           const DevRenderable& R = B.g.rs[find_triangle<PRE>(B.g, (int)C.rs_begin, (int)C.rs_end, id >> 1, gv)];
           Winner N;
-          winner<PRE>(C.v, B.g, R, id, gv, N);
+          winner<PRE, PRE>(C.v, B.g, R, id, gv, N);
           Setup S;
           winner_setup(C.v, N, S);
           float e1, e2;
@@ -1595,7 +1623,7 @@ cudaError_t launch_frame(const FrameParams& F, cudaStream_t st, cudaEvent_t* ev,
 
 size_t batch_smem(int tile_w, int tile_h, int threads) {
   // visibility words of one strip per warp
-  return (size_t)(threads / 32) * strip_rows(tile_w, tile_h) * strip_pitch(tile_w) * sizeof(unsigned long long);
+  return (size_t)(threads / 32) * strip_rows(tile_w, tile_h, kStripMax) * strip_pitch(tile_w) * sizeof(unsigned long long);
 }
 static const void* batch_kernel(int threads, bool pre) {
   if (pre)
@@ -1621,16 +1649,21 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream
     View none = {};
     k_vertex<true><<<grid_for((size_t)B.g.n_verts + B.g.n_nrms, 256), 256, 0, st>>>(B.g, none, B.scenes);
   }
-  if (B.small_max > 0 && B.n_px) {  // small triangles' visibility words of every scene
-    k_clear<<<std::min(grid_for((B.n_px + 1) / 2, 256), sm_count() * 16), 256, 0, st>>>(B.vis, B.n_px);
-  }
   if (ev) cudaEventRecord(ev[1], st);
   if (B.g.n_tris) {
     if (pre) k_setup_batch<true><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
     else k_setup_batch<false><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
   }
   if (ev) cudaEventRecord(ev[2], st);
+  // strips of 256 pixels, cut to as few as 32 where that would leave a warp
+  // fewer than 6 of them (a dense strip would be the batch's tail: two 137x96
+  // scenes 67 us with 256, 30 with 32; 24 scenes of 256x256 92 and 84); smaller
+  // ones read a tile's records and vertices more often (16 soups 242 us, 262
+  // with half the size)
   BatchParams Bc = B;
+  Bc.strip_px = kStripMax;
+  const unsigned long long px = (unsigned long long)B.n_tiles * B.tile_w * B.tile_h, warps = (unsigned long long)grid * threads / 32;
+  while (Bc.strip_px > 32 && px < 6 * warps * Bc.strip_px) Bc.strip_px /= 2;
   void* args[] = {&Bc};
   cudaError_t e = launch_coop(batch_kernel(threads, pre), grid, threads, args,
                               batch_smem(B.tile_w, B.tile_h, threads), st);

@@ -183,9 +183,9 @@ struct BatchParams {
   int n_scenes;
   uint32_t n_tiles;
   int tile_w, tile_h;               // tile width and height (pixels)
+  int strip_px;                     // pixels of a tile that a warp takes at a time
   int small_max;                    // bbox pixels up to which the setup kernel rasterises (0: none)
   unsigned long long* vis;          // all scenes' visibility words (small_max > 0)
-  size_t n_px;                      // pixels of all scenes
   BigRec* recs;
   uint32_t rec_cap;
   uint32_t* rec_scene;              // scene of each record
