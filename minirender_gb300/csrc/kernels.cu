@@ -1073,9 +1073,9 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
   using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;  // see kSetupMinBlocks
   __shared__ Rec s_rec[kSetupThreads / 32][kStageRecs];
   __shared__ int s_pre[kSetupThreads / 32][kStageRecs];
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned w = threadIdx.x >> 5;
-  const bool in = g < F.g.n_tris;
+  const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << F.tri_shift) + lane;
+  const bool in = lane < (1u << F.tri_shift) && g < F.g.n_tris;
   const uint32_t k = ONE ? 0u : (uint32_t)find_base(F.g.tri_base, 0, F.g.n_renderables, in ? g : 0u);
   const DevRenderable& R = renderable<ONE>(F, k);
   const int t = (int)(g - R.tri_base);
@@ -1216,11 +1216,11 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> 
   __shared__ unsigned s_fill, s_base;
   if (threadIdx.x == 0) s_fill = 0;
   __syncthreads();
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << B.tri_shift) + lane;
   uint32_t scene = 0, rk = 0;
   const DevRenderable* R = nullptr;
-  if (g < B.g.n_tris) {
+  if (lane < (1u << B.tri_shift) && g < B.g.n_tris) {
     rk = (uint32_t)find_base(B.g.tri_base, 0, B.g.n_renderables, g);
     R = &B.g.rs[rk];
     scene = R->scene;
@@ -1573,6 +1573,17 @@ static cudaError_t launch_coop(const void* fn, int grid, int block, void** args,
   return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+// Triangles a warp of the setup kernels takes, as a power of two: all 32 lanes
+// hold one when that gives every SM 16 warps, fewer in small frames, whose
+// time is that of one warp's triangles one row batch after another (UV sphere
+// of 3968 triangles 16.4 -> 10.3 us, 64 primitives 17.0 -> 13.9; with 32 warps
+// per SM a 20000-triangle soup is slower again, 9.3 -> 11.3).
+static int triangle_shift(size_t n_tris) {
+  int s = 5;
+  while (s > 1 && (n_tris >> s) < (size_t)sm_count() * 16) s--;
+  return s;
+}
+
 // Launch sequence of one frame.  With F.g.va set, the vertex pass runs first
 // and the setup/resolve kernels read its buffers.  staged (frames of several
 // renderables) is recorded once the staging block has been read.  ev
@@ -1599,7 +1610,10 @@ static cudaError_t launch_stages(const FrameParams& F, cudaStream_t st, cudaEven
   }
   if (ev) cudaEventRecord(ev[1], st);
   if (F.g.n_tris) {
-    le = launch_after(k_setup<PRE, ONE>, grid_for(F.g.n_tris, kSetupThreads), kSetupThreads, st, F);
+    FrameParams Fs = F;
+    Fs.tri_shift = triangle_shift(F.g.n_tris);
+    le = launch_after(k_setup<PRE, ONE>, grid_for((size_t)F.g.n_tris << (5 - Fs.tri_shift), kSetupThreads),
+                      kSetupThreads, st, Fs);
     if (le != cudaSuccess) return le;
   }
   if (ev) cudaEventRecord(ev[2], st);
@@ -1651,19 +1665,23 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream
   }
   if (ev) cudaEventRecord(ev[1], st);
   if (B.g.n_tris) {
-    if (pre) k_setup_batch<true><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
-    else k_setup_batch<false><<<grid_for(B.g.n_tris, kSetupBatchThreads), kSetupBatchThreads, 0, st>>>(B);
+    BatchParams Bs = B;
+    Bs.tri_shift = triangle_shift(B.g.n_tris);
+    const int sgrid = grid_for((size_t)B.g.n_tris << (5 - Bs.tri_shift), kSetupBatchThreads);
+    if (pre) k_setup_batch<true><<<sgrid, kSetupBatchThreads, 0, st>>>(Bs);
+    else k_setup_batch<false><<<sgrid, kSetupBatchThreads, 0, st>>>(Bs);
   }
   if (ev) cudaEventRecord(ev[2], st);
-  // strips of 256 pixels, cut to as few as 32 where that would leave a warp
-  // fewer than 6 of them (a dense strip would be the batch's tail: two 137x96
-  // scenes 67 us with 256, 30 with 32; 24 scenes of 256x256 92 and 84); smaller
-  // ones read a tile's records and vertices more often (16 soups 242 us, 262
-  // with half the size)
+  // strips of 256 pixels, cut to 128 or 64 where that would leave a warp fewer
+  // than 6 of them and to 32 where 64 leaves fewer than 2 (a dense strip would
+  // be the batch's tail: two 137x96 scenes 67 us with 256, 30 with 32; 24
+  // scenes of 256x256 92 with 256, 84 with 64, 89 with 32); smaller ones read a
+  // tile's records and vertices more often (16 soups 242 us, 262 with half)
   BatchParams Bc = B;
   Bc.strip_px = kStripMax;
   const unsigned long long px = (unsigned long long)B.n_tiles * B.tile_w * B.tile_h, warps = (unsigned long long)grid * threads / 32;
-  while (Bc.strip_px > 32 && px < 6 * warps * Bc.strip_px) Bc.strip_px /= 2;
+  while (Bc.strip_px > 64 && px < 6 * warps * Bc.strip_px) Bc.strip_px /= 2;
+  if (px < 2 * warps * 64) Bc.strip_px = 32;
   void* args[] = {&Bc};
   cudaError_t e = launch_coop(batch_kernel(threads, pre), grid, threads, args,
                               batch_smem(B.tile_w, B.tile_h, threads), st);

@@ -146,6 +146,7 @@ struct FrameParams {
   Geo g;
   DevRenderable one;          // the renderable of a frame that has one (no table is staged for it)
   int small_max;
+  int tri_shift;              // log2 of the triangles a warp of the setup kernel takes
   unsigned long long* vis;    // W*H
   BigRec* recs;               // large sub-triangles
   uint32_t rec_cap;
@@ -184,6 +185,7 @@ struct BatchParams {
   uint32_t n_tiles;
   int tile_w, tile_h;               // tile width and height (pixels)
   int strip_px;                     // pixels of a tile that a warp takes at a time
+  int tri_shift;                    // log2 of the triangles a warp of the setup kernel takes
   int small_max;                    // bbox pixels up to which the setup kernel rasterises (0: none)
   unsigned long long* vis;          // all scenes' visibility words (small_max > 0)
   BigRec* recs;
