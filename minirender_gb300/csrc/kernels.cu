@@ -631,10 +631,21 @@ __device__ __forceinline__ void winner(const View& V, const Geo& G, const DevRen
   if (!PRE || cut) project3(V, N.v, N.p, N.zt);
 }
 
+// loadPPM's texel decode b/255.0f (src/io.cpp:410), one division per byte
+// value.  In global memory, where the L1 holds it: as a table in shared memory
+// every block of the resolve paid for a division per thread and a barrier.
+struct DecodeTable {
+  float v[256];
+  constexpr DecodeTable() : v() {
+    for (int i = 0; i < 256; i++) v[i] = (float)i / 255.0f;
+  }
+};
+static __device__ const DecodeTable kDecode;
+
 // Texture and Blinn-Phong lighting of a fragment with perspective-corrected
 // weights k0..k2 over the corners vc, src/Renderer.cpp:262-305 (FAST_LIGHT).
 __device__ __forceinline__ void shade(const View& V, const DevRenderable& R, const Vtx (&vc)[3], float k0,
-                                      float k1, float k2, const float* s_dec, V3& value, V3& normal_out) {
+                                      float k1, float k2, V3& value, V3& normal_out) {
   V3 color = v3(R.diffuse[0], R.diffuse[1], R.diffuse[2]);
   if (R.has_tex) {
     V2 uv = add2(add2(ks2(k0, vc[0].uv), ks2(k1, vc[1].uv)), ks2(k2, vc[2].uv));
@@ -644,7 +655,7 @@ __device__ __forceinline__ void shade(const View& V, const DevRenderable& R, con
     tj = min(max(tj, 0), R.tex_cols - 1);
     size_t o = 3 * ((size_t)ti * R.tex_cols + tj);
     if (R.tex8)
-      color = v3(s_dec[R.tex8[o]], s_dec[R.tex8[o + 1]], s_dec[R.tex8[o + 2]]);
+      color = v3(__ldg(&kDecode.v[R.tex8[o]]), __ldg(&kDecode.v[R.tex8[o + 1]]), __ldg(&kDecode.v[R.tex8[o + 2]]));
     else
       color = v3(R.texf[o], R.texf[o + 1], R.texf[o + 2]);
   }
@@ -1142,17 +1153,15 @@ __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
   }
 }
 
-// Deferred resolve + shade: one thread per pixel, 256-thread blocks over
-// 32x8-pixel tiles.
-constexpr int kResolveTileW = 32, kResolveTileH = 8;
+// Deferred resolve + shade: one thread per pixel, 128-thread blocks over
+// 32x4-pixel tiles (a block keeps its registers until its slowest warp is
+// done: 1080p mesh 40.9 us with 256 threads, 36.9 with 128, 38.9 with 64; 4K
+// soup 235, 225, 229).
+constexpr int kResolveTileW = 32, kResolveTileH = 4, kResolveThreads = kResolveTileW * kResolveTileH;
 template <bool PRE, bool ONE>
-__global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
+__global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_resolve(FrameParams F) {
   pdl_wait();
-  // loadPPM's texel decode b/255.0f (src/io.cpp:410), one division per byte value
-  __shared__ float s_dec[256];
-  s_dec[threadIdx.x] = (float)threadIdx.x / 255.0f;
-  __syncthreads();
-  // 32x8-pixel block tiles, 16x2 per warp: neighbouring rows of a small
+  // 32x4-pixel block tiles, 16x2 per warp: neighbouring rows of a small
   // triangle are shaded by the same warp, so its corner data is fetched once
   const int tiles_x = (F.v.W + kResolveTileW - 1) / kResolveTileW;
   const int bx = blockIdx.x % tiles_x, by = blockIdx.x / tiles_x;
@@ -1182,7 +1191,7 @@ __global__ void __launch_bounds__(256, 4) k_resolve(FrameParams F) {
     float e1, e2, k0, k1, k2;
     replay(S, x, y, e1, e2);
     depth = frag_depth(S, F.v.persp != 0, e1, e2, k0, k1, k2);
-    shade(F.v, R, N.v, k0, k1, k2, s_dec, value, normal);
+    shade(F.v, R, N.v, k0, k1, k2, value, normal);
   }
   if (F.rgb8) {
     F.rgb8[3 * px + 0] = to_byte(value.x);
@@ -1352,7 +1361,6 @@ __device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, u
 template <int MINB, bool PRE>
 __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ float s_dec[256];
   __shared__ unsigned long long s_first;
   __shared__ uint32_t s_next;
   __shared__ SceneRec s_scene[8];
@@ -1361,7 +1369,6 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
   const int TW = B.tile_w, TH = B.tile_h, SH = strip_rows(TW, TH, B.strip_px), pitch = strip_pitch(TW), lw = __ffs(TW) - 1;
   unsigned long long* svis = reinterpret_cast<unsigned long long*>(smem) + (size_t)w * SH * pitch;
-  for (uint32_t i = threadIdx.x; i < 256; i += nt) s_dec[i] = (float)i / 255.0f;
   // 1. the tiles' ranges, in any order: one atomic per warp of tiles
   for (uint32_t t0 = (blockIdx.x * nt + threadIdx.x) & ~31u; t0 < B.n_tiles; t0 += nb * nt) {
     const uint32_t t = t0 + lane, v = t < B.n_tiles ? B.tile_count[t] : 0u;
@@ -1483,7 +1490,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
           replay(S, x, y, e1, e2);
           float k0, k1, k2;
           depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
-          shade(C.v, R, N.v, k0, k1, k2, s_dec, value, normal);
+          shade(C.v, R, N.v, k0, k1, k2, value, normal);
         }
         if (C.rgb8) {
           uint8_t* o8 = C.rgb8 + 3 * (size_t)px;
@@ -1622,7 +1629,7 @@ static cudaError_t launch_stages(const FrameParams& F, cudaStream_t st, cudaEven
   if (ev) cudaEventRecord(ev[3], st);
   if (ev) cudaEventRecord(ev[4], st);
   const int rgrid = ((F.v.W + kResolveTileW - 1) / kResolveTileW) * ((F.v.H + kResolveTileH - 1) / kResolveTileH);
-  le = launch_after(k_resolve<PRE, ONE>, rgrid, 256, st, F);
+  le = launch_after(k_resolve<PRE, ONE>, rgrid, kResolveThreads, st, F);
   if (le != cudaSuccess) return le;
   if (ev) cudaEventRecord(ev[5], st);
   return cudaGetLastError();
