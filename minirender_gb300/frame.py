@@ -36,17 +36,17 @@ class FrameState:
         if proj is None:
             from .projection import projection_ortho
             proj = projection_ortho(-40, 40, -30, 30, 50, 120)
-        f.projection[:] = [float(x) for x in _v(proj, 16)]
-        f.view[:] = [float(x) for x in _v(self.view, 16)]
+        f.projection[:] = _v(proj, 16).tolist()
+        f.view[:] = _v(self.view, 16).tolist()
         light = self.light
         if light is None:
             l = np.array([-0.15, 0.6, 1.0], np.float32)
             ln = np.float32(math.sqrt(float(l[0] * l[0] + l[1] * l[1] + l[2] * l[2])))
             light = l / ln
-        f.light[:] = [float(x) for x in _v(light, 3)]
+        f.light[:] = _v(light, 3).tolist()
         f.light_is_point = int(bool(self.light_is_point))
         f.ambient = float(np.float32(self.ambient))
-        f.background[:] = [float(x) for x in _v(self.background, 3)]
+        f.background[:] = _v(self.background, 3).tolist()
         f.lighting = int(bool(self.lighting))
         f.texturing = int(bool(self.texturing))
         f.save_normals = int(bool(self.save_normals))

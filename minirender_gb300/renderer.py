@@ -251,14 +251,22 @@ class Renderer:
             frame.background[:] = [float(x) for x in self._clear_bg]
         return frame
 
-    def _read(self) -> dict:
+    def _read(self, name: Optional[str] = None) -> dict:
+        """The outputs of the last frame read so far, `name` among them: each
+        is copied from the device when it is first asked for."""
         if self._dirty:
             self._flush_paints()
         if self._out is None:
             if not self._rendered:
                 return self._cleared()
-            self._out = self.ctx.read(rgb8=True, depth=True, rgb_f32=True, tri_id=True,
-                                      normals=self.state.save_normals)
+            self._out = {}
+        want = set() if name is None or name in self._out else {name}
+        if not self._out and self.state.save_normals:
+            want.add("normals")
+        if want:
+            self._out.update(self.ctx.read(rgb8="rgb8" in want, depth="depth" in want, rgb_f32="image" in want,
+                                           tri_id="ids" in want,
+                                           normals="normals" in want and self.state.save_normals))
         return self._out
 
     def _cleared(self) -> dict:
@@ -276,28 +284,34 @@ class Renderer:
 
     # ---- getters, include/minirender/Renderer.h:60-63
     def getDepth(self) -> np.ndarray:
-        return self._read()["depth"]
+        return self._read("depth")["depth"]
 
     def getImage(self) -> np.ndarray:
-        return self._read()["image"]
+        return self._read("image")["image"]
 
     def getImageRGB8(self) -> np.ndarray:
         """getImage() after savePPM's byte conversion (src/io.cpp:358-362)."""
-        return self._read()["rgb8"]
+        return self._read("rgb8")["rgb8"]
 
     def getTriangleIds(self) -> np.ndarray:
         """Visible sub-triangle per pixel: 2*(global triangle)+clip part."""
-        return self._read()["ids"]
+        return self._read("ids")["ids"]
 
     def getRangeImage(self) -> np.ndarray:
         self._read()
         return self.ctx.range_image()
 
     def getNormalsImage(self) -> np.ndarray:
-        return self._read()["normals"]
+        return self._read("normals")["normals"]
 
     def stats(self) -> abi.mr_stats:
         return self.ctx.stats()
 
     def close(self):
+        # outputs of a frame that was being read stay available
+        if self._out and not self._dirty and self.ctx.h:
+            for name, bit in (("rgb8", abi.MR_OUT_RGB8), ("depth", abi.MR_OUT_DEPTH), ("image", abi.MR_OUT_RGB_F32),
+                              ("ids", abi.MR_OUT_TRI_ID)):
+                if self.ctx._outputs & bit:
+                    self._read(name)
         self.ctx.close()
