@@ -63,19 +63,30 @@ namespace mrg {
 // lets the successor's blocks start launching.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
-// 8-byte global-to-shared copy that bypasses registers (cp.async); the
-// thread's copies are complete after cp_async_wait_all().
-__device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 __device__ __forceinline__ int find_base(const uint32_t* base, int lo, int hi, uint32_t g) {
   while (hi - lo > 1) {
     int mid = (lo + hi) >> 1;
     if (base[mid] <= g) lo = mid; else hi = mid;
   }
+  return lo;
+}
+
+// find_base for the warp's consecutive g (lane 0 holds the smallest; every
+// lane calls): 32 candidates a round find lane 0's entry -- three dependent
+// loads for 16384 renderables instead of fourteen -- and the other lanes step
+// on from there.  n entries; base[n] is the end.
+__device__ __forceinline__ int find_base_warp(const uint32_t* base, int n, uint32_t g) {
+  const int lane = (int)(threadIdx.x & 31);
+  const uint32_t g0 = __shfl_sync(0xffffffffu, g, 0);
+  int lo = 0;
+  for (int m = n; m > 1;) {
+    const int step = (m + 31) >> 5, j = lane * step;
+    const unsigned hit = __ballot_sync(0xffffffffu, j < m && base[lo + j] <= g0);
+    const int at = (31 - __clz((int)(hit | 1u))) * step;
+    lo += at;
+    m = min(step, m - at);
+  }
+  while (lo + 1 < n && base[lo + 1] <= g) lo++;
   return lo;
 }
 
@@ -818,7 +829,11 @@ __global__ void __launch_bounds__(256) k_vertex(Geo G, View V, const SceneRec* s
   pdl_wait();
   pdl_trigger();
   const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < G.n_verts) {
+  if ((g & ~31u) + 32 <= G.n_verts) {  // (a whole warp)
+    const DevRenderable& R = G.rs[find_base_warp(G.vert_base, G.n_renderables, g)];
+    if constexpr (BATCH) vertex(G, scenes[R.scene].v, R, g, (int)(g - R.vert_base));
+    else vertex(G, V, R, g, (int)(g - R.vert_base));
+  } else if (g < G.n_verts) {
     const DevRenderable& R = G.rs[find_base(G.vert_base, 0, G.n_renderables, g)];
     if constexpr (BATCH) vertex(G, scenes[R.scene].v, R, g, (int)(g - R.vert_base));
     else vertex(G, V, R, g, (int)(g - R.vert_base));
@@ -1087,7 +1102,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
   const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << F.tri_shift) + lane;
   const bool in = lane < (1u << F.tri_shift) && g < F.g.n_tris;
-  const uint32_t k = ONE ? 0u : (uint32_t)find_base(F.g.tri_base, 0, F.g.n_renderables, in ? g : 0u);
+  const uint32_t k = ONE ? 0u : (uint32_t)find_base_warp(F.g.tri_base, F.g.n_renderables, min(g, F.g.n_tris - 1));
   const DevRenderable& R = renderable<ONE>(F, k);
   const int t = (int)(g - R.tri_base);
   int n_sub = in ? 1 : 0;
@@ -1227,10 +1242,11 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> 
   __syncthreads();
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << B.tri_shift) + lane;
-  uint32_t scene = 0, rk = 0;
+  uint32_t scene = 0;
+  const bool in = lane < (1u << B.tri_shift) && g < B.g.n_tris;
+  const uint32_t rk = (uint32_t)find_base_warp(B.g.tri_base, B.g.n_renderables, min(g, B.g.n_tris - 1));
   const DevRenderable* R = nullptr;
-  if (lane < (1u << B.tri_shift) && g < B.g.n_tris) {
-    rk = (uint32_t)find_base(B.g.tri_base, 0, B.g.n_renderables, g);
+  if (in) {
     R = &B.g.rs[rk];
     scene = R->scene;
   }
@@ -1357,9 +1373,10 @@ __device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, u
 // also captured the winners' edge values where a replay could pass 256
 // columns; with packed adds the replay is the cheaper.)  Groups of two strips
 // a warp: one gives up the shared reads (2822 us), four leave a tail (2723).
-// MINB: blocks of 256 threads per SM the register allocation must allow.
-template <int MINB, bool PRE>
-__global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
+// 64 registers: with 80 the 256 scenes take 2565 us (2270) and 16 soups 221
+// (205), with up to 128, which blocks of 64 threads had, the soups 252.
+template <bool PRE>
+__global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned long long s_first;
   __shared__ uint32_t s_next;
@@ -1445,34 +1462,69 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchParams B) {
       const bool persp = C.v.persp != 0;
       // the tile's list (truncated at capacity on overflow)
       const uint32_t ls = min(B.tile_start[t], B.bin_cap), le = min(B.tile_start[t] + B.tile_count[t], B.bin_cap);
-      if (ls < le) {
-        // the strip starts from the small triangles' words (or empty), copied
-        // with cp.async so all of a lane's loads are in flight at once
-        for (int i = lane; i < SH * TW; i += 32) {
-          const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
-          if (C.vis && x <= px1 && y <= py1) cp_async8(&svis[cy * pitch + cx], &C.vis[(uint32_t)y * (uint32_t)C.v.W + x]);
-          else svis[cy * pitch + cx] = VIS_EMPTY;
-        }
-        cp_async_wait_all();
-        if (C.vis) {  // the frame's words are left empty for the next batch
-          for (int i = lane; i < SH * TW; i += 32) {
-            const int cy = i >> lw, cx = i & (TW - 1);
-            if (svis[cy * pitch + cx] != VIS_EMPTY) C.vis[(uint32_t)(py0 + cy) * (uint32_t)C.v.W + (uint32_t)(px0 + cx)] = VIS_EMPTY;
+      // the strip starts from the small triangles' words (or empty): two
+      // words a load, all of a lane's in flight at once; what is not empty is
+      // left empty for the next batch
+      bool drawn = false;
+      {
+        const bool pairs = ((C.v.W & 1) | (int)((uintptr_t)C.vis >> 3 & 1)) == 0 && px1 - px0 + 1 == TW;
+        ulonglong2 v[kStripMax / 64];
+#pragma unroll
+        for (int j = 0; j < kStripMax / 64; j++) {
+          const int i = 64 * j + 2 * lane, cy = i >> lw, x = px0 + (i & (TW - 1)), y = py0 + cy;
+          v[j] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
+          if (C.vis && i < SH * TW && y <= py1) {
+            unsigned long long* q = C.vis + ((uint32_t)y * (uint32_t)C.v.W + (uint32_t)x);
+            if (pairs) {
+              v[j] = *reinterpret_cast<const ulonglong2*>(q);
+            } else {
+              if (x <= px1) v[j].x = q[0];
+              if (x + 1 <= px1) v[j].y = q[1];
+            }
           }
         }
-        __syncwarp();
-        raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
-        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < kStripMax / 64; j++) {
+          const int i = 64 * j + 2 * lane, cy = i >> lw, cx = i & (TW - 1);
+          if (i >= SH * TW) break;
+          if ((v[j].x & v[j].y) != VIS_EMPTY) {
+            drawn = true;
+            unsigned long long* q = C.vis + ((uint32_t)(py0 + cy) * (uint32_t)C.v.W + (uint32_t)(px0 + cx));
+            if (v[j].x != VIS_EMPTY) q[0] = VIS_EMPTY;
+            if (v[j].y != VIS_EMPTY) q[1] = VIS_EMPTY;
+          }
+          *reinterpret_cast<ulonglong2*>(svis + cy * pitch + cx) = v[j];
+        }
       }
-      const bool direct = ls >= le;
+      __syncwarp();
+      if (ls < le) raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
+      // nothing drawn: the background, four pixels a lane where whole groups
+      // of four lie aligned in every output
+      if (ls >= le && !__any_sync(0xffffffffu, drawn) && px1 - px0 + 1 == TW && (C.v.W & 3) == 0 &&
+          (((uintptr_t)C.depth | (uintptr_t)C.ids) & 15) == 0 && ((uintptr_t)C.rgb8 & 3) == 0) {
+        const uint32_t c = to_byte(C.v.bg[0]) | ((uint32_t)to_byte(C.v.bg[1]) << 8) | ((uint32_t)to_byte(C.v.bg[2]) << 16);
+        for (int i = 4 * lane; i < SH * TW; i += 128) {
+          const int y = py0 + (i >> lw);
+          if (y > py1) break;
+          const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)(px0 + (i & (TW - 1)));
+          if (C.rgb8) {
+            uint32_t* o = reinterpret_cast<uint32_t*>(C.rgb8 + 3 * (size_t)px);
+            o[0] = c | (c << 24);
+            o[1] = (c >> 8) | (c << 16);
+            o[2] = (c >> 16) | (c << 8);
+          }
+          if (C.depth) *reinterpret_cast<float4*>(C.depth + px) = make_float4(1e11f, 1e11f, 1e11f, 1e11f);
+          if (C.ids) *reinterpret_cast<uint4*>(C.ids + px) = make_uint4(MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE);
+        }
+        continue;
+      }
       const uint32_t id0 = 2u * B.g.tri_base[C.rs_begin];  // ids are reported per scene
 #pragma unroll 1
       for (int i = lane; i < SH * TW; i += 32) {
         const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
         if (x > px1 || y > py1) continue;
         const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)x;
-        const unsigned long long vw = !direct ? svis[cy * pitch + cx] : C.vis ? C.vis[px] : VIS_EMPTY;
-        if (direct && vw != VIS_EMPTY) C.vis[px] = VIS_EMPTY;
+        const unsigned long long vw = svis[cy * pitch + cx];
         V3 value, normal;
         float depth;
         const uint32_t id = (uint32_t)vw;
@@ -1646,18 +1698,12 @@ size_t batch_smem(int tile_w, int tile_h, int threads) {
   // visibility words of one strip per warp
   return (size_t)(threads / 32) * strip_rows(tile_w, tile_h, kStripMax) * strip_pitch(tile_w) * sizeof(unsigned long long);
 }
-static const void* batch_kernel(int threads, bool pre) {
-  if (pre)
-    return threads <= 64 ? (const void*)k_batch<2, true>
-                         : (const void*)k_batch<4, true>;
-  return threads <= 64 ? (const void*)k_batch<2, false>
-                       : (const void*)k_batch<4, false>;
-}
+static const void* batch_kernel(bool pre) { return pre ? (const void*)k_batch<true> : (const void*)k_batch<false>; }
 // Co-resident blocks of k_batch for the given shape (its cooperative grid).
 int batch_grid(int tile_w, int tile_h, int threads, bool pre) {
   int per = 0;
   size_t smem = batch_smem(tile_w, tile_h, threads);
-  const void* k = batch_kernel(threads, pre);
+  const void* k = batch_kernel(pre);
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, smem);
   if (per <= 0) return 0;
@@ -1690,7 +1736,7 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream
   while (Bc.strip_px > 64 && px < 6 * warps * Bc.strip_px) Bc.strip_px /= 2;
   if (px < 2 * warps * 64) Bc.strip_px = 32;
   void* args[] = {&Bc};
-  cudaError_t e = launch_coop(batch_kernel(threads, pre), grid, threads, args,
+  cudaError_t e = launch_coop(batch_kernel(pre), grid, threads, args,
                               batch_smem(B.tile_w, B.tile_h, threads), st);
   if (ev) cudaEventRecord(ev[3], st);
   if (e != cudaSuccess) return e;
