@@ -436,23 +436,70 @@ __device__ __forceinline__ void covered_run(const Setup& S, unsigned long long e
   hi = (int)floorf(fmaxf(b, -1.f));
 }
 
-// The columns of xs..xe of row y that the row may cover, in order, with their
-// running edge values (which step column by column from S.x0).
-template <typename Visit>
-__device__ __forceinline__ void walk_span(const Setup& S, int y, int xs, int xe, Visit visit) {
-  const unsigned long long d = pack2(S.n1.x, S.n2.x);
-  unsigned long long e = row_start2(S, y);
+// The first column of xs..xe of row y that the row may cover, with its running
+// edge values e (which step column by column from S.x0), and the length of the
+// run up to the last such column (0: none).
+__device__ __forceinline__ int row_run(const Setup& S, int y, int& xs, int xe, unsigned long long& e) {
+  e = row_start2(S, y);
   int lo, hi;
   covered_run(S, e, xe - S.x0 + 1, lo, hi);
   xs = max(xs, S.x0 + lo);
-  xe = min(xe, S.x0 + hi);
-  if (xs > xe) return;
-  e = advance2(e, d, xs - S.x0);
-  for (int x = xs; x <= xe; x++) {
-    float e1, e2;
-    unpack2(e, e1, e2);
-    visit(x, e1, e2);
-    e = add2(e, d);
+  const int len = max(0, min(xe, S.x0 + hi) - xs + 1);
+  if (len) e = advance2(e, pack2(S.n1.x, S.n2.x), xs - S.x0);
+  return len;
+}
+
+// The runs of a warp's rows (one row per lane: len columns from the edge
+// values e0, its first pixel at `at`), cut into pieces of kPiece columns and
+// dealt one per lane: depth and put(pixel, word) of every fragment that passes
+// z < 1e11f (src/Renderer.cpp:243-269).  A lane that walked its own row to the
+// end waited for the warp's longest: 256 scenes' fused stage 2266 us so, 1975
+// with pieces of 4, 1955 with 2, 2014 with 1, 2018 with 8.  Called by all
+// lanes of the warp.
+constexpr int kPiece = 2;
+template <typename Cell, typename Put>
+__device__ __forceinline__ void raster_runs(const Setup& S, bool persp, uint32_t id, unsigned long long e0, int len,
+                                            Cell at, Put put) {
+  const int lane = (int)(threadIdx.x & 31);
+  const int pieces = (len + kPiece - 1) / kPiece;
+  int inc = pieces;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll 1
+  for (int q = 0; q < total; q += 32) {
+    const int j = q + lane;
+    int own = 0;  // the lane whose row piece j belongs to
+#pragma unroll
+    for (int step = 16; step; step >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= j) own += step;
+    const int first = kPiece * (j - __shfl_sync(0xffffffffu, inc - pieces, own));
+    Setup T;
+    T.n1.x = __shfl_sync(0xffffffffu, S.n1.x, own);
+    T.n2.x = __shfl_sync(0xffffffffu, S.n2.x, own);
+#pragma unroll
+    for (int c = 0; c < 3; c++) T.z[c] = __shfl_sync(0xffffffffu, S.z[c], own);
+    const uint32_t tid = __shfl_sync(0xffffffffu, id, own);
+    unsigned long long e = __shfl_sync(0xffffffffu, e0, own);
+    const Cell cell = __shfl_sync(0xffffffffu, at, own) + (Cell)first;
+    const int n = __shfl_sync(0xffffffffu, len, own) - first;
+    if (j >= total) continue;
+    const unsigned long long d = pack2(T.n1.x, T.n2.x);
+    e = advance2(e, d, first);
+#pragma unroll
+    for (int x = 0; x < kPiece; x++) {
+      float e1, e2;
+      unpack2(e, e1, e2);
+      if (x < n && covered(e1, e2)) {
+        float k0, k1, k2;
+        const float z = frag_depth(T, persp, e1, e2, k0, k1, k2);
+        if (z < 1e11f) put(cell + (Cell)x, ((unsigned long long)depth_key(z) << 32) | tid);
+      }
+      if (x + 1 < kPiece) e = add2(e, d);
+    }
   }
 }
 
@@ -1125,30 +1172,44 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
 }
 
 // Large sub-triangles, one warp per block of kLargeRows rows by one column
-// segment of a record's bounding box, one row per lane: the lane replays its
-// row to the segment and walks it with 64-bit atomicMin into vis[]
-// (src/Renderer.cpp:238-269).  Then the spill list: one warp per record, its
-// remaining blocks.  An ordinary launch: with no large record every warp
-// leaves at once.
+// segment of a record's bounding box (src/Renderer.cpp:238-269): each lane
+// finds its row's covered run in the segment, then the runs are walked a row
+// per lane, or dealt in pieces where a few rows or ragged runs would leave
+// lanes waiting.  Then the spill list: one warp per record, its remaining
+// blocks.  An ordinary launch: with no large record every warp leaves at once.
 // Bound by the serial walk of a row, which is why rows are cut into segments
-// (large_segs): 64 primitives at 1280x720, 30.4 -> 10.9 us.
+// (large_segs): 64 primitives at 1280x720, 30.4 us with whole rows.
 __device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, uint32_t rec, uint32_t k) {
   const BigRec& R = F.recs[rec];
   const Setup S = rec_setup(R);
+  const uint32_t id = R.id;
   const int segs = large_segs(S.x0, S.x1), w = large_seg_cols(S.x0, S.x1);
   const int b = (int)k / segs, c = (int)k - b * segs;
   const int y = S.y0 + b * kLargeRows + (int)(threadIdx.x & 31);
-  if (y > S.y1) return;
-  const int xs = S.x0 + c * w;
-  unsigned long long* row = F.vis + (size_t)y * F.v.W;
-  const uint32_t id = R.id;
-  walk_span(S, y, xs, min(xs + w - 1, S.x1), [&](int x, float e1, float e2) {
-    if (covered(e1, e2)) {
-      float k0, k1, k2;
-      const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
-      if (z < 1e11f) atomicMin(row + x, ((unsigned long long)depth_key(z) << 32) | id);
+  int xs = S.x0 + c * w, len = 0;
+  unsigned long long e = 0;
+  if (y <= S.y1) len = row_run(S, y, xs, min(xs + w - 1, S.x1), e);
+  const uint32_t at = (uint32_t)y * (uint32_t)F.v.W + (uint32_t)xs;
+  const auto put = [&](uint32_t p, unsigned long long v) { atomicMin(F.vis + p, v); };
+  // a row per lane walks as many columns as the longest run has; 32 pieces take
+  // about three columns' time
+  const unsigned longest = __reduce_max_sync(0xffffffffu, (unsigned)len);
+  const unsigned pieces = __reduce_add_sync(0xffffffffu, (unsigned)(len + kPiece - 1) / kPiece);
+  if (3 * ((pieces + 31) / 32) < longest) {
+    raster_runs(S, persp, id, e, len, at, put);
+  } else {
+    const unsigned long long d = pack2(S.n1.x, S.n2.x);
+    for (int x = 0; x < len; x++) {
+      float e1, e2;
+      unpack2(e, e1, e2);
+      if (covered(e1, e2)) {
+        float k0, k1, k2;
+        const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
+        if (z < 1e11f) put(at + (uint32_t)x, ((unsigned long long)depth_key(z) << 32) | id);
+      }
+      e = add2(e, d);
     }
-  });
+  }
 }
 
 __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
@@ -1338,20 +1399,22 @@ __device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, u
         if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= i) own += step;
       const int k = i - __shfl_sync(0xffffffffu, inc - rows, own);
       const uint32_t r = __shfl_sync(0xffffffffu, rec, own);
+      Setup S;
+      uint32_t id = 0, at = 0;
+      int len = 0;
+      unsigned long long e = 0;
+      S.n1 = S.n2 = v2(0, 0);
+      S.z[0] = S.z[1] = S.z[2] = 0;
       if (i < total) {
         const BigRec& R = B.recs[r];
-        const Setup S = rec_setup(R);
+        S = rec_setup(R);
+        id = R.id;
         const int y = max(S.y0, py0) + k;
-        const uint32_t id = R.id;
-        unsigned long long* row = svis + (y - py0) * pitch - px0;
-        walk_span(S, y, max(S.x0, px0), min(S.x1, px1), [&](int x, float e1, float e2) {
-          if (covered(e1, e2)) {
-            float k0, k1, k2;
-            const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
-            if (z < 1e11f) atomicMin(row + x, ((unsigned long long)depth_key(z) << 32) | id);
-          }
-        });
+        int xs = max(S.x0, px0);
+        len = row_run(S, y, xs, min(S.x1, px1), e);
+        at = (uint32_t)((y - py0) * pitch + xs - px0);
       }
+      raster_runs(S, persp, id, e, len, at, [&](uint32_t c, unsigned long long v) { atomicMin(svis + c, v); });
     }
     __syncwarp();
   }

@@ -57,9 +57,10 @@ def _boxes(widths, heights, w, h, meshes=1):
 
 @pytest.mark.parametrize("meshes", [1, 3])
 def test_large_triangle_column_segments(product_lib, meshes):
-    """Widths and heights on either side of the column segments (32 columns up
-    to a width of 512, then 64, 96, ...) and row blocks of large triangles."""
-    st, sc = _boxes((9, 31, 32, 33, 64, 65, 511, 512, 513, 545, 1025, 1300), (8, 31, 32, 33, 65, 90), 1400, 100, meshes)
+    """Widths and heights on either side of the column segments (16 columns up
+    to a width of 256, then 32, 48, ...) and row blocks of large triangles."""
+    st, sc = _boxes((9, 15, 16, 17, 31, 33, 65, 255, 256, 257, 511, 513, 769, 1025, 1300), (8, 31, 32, 33, 65, 90), 1400,
+                    100, meshes)
     _same(_render(st, sc), O.render(st, sc), "boxes")
 
 
