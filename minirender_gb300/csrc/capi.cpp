@@ -674,9 +674,10 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   if (outputs & MR_OUT_RGB_F32) CK(c->rgbf.ensure(3 * npx), "rgb buffer");
   if (outputs & MR_OUT_TRI_ID) CK(c->ids.ensure(npx), "id buffer");
   if (f->save_normals) CK(c->normals.ensure(3 * npx), "normals buffer");
-  CK(c->recs.ensure((size_t)2 * total), "record buffer");
-  CK(c->spill.ensure((size_t)2 * total), "spill buffer");
-  if (c->items.cap < ((size_t)1 << 18)) CK(c->items.ensure((size_t)1 << 18), "block list");
+  const size_t share = rec_share_for((size_t)total);
+  CK(c->recs.ensure(share * kShares), "record buffer");
+  CK(c->spill.ensure(share * kShares), "spill buffer");
+  if (c->items.cap < ((size_t)1 << 19)) CK(c->items.ensure((size_t)1 << 19), "block list");
   // The per-vertex pass pays off when vertices are shared (each one used by
   // two or more triangle corners on average); for triangle soups every
   // corner is its own vertex and the kernels transform corners themselves.
@@ -721,9 +722,9 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   F.g.vn = vertex_pass ? c->vn.p : nullptr;
   F.vis = c->vis.p;
   F.recs = c->recs.p;
-  F.rec_cap = (uint32_t)std::min<size_t>(c->recs.cap, 0xFFFFFFFFu);
+  F.rec_share = (uint32_t)share;
   F.items = c->items.p;
-  F.item_cap = (uint32_t)std::min<size_t>(c->items.cap, 0xFFFFFFFFu);
+  F.item_share = (uint32_t)std::min<size_t>(c->items.cap / kShares, 0xFFFFFFFFu);
   F.spill = c->spill.p;
   F.rgb8 = (outputs & MR_OUT_RGB8) ? c->rgb8.p : nullptr;
   F.depth = (outputs & MR_OUT_DEPTH) ? c->depth.p : nullptr;
@@ -772,8 +773,10 @@ static int settle(mr_ctx* c) {
   }
   c->pending = false;
   const Counters& k = *c->h_cnt;
-  if (k.item_count > c->last.item_cap) {
-    const size_t want = std::min<size_t>((size_t)(k.item_count + k.item_count / 4 + 1024), kMaxItems);
+  unsigned long long most = 0;  // of any share
+  for (const ShareSlot& t : k.share) most = std::max(most, t.item_count);
+  if (most > c->last.item_share) {
+    const size_t want = kShares * std::min<size_t>((size_t)(most + most / 4 + 1024), kMaxItems / kShares);
     CK(c->items.ensure(want), "block list");
   }
   return (k.error_flags & 1u) ? fail(c, MR_E_BAD_INDEX, "a mesh index was out of range; those triangles were skipped") : MR_OK;
@@ -854,6 +857,10 @@ static void sum_stats(const Counters& k, mr_stats* s, bool small) {
     s->rasterised += (int64_t)(t.drawn >> 32);
     if (small) s->small_direct += (int64_t)(t.drawn & 0xFFFFFFFFu);
   }
+  for (const ShareSlot& t : k.share) {
+    s->binned += (int64_t)t.rec_count;
+    s->bin_entries += (int64_t)t.item_count;
+  }
 }
 
 MR_API int mr_get_stats(mr_ctx* c, mr_stats* s) {
@@ -866,8 +873,6 @@ MR_API int mr_get_stats(mr_ctx* c, mr_stats* s) {
   const Counters& k = *c->h_cnt;
   s->triangles = c->last.g.n_tris;
   sum_stats(k, s, true);
-  s->binned = (int64_t)k.rec_count;
-  s->bin_entries = (int64_t)k.item_count;
   s->error_flags = k.error_flags;
   if (c->profiling) {
     s->n_stages = 5;
@@ -990,7 +995,7 @@ static int batch_launch(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling
                                (uint64_t)(uintptr_t)B.bases.p, (uint64_t)(uintptr_t)B.scenes.p,
                                (uint64_t)(uintptr_t)B.va.p, (uint64_t)(uintptr_t)B.vn.p, (uint64_t)(uintptr_t)B.vc.p,
                                (uint64_t)(uintptr_t)B.tri.p,
-                               (uint64_t)(uintptr_t)B.recs.p, (uint64_t)B.P.rec_cap, (uint64_t)(uintptr_t)B.bins.p,
+                               (uint64_t)(uintptr_t)B.recs.p, (uint64_t)B.P.rec_share, (uint64_t)(uintptr_t)B.bins.p,
                                (uint64_t)B.P.bin_cap, (uint64_t)(uintptr_t)B.tiles.p, B.P.n_tiles};
   for (int s = 0; s < B.n_scenes; s++) {
     key.push_back(((uint64_t)B.W[s] << 32) | (uint64_t)B.H[s]);
@@ -1134,8 +1139,9 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
     CK(B.tri.ensure(tris), "batch triangle table");
     CK(B.vn.ensure(nrms), "batch normal buffer");
   }
-  CK(B.recs.ensure(2 * tris), "batch records");
-  CK(B.rec_scene.ensure(2 * tris), "batch records");
+  const size_t share = rec_share_for((size_t)tris);
+  CK(B.recs.ensure(share * kShares), "batch records");
+  CK(B.rec_scene.ensure(share * kShares), "batch records");
   CK(B.tiles.ensure(3 * tiles + 1), "batch tiles");
   if (B.small_max > 0) {
     const void* before = B.vis.p;
@@ -1240,7 +1246,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   P.small_max = B.small_max;
   P.vis = B.small_max > 0 ? B.vis.p : nullptr;
   P.recs = B.recs.p;
-  P.rec_cap = (uint32_t)std::min<size_t>(B.recs.cap, 0xFFFFFFFFu);
+  P.rec_share = (uint32_t)share;
   P.rec_scene = B.rec_scene.p;
   P.tile_count = B.tiles.p;
   P.tile_fill = B.tiles.p + tile_base;
@@ -1340,7 +1346,6 @@ MR_API int mr_get_batch_stats(mr_ctx* c, mr_stats* s) {
   const Counters& k = *c->b.h_cnt;
   s->triangles = c->b.P.g.n_tris;
   sum_stats(k, s, false);
-  s->binned = (int64_t)k.rec_count;
   s->bin_entries = (int64_t)k.bin_needed;
   s->error_flags = k.error_flags;
   if (c->profiling) {

@@ -508,6 +508,14 @@ __device__ __forceinline__ int large_seg_cols(int x0, int x1) {
   return kLargeCols * ((x1 - x0) / (kLargeCols * kLargeSegs) + 1);
 }
 __device__ __forceinline__ int large_segs(int x0, int x1) { return (x1 - x0) / large_seg_cols(x0, x1) + 1; }
+__device__ __forceinline__ int large_blocks(int x0, int y0, int x1, int y1) {
+  return ((y1 - y0) / kLargeRows + 1) * large_segs(x0, x1);
+}
+
+// The counters' slots of a warp: its statistics, and its share of the record
+// store and block list.
+__device__ __forceinline__ uint32_t warp_slot() { return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kStatSlots; }
+__device__ __forceinline__ uint32_t warp_share() { return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kShares; }
 
 // Adds a warp's sub-triangles (small: rasterised by the setup kernel) and
 // cut triangles to its statistics slot.  Called by all lanes of the warp.
@@ -515,7 +523,7 @@ __device__ __forceinline__ void count_triangles(Counters* c, bool small, bool bi
   const unsigned s = __ballot_sync(0xffffffffu, small), l = __ballot_sync(0xffffffffu, big);
   const unsigned k = __ballot_sync(0xffffffffu, cut);
   if ((threadIdx.x & 31) == 0 && (s | l | k)) {
-    StatSlot& slot = c->stat[((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kStatSlots];
+    StatSlot& slot = c->stat[warp_slot()];
     if (s | l) atomicAdd(&slot.drawn, ((unsigned long long)(__popc(s) + __popc(l)) << 32) | (unsigned)__popc(s));
     if (k) atomicAdd(&slot.clipped, (unsigned long long)__popc(k));
   }
@@ -945,13 +953,13 @@ __device__ __forceinline__ Setup rec_get(const Rec& q) {
 }
 constexpr int kStageRecs = 32;  // records staged per warp and round
 
-// Threads per block of the setup kernels.  Their warps share nothing in a
-// frame (statistics go to slots, staging is per warp), and a block keeps its
-// place until its slowest warp is done, so frames take small blocks: 1080p
-// mesh setup 48.8 us with 256 threads, 46.6 with 128, 44.6 with 64; 10M-
-// triangle soup 378, 368, 366 us.  Batches reserve records per block, one
-// global atomic each, and take 128 (256 scenes: 428, 417, 420 us).
-constexpr int kSetupThreads = 64, kSetupBatchThreads = 128;
+// Threads per block of the setup kernels.  Their warps share nothing
+// (statistics go to slots, staging is per warp, records are reserved by a warp
+// at a time), and a block keeps its place until its slowest warp is done:
+// 1080p mesh setup 48.8 us with 256 threads, 46.6 with 128, 44.6 with 64; 10M-
+// triangle soup 378, 368, 366 us; 256 scenes 387 us with 128 threads and
+// records reserved by the block, 379 so.
+constexpr int kSetupThreads = 64;
 
 // Where small triangles' fragments go: the frame's visibility buffer...
 struct FrameTarget {
@@ -1072,22 +1080,22 @@ __device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t i
   __syncwarp();  // s_rec / s_pre free for the warp's next use
 }
 
-// Appends the warp's large sub-triangles (one per lane where `big`) to the
-// record list, one atomic per warp, and their blocks to the block list.
+// Appends the warp's large sub-triangles (one per lane where `big`) to its
+// share of the record store, and their blocks to its share of the block list.
 // False in a lane whose record found no place (a fixed record store).
 __device__ __forceinline__ bool append_large(const FrameParams& F, const Setup& S, bool big, uint32_t id) {
   const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
   const unsigned m = __ballot_sync(0xffffffffu, big);
   if (m == 0) return true;
   unsigned base = 0;
-  if (lane == 0) base = atomicAdd(&F.counters->rec_count, (unsigned)__popc(m));
+  if (lane == 0) base = atomicAdd(&F.counters->share[warp_share()].rec_count, (unsigned)__popc(m));
   base = __shfl_sync(0xffffffffu, base, 0);
   unsigned n_items = 0;
-  const unsigned slot = base + __popc(m & lt);
-  const bool placed = slot < F.rec_cap;
+  const bool placed = base + __popc(m & lt) < F.rec_share;
+  base += warp_share() * F.rec_share;
   if (big && placed) {
-    F.recs[slot] = to_rec(S, id);
-    n_items = (unsigned)(((S.y1 - S.y0) / kLargeRows + 1) * large_segs(S.x0, S.x1));
+    F.recs[base + __popc(m & lt)] = to_rec(S, id);
+    n_items = (unsigned)large_blocks(S.x0, S.y0, S.x1, S.y1);
   }
   // the blocks: one range per warp, each lane's at its exclusive prefix,
   // written by all lanes (a screen-sized triangle has hundreds)
@@ -1098,9 +1106,11 @@ __device__ __forceinline__ bool append_large(const FrameParams& F, const Setup& 
     if (lane >= (unsigned)o) inc += u;
   }
   const unsigned total = __shfl_sync(0xffffffffu, inc, 31);
+  if (total == 0) return placed || !big;
   unsigned long long ibase = 0;
-  if (lane == 0 && total) ibase = atomicAdd(&F.counters->item_count, (unsigned long long)total);
+  if (lane == 0) ibase = atomicAdd(&F.counters->share[warp_share()].item_count, (unsigned long long)total);
   ibase = __shfl_sync(0xffffffffu, ibase, 0);
+  LargeItem* items = F.items + (size_t)warp_share() * F.item_share;
   for (unsigned b = 0; b < total; b += 32) {
     const unsigned i = b + lane;
     unsigned own = 0;  // the lane whose record block i belongs to
@@ -1112,8 +1122,8 @@ __device__ __forceinline__ bool append_large(const FrameParams& F, const Setup& 
     const LargeItem item{base + __popc(m & ((1u << own) - 1u)), k};
     // blocks past the end of the list: the record's remaining ones go to the
     // spill list (one entry per record, so it cannot overflow)
-    if (ibase + i < F.item_cap) F.items[ibase + i] = item;
-    else if (k == 0 || ibase + i == F.item_cap) F.spill[atomicAdd(&F.counters->spill_count, 1u)] = item;
+    if (ibase + i < F.item_share) items[ibase + i] = item;
+    else if (k == 0 || ibase + i == F.item_share) F.spill[atomicAdd(&F.counters->spill_count, 1u)] = item;
   }
   return placed || !big;
 }
@@ -1129,17 +1139,14 @@ __device__ __forceinline__ const DevRenderable& renderable(const FrameParams& F,
 
 // Blocks of 256 threads per SM the register budget of the setup kernels must
 // allow.  With the vertex pass the kernel waits on index -> vertex gathers
-// and more resident warps hide that, at the price of spills: 5 in frames
-// (1080p mesh: 42.5 us, 44.6 with 6), 6 in batches, which spill more either
-// way (256 scenes: 420 us, 446 with 5); with the packed staging records, which
-// leave more L1 to the spills.  Without it (triangle soups) it is bound by its
-// strided position loads and by instruction issue, spilling and a smaller L1
-// cost more than the extra warps hide, and the aligned records' vector copies
-// are cheaper: 4 (64 registers).
+// and more resident warps hide that, until they spill: 5 (1080p mesh: 42.5
+// us, 44.6 with 6), with the packed staging records, which leave more of the
+// L1.  Without it (triangle soups) it is bound by its strided position loads
+// and by instruction issue, spilling and a smaller L1 cost more than the extra
+// warps hide, and the aligned records' vector copies are cheaper: 4 (64
+// registers).
 template <bool PRE>
 constexpr int kSetupMinBlocks = PRE ? 5 : 4;
-template <bool PRE>
-constexpr int kSetupBatchMinBlocks = PRE ? 6 : 4;
 template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup(FrameParams F) {
   pdl_wait();
@@ -1215,16 +1222,32 @@ __device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, u
 __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
   pdl_wait();
   pdl_trigger();
-  const uint32_t n = (uint32_t)min(F.counters->item_count, (unsigned long long)F.item_cap);
+  // the shares' blocks in one numbering: lane l holds the end of share l's, and
+  // a warp takes every nw-th block of all of them
+  const int lane = (int)(threadIdx.x & 31);
+  const uint32_t mine =
+      lane < kShares ? (uint32_t)min(F.counters->share[lane].item_count, (unsigned long long)F.item_share) : 0u;
+  uint32_t end = mine;
+#pragma unroll
+  for (int o = 1; o < kShares; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xffffffffu, end, o, kShares);
+    if (lane % kShares >= o) end += u;
+  }
+  const uint32_t n = __shfl_sync(0xffffffffu, end, kShares - 1);
   const uint32_t n_spill = F.counters->spill_count;
   const bool persp = F.v.persp != 0;
   const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
   const uint32_t w0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (uint32_t it = w0; it < n; it += nw) raster_block(F, persp, F.items[it].rec, F.items[it].k);
+  for (uint32_t it = w0; it < n; it += nw) {
+    const int own = __popc(__ballot_sync(0xffffffffu, lane < kShares && end <= it));
+    const uint32_t at = it - __shfl_sync(0xffffffffu, end - mine, own);
+    const LargeItem item = F.items[(size_t)own * F.item_share + at];
+    raster_block(F, persp, item.rec, item.k);
+  }
   for (uint32_t it = w0; it < n_spill; it += nw) {
     const LargeItem item = F.spill[it];
     const BigRec& R = F.recs[item.rec];
-    const uint32_t blocks = (uint32_t)(((R.y1 - R.y0) / kLargeRows + 1) * large_segs(R.x0, R.x1));
+    const uint32_t blocks = (uint32_t)large_blocks(R.x0, R.y0, R.x1, R.y1);
     for (uint32_t k = item.k; k < blocks; k++) raster_block(F, persp, item.rec, k);
   }
 }
@@ -1294,13 +1317,10 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
 // (the register budget and staging layout of k_setup, for the same reasons;
 // on the 256-scene batch: 0.665 -> 0.453 ms)
 template <bool PRE>
-__global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> * 256 / kSetupBatchThreads) k_setup_batch(BatchParams B) {
+__global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup_batch(BatchParams B) {
   using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;
-  __shared__ Rec s_rec[kSetupBatchThreads / 32][kStageRecs];
-  __shared__ int s_pre[kSetupBatchThreads / 32][kStageRecs];
-  __shared__ unsigned s_fill, s_base;
-  if (threadIdx.x == 0) s_fill = 0;
-  __syncthreads();
+  __shared__ Rec s_rec[kSetupThreads / 32][kStageRecs];
+  __shared__ int s_pre[kSetupThreads / 32][kStageRecs];
   const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
   const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << B.tri_shift) + lane;
   uint32_t scene = 0;
@@ -1325,24 +1345,15 @@ __global__ void __launch_bounds__(kSetupBatchThreads, kSetupBatchMinBlocks<PRE> 
     if (PRE && (small || big)) note_triangle(B.g, *R, rk, (int)(g - R->tri_base));
     if (sub == 0 && n_sub < 0) atomicOr(&B.counters->error_flags, 1u);
     count_triangles(B.counters, small, big, sub == 0 && cut && n_sub > 0);
-    // record slots: in the first round each warp reserves within the block
-    // and the block once globally
+    // record slots, one reservation per warp in its share of the store
     const unsigned m = __ballot_sync(0xffffffffu, big);
     unsigned base = 0;
-    if (sub == 0) {
-      if (lane == 0 && m) base = atomicAdd(&s_fill, (unsigned)__popc(m));
-      __syncthreads();
-      if (threadIdx.x == 0) s_base = s_fill ? atomicAdd(&B.counters->rec_count, s_fill) : 0;
-      __syncthreads();
-      base += s_base;
-    } else if (lane == 0 && m) {
-      base = atomicAdd(&B.counters->rec_count, (unsigned)__popc(m));
-    }
+    if (lane == 0 && m) base = atomicAdd(&B.counters->share[warp_share()].rec_count, (unsigned)__popc(m));
     base = __shfl_sync(0xffffffffu, base, 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
     if (big) {
-      const unsigned slot = base + __popc(m & lt);
-      if (slot < B.rec_cap) {
+      const unsigned at = base + __popc(m & lt), slot = warp_share() * B.rec_share + at;
+      if (at < B.rec_share) {
         B.recs[slot] = to_rec(S, id);
         B.rec_scene[slot] = scene;
         const SceneRec& SR = B.scenes[scene];
@@ -1465,8 +1476,11 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   }
   grid.sync();
   // 2. scatter
-  const uint32_t nrec = min(B.counters->rec_count, B.rec_cap);
-  for (uint32_t i = blockIdx.x * nt + threadIdx.x; i < nrec; i += nb * nt) {
+  const uint32_t gw = (blockIdx.x * nt + threadIdx.x) >> 5, share = gw % kShares;
+  const uint32_t nrec = min(B.counters->share[share].rec_count, B.rec_share);
+  const uint32_t per = (nb * (nt >> 5) + kShares - 1 - share) / kShares;  // warps on this share
+  for (uint32_t r = (gw / kShares) * 32 + lane; r < nrec; r += per * 32) {
+    const uint32_t i = share * B.rec_share + r;
     const BigRec& R = B.recs[i];
     const SceneRec& SR = B.scenes[B.rec_scene[i]];
     int tx0 = R.x0 / TW, tx1 = R.x1 / TW, ty0 = R.y0 / TH, ty1 = R.y1 / TH;
@@ -1783,9 +1797,9 @@ cudaError_t launch_batch(const BatchParams& B, int threads, int grid, cudaStream
   if (B.g.n_tris) {
     BatchParams Bs = B;
     Bs.tri_shift = triangle_shift(B.g.n_tris);
-    const int sgrid = grid_for((size_t)B.g.n_tris << (5 - Bs.tri_shift), kSetupBatchThreads);
-    if (pre) k_setup_batch<true><<<sgrid, kSetupBatchThreads, 0, st>>>(Bs);
-    else k_setup_batch<false><<<sgrid, kSetupBatchThreads, 0, st>>>(Bs);
+    const int sgrid = grid_for((size_t)B.g.n_tris << (5 - Bs.tri_shift), kSetupThreads);
+    if (pre) k_setup_batch<true><<<sgrid, kSetupThreads, 0, st>>>(Bs);
+    else k_setup_batch<false><<<sgrid, kSetupThreads, 0, st>>>(Bs);
   }
   if (ev) cudaEventRecord(ev[2], st);
   // strips of 256 pixels, cut to 128 or 64 where that would leave a warp fewer

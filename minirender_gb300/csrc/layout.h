@@ -115,16 +115,25 @@ struct alignas(32) StatSlot {
   unsigned long long clipped;  // triangles cut by the near plane
 };
 
+// Counters of one share of the record store and of the block list.  Every warp
+// of the setup waits for these, so they are spread, too: on one address an
+// update takes some 2 ns, 10 us of the setup of 327,680 triangles of 18
+// pixels.  (64 shares cost the large raster 2 us to add up, 16 cost none.)
+constexpr int kShares = 16;
+struct alignas(32) ShareSlot {
+  unsigned long long item_count;  // large-triangle blocks requested (single frames; 64 bits: a frame
+                                  // of many screen-sized triangles passes 2^32)
+  unsigned int rec_count;         // records requested
+};
+
 struct Counters {
   StatSlot stat[kStatSlots];
+  ShareSlot share[kShares];
   unsigned int error_flags;
-  unsigned int rec_count;      // records written
   unsigned int bin_needed;     // total (tile, record) pairs requested
   unsigned int bin_overflow;
   unsigned int work_next;      // persistent-kernel work counter
   unsigned int spill_count;    // records whose remaining blocks did not fit the block list
-  unsigned long long item_count;  // large-triangle blocks requested (single frames; 64 bits: a
-                                  // frame of many screen-sized triangles passes 2^32)
 };
 
 // One-frame launch.
@@ -142,6 +151,11 @@ constexpr int kLargeRows = 32;
 // columns, 14 with 32, 12 with 16.)
 constexpr int kLargeCols = 16, kLargeSegs = 16;
 
+// Records per share in which T triangles always find room: a share's warps hold
+// at most T / kShares + 64 of them (setup warps, 2 to 32 triangles each, take
+// shares in turn), two sub-triangles each.
+inline size_t rec_share_for(size_t T) { return T / (kShares / 2) + 128; }
+
 struct FrameParams {
   View v;
   Geo g;
@@ -150,10 +164,10 @@ struct FrameParams {
   int tri_shift;              // log2 of the triangles a warp of the setup kernel takes
   unsigned long long* vis;    // W*H
   BigRec* recs;               // large sub-triangles
-  uint32_t rec_cap;
-  LargeItem* items;           // their row blocks
-  uint32_t item_cap;
-  LargeItem* spill;           // rec_cap entries: records past the end of items[]
+  uint32_t rec_share;         // of these, records per share
+  LargeItem* items;           // their blocks
+  uint32_t item_share;        // of these, blocks per share
+  LargeItem* spill;           // an entry per record: records whose blocks did not fit items[]
   const uint4* stage_src;     // the frame's staging block in mapped pinned host memory (several
   uint4* stage_dst;           // renderables), fetched by the clear kernel (no copy-engine transfer)
   uint32_t stage_n16;         // its size in 16-byte units
@@ -190,7 +204,7 @@ struct BatchParams {
   int small_max;                    // bbox pixels up to which the setup kernel rasterises (0: none)
   unsigned long long* vis;          // all scenes' visibility words (small_max > 0)
   BigRec* recs;
-  uint32_t rec_cap;
+  uint32_t rec_share;               // of these, records per share
   uint32_t* rec_scene;              // scene of each record
   uint32_t* tile_count;             // n_tiles
   uint32_t* tile_start;             // n_tiles + 1

@@ -146,9 +146,9 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
   F.one = R;
   F.vis = (unsigned long long*)(S + kVisOff);
   F.recs = (BigRec*)(S + kRecOff);
-  F.rec_cap = kRecCap;
+  F.rec_share = kRecCap / kShares;
   F.items = (LargeItem*)(S + kItemOff);
-  F.item_cap = kItemCap;
+  F.item_share = kItemCap / kShares;
   F.spill = (LargeItem*)(S + kSpillOff);
   F.rgb8 = rgb8;
   F.depth = depth;

@@ -157,3 +157,23 @@ def test_shared_indices_with_unused_tail(product_lib, meshes):
     for lighting, texturing, point in ((True, True, False), (True, False, True), (False, True, False), (False, False, False)):
         st.lighting, st.texturing, st.light_is_point = lighting, texturing, point
         _same(_render(st, sc), O.render(st, sc), f"lighting {lighting}, texturing {texturing}, point {point}")
+
+
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_record_shares(product_lib, noalloc):
+    """More large triangles in one part of the triangle list than a share of
+    the fixed record store holds (the rest is rasterised by the setup), beside
+    parts with none; in the growing store every one finds room."""
+    import test_zz_no_alloc as N
+    st, sc = N._strips(5000, 640, 480, 9)
+    m = sc.children[0]
+    v = m.vertices.reshape(-1, 3, 3).copy()
+    t = np.arange(len(v))
+    v[(t // 32) % 16 > 2] *= np.float32([0.02, 0.02, 1])  # small ones outside three shares of sixteen
+    v = np.concatenate([v, np.tile(v[:96], (120, 1, 1))])  # and the large ones of those, again and again
+    idx = np.arange(3 * len(v), dtype=np.int32)
+    nrm = np.tile(np.array([[0.2, 0.3, 1]], np.float32), (3 * len(v), 1))
+    sc.children = [S.TriMesh(v.reshape(-1, 3), nrm, idx, normalsI=idx, material=m.material)]
+    ref = O.render(st, sc)
+    got = N._noalloc(st, sc, calls=1)[0] if noalloc else _render(st, sc)
+    _same(got, ref, "strips")
