@@ -46,7 +46,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 #include <utility>
 
 #include "raster.cuh"
@@ -270,7 +269,9 @@ constexpr uint32_t kRecPerFace = 1u;
 // 344-348, 356-373).  A per-face record needs its first 64 bytes only.
 __device__ __forceinline__ void corners_rec(const DevRenderable& R, int t, Vtx (&v)[3]) {
   const float4* r = R.mesh.rec + (size_t)8 * t;
-  const float4 q0 = __ldg(r), q1 = __ldg(r + 1), q2 = __ldg(r + 2), q3 = __ldg(r + 3);
+  float4 q0, q1, q2, q3;  // two 32-byte loads
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(q0.x), "=f"(q0.y), "=f"(q0.z), "=f"(q0.w), "=f"(q1.x), "=f"(q1.y), "=f"(q1.z), "=f"(q1.w) : "l"(r));
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=f"(q2.x), "=f"(q2.y), "=f"(q2.z), "=f"(q2.w), "=f"(q3.x), "=f"(q3.y), "=f"(q3.z), "=f"(q3.w) : "l"(r + 2));
   v[0].pos = affine(R.mv, v3(q0.x, q0.y, q0.z));
   v[1].pos = affine(R.mv, v3(q0.w, q1.x, q1.y));
   v[2].pos = affine(R.mv, v3(q1.z, q1.w, q2.x));
@@ -577,13 +578,13 @@ __device__ __forceinline__ bool sub_setup(const View& V, const Geo& G, const Dev
   Vtx v[3];
   int ip[3];
   if (PRE) {
+    float4 a[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) ip[c] = (int)R.vert_base + __ldg(R.mesh.idx + 3 * t + c);
     if (bad_triangle(R.mesh, t)) {
       n_sub = -1;
       return false;
     }
-    float4 a[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) ip[c] = (int)R.vert_base + __ldg(R.mesh.idx + 3 * t + c);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       a[c] = G.va[(uint32_t)ip[c]];
@@ -899,63 +900,8 @@ __global__ void __launch_bounds__(256) k_vertex(Geo G, View V, const SceneRec* s
   }
 }
 
-// Small-triangle records staged in shared memory for the warp's cooperative
-// raster, in two layouts: SmallRec (80 bytes, 16-byte aligned, copied with
-// vector accesses) and PackedRec (60 bytes: pixel coordinates in 16 bits, an
-// odd word stride so lanes touching different records still hit different
-// banks), which leaves more of the SM's L1 to a kernel that spills.
-struct __align__(16) SmallRec {
-  float p0x, p0y, p2x, p2y, n1x, n1y, n2x, n2y, z0, z1, z2;
-  uint32_t id;
-  int x0, y0, x1, rows;
-  uint32_t tag;  // target frame (batches: scene)
-};
-struct PackedRec {
-  float p0x, p0y, p2x, p2y, n1x, n1y, n2x, n2y, z0, z1, z2;
-  uint32_t id;
-  uint32_t tag;
-  uint32_t lo;  // x0 | y0 << 16
-  uint32_t hi;  // x1 | rows << 16
-};
-__device__ __forceinline__ void rec_put(SmallRec& q, const Setup& S, uint32_t id, uint32_t tag) {
-  q.p0x = S.p0.x; q.p0y = S.p0.y; q.p2x = S.p2.x; q.p2y = S.p2.y;
-  q.n1x = S.n1.x; q.n1y = S.n1.y; q.n2x = S.n2.x; q.n2y = S.n2.y;
-  q.z0 = S.z[0]; q.z1 = S.z[1]; q.z2 = S.z[2];
-  q.id = id;
-  q.x0 = S.x0; q.y0 = S.y0; q.x1 = S.x1;
-  q.rows = S.y1 - S.y0 + 1;
-  q.tag = tag;
-}
-__device__ __forceinline__ void rec_put(PackedRec& q, const Setup& S, uint32_t id, uint32_t tag) {
-  q.p0x = S.p0.x; q.p0y = S.p0.y; q.p2x = S.p2.x; q.p2y = S.p2.y;
-  q.n1x = S.n1.x; q.n1y = S.n1.y; q.n2x = S.n2.x; q.n2y = S.n2.y;
-  q.z0 = S.z[0]; q.z1 = S.z[1]; q.z2 = S.z[2];
-  q.id = id;
-  q.tag = tag;
-  // frame coordinates and small boxes' row counts fit 16 bits (sides <= 65536)
-  q.lo = (uint32_t)S.x0 | ((uint32_t)S.y0 << 16);
-  q.hi = (uint32_t)S.x1 | ((uint32_t)(S.y1 - S.y0 + 1) << 16);
-}
-__device__ __forceinline__ int rec_rows(const SmallRec& q) { return q.rows; }
-__device__ __forceinline__ int rec_rows(const PackedRec& q) { return (int)(q.hi >> 16); }
-template <class Rec>
-__device__ __forceinline__ Setup rec_get(const Rec& q) {
-  Setup U;
-  U.p0 = v2(q.p0x, q.p0y); U.p2 = v2(q.p2x, q.p2y);
-  U.n1 = v2(q.n1x, q.n1y); U.n2 = v2(q.n2x, q.n2y);
-  U.z[0] = q.z0; U.z[1] = q.z1; U.z[2] = q.z2;
-  if constexpr (sizeof(Rec) == sizeof(PackedRec)) {
-    U.x0 = (int)(q.lo & 0xffffu); U.y0 = (int)(q.lo >> 16); U.x1 = (int)(q.hi & 0xffffu);
-  } else {
-    U.x0 = q.x0; U.y0 = q.y0; U.x1 = q.x1;
-  }
-  return U;
-}
-constexpr int kStageRecs = 32;  // records staged per warp and round
-
 // Threads per block of the setup kernels.  Their warps share nothing
-// (statistics go to slots, staging is per warp, records are reserved by a warp
-// at a time), and a block keeps its place until its slowest warp is done:
+// (statistics go to slots, records are reserved by a warp at a time), and a block keeps its place until its slowest warp is done:
 // 1080p mesh setup 48.8 us with 256 threads, 46.6 with 128, 44.6 with 64; 10M-
 // triangle soup 378, 368, 366 us; 256 scenes 387 us with 128 threads and
 // records reserved by the block, 379 so.
@@ -963,6 +909,7 @@ constexpr int kSetupThreads = 64;
 
 // Where small triangles' fragments go: the frame's visibility buffer...
 struct FrameTarget {
+  static constexpr bool one = true;  // (every tag is 0)
   unsigned long long* vis;
   int W;
   bool persp;
@@ -972,6 +919,7 @@ struct FrameTarget {
 };
 // ...or, in a batch, the visibility buffer of the triangle's scene (tag).
 struct BatchTarget {
+  static constexpr bool one = false;
   const SceneRec* scenes;
   __device__ unsigned long long* row(uint32_t sc, int y) const {
     return scenes[sc].vis + (size_t)y * scenes[sc].v.W;
@@ -1030,54 +978,59 @@ __device__ __forceinline__ void raster_tiny(const Setup& Q, bool persp, uint32_t
   }
 }
 
-// Raster of the warp's small sub-triangles (one per lane where `on`), whose
-// frame is `tag`, with 64-bit atomicMin into the target (src/Renderer.cpp:
-// 238-269).  When every one in the warp spans at most 4x4 pixels the lanes
-// rasterise their own (the loops are short and nearly uniform); otherwise
-// they are staged in shared memory and rasterised with one (triangle, row)
-// per lane so every lane has work.  Called by all lanes of the warp.
-template <class Target, class Rec>
-__device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t id, uint32_t tag, const Target& T,
-                                             Rec* s_rec, int* s_pre) {
-  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+// Raster of the warp's small sub-triangles (one per lane where `on`; ids step
+// by two from lane to lane), whose frame is `tag`, with 64-bit atomicMin into
+// the target (src/Renderer.cpp:238-269).  When every one in the warp spans at
+// most 4x4 pixels the lanes rasterise their own (LIST: see raster_tiny);
+// otherwise their rows are numbered by a prefix sum and taken one per lane,
+// each lane fetching its row's setup from the lane that holds it.  (Staged in
+// shared memory, the setups cost the vertex gathers 4 KB of L1 a block: 1080p
+// mesh 42.5 us, 40.1 so; 256 scenes 375 and 366.)  Called by all lanes.
+template <bool LIST, class Target>
+__device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t id, uint32_t tag, const Target& T) {
+  const unsigned lane = threadIdx.x & 31;
   const unsigned m = __ballot_sync(0xffffffffu, on);
   if (m == 0) return;
   const int span = on ? max(S.x1 - S.x0, S.y1 - S.y0) + 1 : 0;
   if (__reduce_max_sync(0xffffffffu, (unsigned)span) <= 4u) {
-    constexpr bool list = std::is_same_v<Rec, SmallRec>;
-    if (on) raster_tiny<list>(S, T.perspective(tag), id, [&](int y) { return T.row(tag, y); });
+    if (on) raster_tiny<LIST>(S, T.perspective(tag), id, [&](int y) { return T.row(tag, y); });
     return;
   }
-  const int n = __popc(m);
-  if (on) rec_put(s_rec[__popc(m & lt)], S, id, tag);
-  __syncwarp();
-  const int c = (int)lane < n ? rec_rows(s_rec[lane]) : 0;
-  int inc = c;
+  const int rows = on ? S.y1 - S.y0 + 1 : 0;
+  int inc = rows;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int u = __shfl_up_sync(0xffffffffu, inc, o);
     if ((int)lane >= o) inc += u;
   }
   const int total = __shfl_sync(0xffffffffu, inc, 31);
-  s_pre[lane] = inc - c;
-  __syncwarp();
+#pragma unroll 1
   for (int b = 0; b < total; b += 32) {
-    const int k = b + (int)lane;
-    if (k < total) {
-      int lo = 0;  // the last record lo < n with s_pre[lo] <= k
+    const int i = b + (int)lane;
+    int own = 0;  // the lane whose record row i belongs to
 #pragma unroll
-      for (int step = 16; step; step >>= 1)
-        if (lo + step < n && s_pre[lo + step] <= k) lo += step;
-      const Rec& q = s_rec[lo];
-      const Setup U = rec_get(q);
-      const int y = U.y0 + (k - s_pre[lo]);
-      const uint32_t tg = q.tag;
+    for (int step = 16; step; step >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= i) own += step;
+    const int k = i - __shfl_sync(0xffffffffu, inc - rows, own);
+    Setup U;
+    U.p0 = v2(__shfl_sync(0xffffffffu, S.p0.x, own), __shfl_sync(0xffffffffu, S.p0.y, own));
+    U.p2 = v2(__shfl_sync(0xffffffffu, S.p2.x, own), __shfl_sync(0xffffffffu, S.p2.y, own));
+    U.n1 = v2(__shfl_sync(0xffffffffu, S.n1.x, own), __shfl_sync(0xffffffffu, S.n1.y, own));
+    U.n2 = v2(__shfl_sync(0xffffffffu, S.n2.x, own), __shfl_sync(0xffffffffu, S.n2.y, own));
+#pragma unroll
+    for (int c = 0; c < 3; c++) U.z[c] = __shfl_sync(0xffffffffu, S.z[c], own);
+    // (frame coordinates fit 16 bits: sides <= 65536)
+    const uint32_t at = __shfl_sync(0xffffffffu, (uint32_t)S.x0 | ((uint32_t)S.y0 << 16), own);
+    U.x0 = (int)(at & 0xffffu);
+    U.x1 = __shfl_sync(0xffffffffu, S.x1, own);
+    const uint32_t tg = T.one ? 0u : __shfl_sync(0xffffffffu, tag, own);
+    if (i < total) {
+      const int y = (int)(at >> 16) + k;
       unsigned long long* row = T.row(tg, y);
-      walk_row(U, T.perspective(tg), q.id, y, U.x0, U.x1,
+      walk_row(U, T.perspective(tg), id + 2u * (uint32_t)(own - (int)lane), y, U.x0, U.x1,
                [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
     }
   }
-  __syncwarp();  // s_rec / s_pre free for the warp's next use
 }
 
 // Appends the warp's large sub-triangles (one per lane where `big`) to its
@@ -1140,20 +1093,15 @@ __device__ __forceinline__ const DevRenderable& renderable(const FrameParams& F,
 // Blocks of 256 threads per SM the register budget of the setup kernels must
 // allow.  With the vertex pass the kernel waits on index -> vertex gathers
 // and more resident warps hide that, until they spill: 5 (1080p mesh: 42.5
-// us, 44.6 with 6), with the packed staging records, which leave more of the
-// L1.  Without it (triangle soups) it is bound by its strided position loads
-// and by instruction issue, spilling and a smaller L1 cost more than the extra
-// warps hide, and the aligned records' vector copies are cheaper: 4 (64
-// registers).
+// us, 44.6 with 6).  Without it (triangle soups) it is bound by its strided
+// position loads and by instruction issue, and spilling and a smaller share of
+// the L1 cost more than the extra warps hide: 4 (64 registers).
 template <bool PRE>
 constexpr int kSetupMinBlocks = PRE ? 5 : 4;
 template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup(FrameParams F) {
   pdl_wait();
-  using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;  // see kSetupMinBlocks
-  __shared__ Rec s_rec[kSetupThreads / 32][kStageRecs];
-  __shared__ int s_pre[kSetupThreads / 32][kStageRecs];
-  const unsigned w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const unsigned lane = threadIdx.x & 31;
   const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << F.tri_shift) + lane;
   const bool in = lane < (1u << F.tri_shift) && g < F.g.n_tris;
   const uint32_t k = ONE ? 0u : (uint32_t)find_base_warp(F.g.tri_base, F.g.n_renderables, min(g, F.g.n_tris - 1));
@@ -1174,7 +1122,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
     count_triangles(F.counters, small, big, sub == 0 && cut && n_sub > 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
     if (!append_large(F, S, big, id)) small = true;  // rasterised here, as small ones are
-    raster_small(S, small, id, 0u, FrameTarget{F.vis, F.v.W, F.v.persp != 0}, s_rec[w], s_pre[w]);
+    raster_small<!PRE>(S, small, id, 0u, FrameTarget{F.vis, F.v.W, F.v.persp != 0});
   }
 }
 
@@ -1314,14 +1262,9 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
 // ---------------------------------------------------------------- batches
 // Setup of every triangle of every scene: each sub-triangle with pixels to
 // test becomes a record (warp-compacted), counted into its scene's tiles.
-// (the register budget and staging layout of k_setup, for the same reasons;
-// on the 256-scene batch: 0.665 -> 0.453 ms)
 template <bool PRE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup_batch(BatchParams B) {
-  using Rec = std::conditional_t<PRE, PackedRec, SmallRec>;
-  __shared__ Rec s_rec[kSetupThreads / 32][kStageRecs];
-  __shared__ int s_pre[kSetupThreads / 32][kStageRecs];
-  const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5, lt = (1u << lane) - 1u;
+  const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
   const uint32_t g = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << B.tri_shift) + lane;
   uint32_t scene = 0;
   const bool in = lane < (1u << B.tri_shift) && g < B.g.n_tris;
@@ -1363,7 +1306,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
             atomicAdd(B.tile_count + SR.tile_base + ty * SR.tiles_x + tx, 1u);
       }
     }
-    if (B.small_max > 0) raster_small(S, small, id, scene, BatchTarget{B.scenes}, s_rec[w], s_pre[w]);
+    if (B.small_max > 0) raster_small<!PRE>(S, small, id, scene, BatchTarget{B.scenes});
   }
 }
 
