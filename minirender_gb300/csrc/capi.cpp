@@ -1144,9 +1144,9 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   CK(B.rec_scene.ensure(share * kShares), "batch records");
   CK(B.tiles.ensure(3 * tiles + 1), "batch tiles");
   if (B.small_max > 0) {
-    const void* before = B.vis.p;
+    // a grown buffer may come back at the old address, so its size tells
+    if (pixels > B.vis.cap) B.vis_empty = false;
     CK(B.vis.ensure(pixels), "batch visibility");
-    if (B.vis.p != before) B.vis_empty = false;
   }
   if (B.bins.cap < std::max<size_t>((size_t)1 << 20, 2 * tris))
     CK(B.bins.ensure(std::max<size_t>((size_t)1 << 20, 2 * tris)), "batch bins");

@@ -177,3 +177,20 @@ def test_record_shares(product_lib, noalloc):
     ref = O.render(st, sc)
     got = N._noalloc(st, sc, calls=1)[0] if noalloc else _render(st, sc)
     _same(got, ref, "strips")
+
+
+def test_batches_of_growing_and_shrinking_frames(product_lib):
+    """A batch leaves the visibility words empty for the next one; the words a
+    larger batch adds (its buffer grown, maybe in place) are cleared first."""
+    from minirender_gb300 import workloads as W
+    from minirender_gb300.batch import BatchRenderer
+    br = BatchRenderer(0)
+    try:
+        for w, h in ((64, 48), (65, 49), (400, 301), (31, 17), (801, 602), (801, 602)):
+            item = W.config4_scene(w, 8, (w, h))
+            br.render([item, item])
+            ref = O.render(*item)
+            for k in range(2):
+                _same(br.read(k), ref, f"{w}x{h} scene {k}")
+    finally:
+        br.close()
