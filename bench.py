@@ -293,7 +293,7 @@ STAGES = ["clear+vertex", "setup", "large_raster", "-", "resolve"]
 TUNING_KEYS = ("tile_w", "tile_h", "threads", "chunk", "small_max")
 # kernels between the stage events of one plain frame ("-" is an empty
 # interval kept so the stage list keeps its five slots)
-KERNELS = {"clear+vertex": "k_clear+k_vertex", "setup": "k_setup", "large_raster": "k_raster_large",
+KERNELS = {"clear+vertex": "k_begin", "setup": "k_setup", "large_raster": "k_raster_large",
            "-": "k_raster_large", "resolve": "k_resolve"}
 
 
@@ -822,7 +822,7 @@ def gpu_arm(args, ws, rank, local):
     alg = {
         "clear+vertex": 8 * P + (12 * V + 24 * V + 16 * V if vertex_pass else 0),
         "setup": 12 * T + 12 * V + 64 * n_big,
-        # row blocks (8 B each) and their records; the vis words it updates
+        # blocks (8 B each) and their records; the vis words it updates
         # are the clear's, resident in L2
         "large_raster": 8 * int(stats.bin_entries) + 64 * n_big,
         "-": 0,
@@ -871,8 +871,9 @@ def gpu_arm(args, ws, rank, local):
         "counters": {"clipped": int(stats.clipped), "rasterised": int(stats.rasterised),
                      "small_direct": int(stats.small_direct), "binned": int(stats.binned),
                      "bin_entries": int(stats.bin_entries)},
-        # k_clear, [k_vertex], k_setup, k_raster_large, k_resolve per frame
-        "gpu_launches": (5 if vertex_pass else 4) * args.steps,
+        # k_begin, [k_vertex], k_setup, k_raster_large, k_resolve per frame; a
+        # frame of one renderable has its vertex pass in k_begin
+        "gpu_launches": (5 if vertex_pass and n != 1 else 4) * args.steps,
         "clocks": clk,
     }
     if args.views > 0 and not args.no_e2e:

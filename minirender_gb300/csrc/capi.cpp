@@ -4,10 +4,10 @@
 // Memory: the context owns every device buffer.  Meshes and textures are
 // allocated once at upload; frame buffers grow to the largest frame seen and
 // are then reused, so steady-state frames allocate nothing.  The one
-// single-frame buffer whose size is data dependent -- the list of 32-row
-// blocks of large triangles -- is checked on the device: blocks past its end
-// go to a per-record spill list (which cannot overflow), and the list grows
-// for later frames.  Batches keep a (tile, record) list; an overflow there is
+// single-frame buffer whose size is data dependent -- the list of blocks
+// (32 rows by a column segment) of large triangles -- is checked on the
+// device: blocks past the end of their share of it go to a per-record spill
+// list (which cannot overflow), and the list grows for later frames.  Batches keep a (tile, record) list; an overflow there is
 // detected at the next synchronisation and the batch is re-run.
 #include <unistd.h>
 
@@ -615,7 +615,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     h_tbase = c->h_tri_base;
   }
   uint32_t base = 0;
-  uint64_t vbase = 0, nbase = 0;
+  uint64_t vbase = 0, nbase = 0, normals = 0;  // normals: all of them; nbase: those with a buffer of their own
   uint32_t* h_vbase = h_tbase + (n + 1);
   uint32_t* h_nbase = h_tbase + 2 * (n + 1);
   for (int32_t i = 0; i < n; i++) {
@@ -639,7 +639,8 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     h_vbase[i] = (uint32_t)vbase;
     h_nbase[i] = (uint32_t)nbase;
     vbase += (uint64_t)m.d.n_pos;
-    if (vbase >= ((uint64_t)1 << 32))
+    normals += (uint64_t)m.d.n_nrm;
+    if (vbase >= ((uint64_t)1 << 32) || normals >= ((uint64_t)1 << 32))
       return fail(c, MR_E_INVALID, "more than 2^32-1 vertices or normals in one frame");
     const mr_material& M = rs[i].material;
     memcpy(R.diffuse, M.diffuse, sizeof(R.diffuse));
@@ -660,7 +661,6 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
     }
     set_reads(R);
     if (!R.unified) nbase += (uint64_t)m.d.n_nrm;
-    if (nbase >= ((uint64_t)1 << 32)) return fail(c, MR_E_INVALID, "more than 2^32-1 vertices or normals in one frame");
   }
   h_tbase[n] = base;
   h_vbase[n] = (uint32_t)vbase;
@@ -760,7 +760,7 @@ constexpr size_t kMaxItems = (size_t)1 << 26;
 // mr_read_async completes here: its counter copy was queued behind the frame
 // and its output copies before the read_done event (work queued on the
 // stream after them, such as the next frame's mesh upload, is not waited
-// for).  A frame whose row blocks overflowed the list was still rasterised
+// for).  A frame whose blocks overflowed the list was still rasterised
 // completely (through the spill list); the list grows for the next frames.
 static int settle(mr_ctx* c) {
   if (!c->have_frame) return fail(c, MR_E_INVALID, "no frame rendered yet");
@@ -1036,14 +1036,17 @@ static int batch_launch(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling
 
 // batch_launch with the visibility words it starts from empty: a batch leaves
 // them so (a separate clear of every scene's words was 110 us of a 256-scene
-// batch), unless the buffer is new or a launch failed.
+// batch), unless the buffer is new, a launch failed or the batch is only
+// recorded (into the caller's capture of st, which then clears at each replay).
 int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
-  if (B.small_max > 0 && !B.vis_empty) {  // a new buffer, or a batch that was not completed
+  cudaStreamCaptureStatus cap;
+  CK(cudaStreamIsCapturing(st, &cap), "capture status");
+  const bool runs = cap == cudaStreamCaptureStatusNone;
+  if (B.small_max > 0 && !(B.vis_empty && runs))
     CK(cudaMemsetAsync(B.vis.p, 0xFF, B.vis.cap * sizeof(unsigned long long), st), "visibility clear");
-  }
   B.vis_empty = false;
   const int rc = batch_launch(c, B, st, profiling, ev);
-  B.vis_empty = rc == MR_OK;
+  B.vis_empty = rc == MR_OK && runs;
   return rc;
 }
 
@@ -1075,7 +1078,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   if (!B.h_cnt) CK(cudaMallocHost(&B.h_cnt, sizeof(Counters)), "batch counters");
   if (!B.done) CK(cudaEventCreateWithFlags(&B.done, cudaEventDisableTiming), "batch event");
   if (!B.staged) CK(cudaEventCreateWithFlags(&B.staged, cudaEventDisableTiming), "batch event");
-  uint64_t tris = 0, verts = 0, nrms = 0, pixels = 0, tiles = 0;
+  uint64_t tris = 0, verts = 0, nrms = 0, normals = 0, pixels = 0, tiles = 0;
   const int TW = B.tile_w, TH = B.tile_h;
   for (int32_t s = 0; s < n_scenes; s++) {
     const mr_frame* f = &sc[s].frame;
@@ -1101,9 +1104,10 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
     if (rs[i].flags & ~kRenderableFlags) return fail(c, MR_E_INVALID, "unknown renderable flags");
     tris += (uint64_t)c->meshes[h].d.n_tri;
     verts += (uint64_t)c->meshes[h].d.n_pos;
+    normals += (uint64_t)c->meshes[h].d.n_nrm;
     nrms += mesh_unified(c->meshes[h].d) ? 0 : (uint64_t)c->meshes[h].d.n_nrm;
   }
-  if (tris >= ((uint64_t)1 << 31) || verts >= ((uint64_t)1 << 32) || nrms >= ((uint64_t)1 << 32) ||
+  if (tris >= ((uint64_t)1 << 31) || verts >= ((uint64_t)1 << 32) || normals >= ((uint64_t)1 << 32) ||
       tiles >= ((uint64_t)1 << 31))
     return fail(c, MR_E_INVALID, "batch too large for 32-bit indices");
   // staging (wait until the previous batch of this slot has copied it; its

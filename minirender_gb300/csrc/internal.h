@@ -167,8 +167,8 @@ struct mr_ctx {
   DevBuf<float> depth, rgbf, normals, range;
   DevBuf<uint32_t> ids;
   DevBuf<BigRec> recs;
-  DevBuf<LargeItem> items;     // large-triangle row blocks of the last frame
-  DevBuf<LargeItem> spill;     // records whose rows did not fit items (one entry each)
+  DevBuf<LargeItem> items;     // large-triangle blocks of the last frame
+  DevBuf<LargeItem> spill;     // records whose blocks did not fit items (one entry each)
   // Per-frame staging of frames of several renderables, one block on both
   // sides: renderables (cap) | tri, vertex and normal base tables 3 x (cap+1)
   DevBuf<unsigned char> stage;

@@ -13,11 +13,10 @@
 // kernels receive.  The address belongs to the device's primary context, so
 // the device must not be reset (cudaDeviceReset) while the library is in use.
 // Every call shares the array and inherits the previous call's contents, so
-// the counters are cleared each call; the visibility buffer is cleared by the
-// frame's own clear kernel and the index mask is rewritten by the validation
-// kernel.  Large sub-triangles get records and row blocks in the array as in
-// mr_render, up to kRecCap of them; any further ones are rasterised by the
-// setup kernel itself.  Calls whose GPU work overlaps race on the array.
+// the frame's first kernel clears the counters and the visibility buffer, and
+// the validation kernel rewrites the index mask.  Large sub-triangles get
+// records and blocks in the array as in mr_render, up to kRecCap / kShares in
+// each share; any further ones are rasterised by the setup kernel itself.  Calls whose GPU work overlaps race on the array.
 #include <cuda_runtime.h>
 #include <string.h>
 
@@ -140,7 +139,7 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
   F.g.n_renderables = 1;
   F.g.n_tris = (uint32_t)M.n_tri;
   // Sub-triangles up to 64 pixels of bounding box are rasterised by the setup
-  // kernel; larger ones take records and row blocks from the fixed store
+  // kernel; larger ones take records and blocks from the fixed store
   // (the spill list holds one entry per record, so it cannot overflow).
   F.small_max = 64;
   F.one = R;
