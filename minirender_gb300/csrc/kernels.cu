@@ -1381,23 +1381,22 @@ __device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, u
 //   the scene's small-triangle words; its records are rasterised into shared
 //   memory, then every pixel is resolved, shaded and written to its scene's
 //   outputs.
-// A strip is one warp's alone, so nothing in it waits for other warps; a block
-// takes groups of strips from a work counter and its warps share a group
-// through a counter in shared memory (neighbouring strips read the same
-// records and vertices).  With a block per tile, block barriers between the
-// phases were 38 % of the warps' time: 256 scenes 2934 -> 2670 us, 16 soups 260
-// -> 240, eight 3840x2160 scenes in 16x16 tiles 5037 -> 3558.  (The old form
-// also captured the winners' edge values where a replay could pass 256
-// columns; with packed adds the replay is the cheaper.)  Groups of two strips
-// a warp: one gives up the shared reads (2822 us), four leave a tail (2723).
+// A strip is one warp's alone and each warp takes its own from a work counter,
+// so no warp waits for another once the lists stand.  With a block per tile,
+// barriers between the phases were 38 % of the warps' time (256 scenes 2934 us,
+// 16 soups 260, eight 3840x2160 scenes in 16x16 tiles 5037); with strips handed
+// to a block two a warp at a time, the barrier around the hand-over was still
+// a fifth (1945, 207); now 1807 and 198, and 24 scenes of 256x256 74 -> 65.
+// (Groups a block's warps share and refill without a barrier: 1830 and 211.)
+// (The old form also captured the winners' edge values where a replay could
+// pass 256 columns; with packed adds the replay is the cheaper.)
 // 64 registers: with 80 the 256 scenes take 2565 us (2270) and 16 soups 221
 // (205), with up to 128, which blocks of 64 threads had, the soups 252.
 template <bool PRE>
 __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ unsigned long long s_first;
-  __shared__ uint32_t s_next;
   __shared__ SceneRec s_scene[8];
+  __shared__ unsigned long long s_at[8];
   cg::grid_group grid = cg::this_grid();
   const uint32_t nb = gridDim.x, nt = blockDim.x;
   const int lane = (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
@@ -1436,144 +1435,141 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
       }
   }
   grid.sync();
-  // 3. strips, in groups of two per warp of the block
-  const uint32_t warps = nt >> 5;
+  // 3. strips.  A fetch is one strip, or as many as make half of strip_px where
+  // tiles are smaller (the counter takes one atomic at a time: 64 scenes of
+  // 512x512 in 4x16 tiles 1381 us with groups of four for two warps, 1399 with
+  // all of strip_px, 1364 so).  A warp's place is kept in shared memory: in
+  // registers it spills what the shading needs (256 scenes 1832 us, 1807).
   const int ls2 = __ffs(TH / SH) - 1;  // strips per tile, a power of two
-  const unsigned long long units = (unsigned long long)B.n_tiles << ls2;
-  const uint32_t group = 2u * warps;
+  const uint32_t run = max(1u, (uint32_t)B.strip_px / (uint32_t)(2 * TW * SH));  // strips per fetch, likewise
+  if (lane == 0) s_at[w] = ~0ull;
   for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_first = (unsigned long long)atomicAdd(&B.counters->work_next, 1u) * group;
-      s_next = 0;
+    __syncwarp();  // the last strip's words and scene may be overwritten
+    unsigned long long u = s_at[w] + 1;
+    if (!(u & (run - 1))) {
+      uint32_t f = 0;
+      if (lane == 0) f = atomicAdd(&B.counters->work_next, 1u);
+      u = (unsigned long long)__shfl_sync(0xffffffffu, f, 0) * run;
     }
-    __syncthreads();
-    const unsigned long long first = s_first;
-    if (first >= units) break;
-    const uint32_t n_units = (uint32_t)min((unsigned long long)group, units - first);
-    for (;;) {
-      uint32_t k = 0;
-      if (lane == 0) k = atomicAdd(&s_next, 1u);
-      k = __shfl_sync(0xffffffffu, k, 0);
-      if (k >= n_units) break;
-      const uint32_t t = (uint32_t)((first + k) >> ls2), strip = (uint32_t)(first + k) & ((1u << ls2) - 1u);
-      // the scene: the last j with scene_tile_base[j] <= t (bases ascending,
-      // the first 0), 32 candidates at a time
-      int sc = 0;
-      for (int n = B.n_scenes; n > 1;) {
-        const int step = (n + 31) >> 5, j = sc + lane * step;
-        const unsigned m = __ballot_sync(0xffffffffu, lane * step < n && B.scene_tile_base[j] <= t);
-        const int at = (31 - __clz((int)m)) * step;
-        sc += at;
-        n = min(step, n - at);
-      }
-      __syncwarp();
-      {
-        const uint32_t* src = reinterpret_cast<const uint32_t*>(&B.scenes[sc]);
-        uint32_t* dst = reinterpret_cast<uint32_t*>(&s_scene[w]);
-        for (int i = lane; i < (int)(sizeof(SceneRec) / 4); i += 32) dst[i] = src[i];
-      }
-      __syncwarp();
-      const SceneRec& C = s_scene[w];
-      const int lt = (int)(t - C.tile_base), ty = lt / C.tiles_x, tx = lt - ty * C.tiles_x;
-      const int px0 = tx * TW, py0 = ty * TH + (int)strip * SH;
-      const int px1 = min(px0 + TW, C.v.W) - 1, py1 = min(py0 + SH, C.v.H) - 1;
-      if (py0 > py1) continue;
-      const bool persp = C.v.persp != 0;
-      // the tile's list (truncated at capacity on overflow)
-      const uint32_t ls = min(B.tile_start[t], B.bin_cap), le = min(B.tile_start[t] + B.tile_count[t], B.bin_cap);
-      // the strip starts from the small triangles' words (or empty): two
-      // words a load, all of a lane's in flight at once; what is not empty is
-      // left empty for the next batch
-      bool drawn = false;
-      {
-        const bool pairs = ((C.v.W & 1) | (int)((uintptr_t)C.vis >> 3 & 1)) == 0 && px1 - px0 + 1 == TW;
-        ulonglong2 v[kStripMax / 64];
+    __syncwarp();
+    if (lane == 0) s_at[w] = u;
+    const uint32_t t = (uint32_t)(u >> ls2), strip = (uint32_t)u & ((1u << ls2) - 1u);
+    if (t >= B.n_tiles) break;
+    // the scene: the last j with scene_tile_base[j] <= t (bases ascending,
+    // the first 0), 32 candidates at a time
+    int sc = 0;
+    for (int n = B.n_scenes; n > 1;) {
+      const int step = (n + 31) >> 5, j = sc + lane * step;
+      const unsigned m = __ballot_sync(0xffffffffu, lane * step < n && B.scene_tile_base[j] <= t);
+      const int at = (31 - __clz((int)m)) * step;
+      sc += at;
+      n = min(step, n - at);
+    }
+    __syncwarp();
+    {
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(&B.scenes[sc]);
+      uint32_t* dst = reinterpret_cast<uint32_t*>(&s_scene[w]);
+      for (int i = lane; i < (int)(sizeof(SceneRec) / 4); i += 32) dst[i] = src[i];
+    }
+    __syncwarp();
+    const SceneRec& C = s_scene[w];
+    const int lt = (int)(t - C.tile_base), ty = lt / C.tiles_x, tx = lt - ty * C.tiles_x;
+    const int px0 = tx * TW, py0 = ty * TH + (int)strip * SH;
+    const int px1 = min(px0 + TW, C.v.W) - 1, py1 = min(py0 + SH, C.v.H) - 1;
+    if (py0 > py1) continue;
+    const bool persp = C.v.persp != 0;
+    // the tile's list (truncated at capacity on overflow)
+    const uint32_t ls = min(B.tile_start[t], B.bin_cap), le = min(B.tile_start[t] + B.tile_count[t], B.bin_cap);
+    // the strip starts from the small triangles' words (or empty): two
+    // words a load, all of a lane's in flight at once; what is not empty is
+    // left empty for the next batch
+    bool drawn = false;
+    {
+      const bool pairs = ((C.v.W & 1) | (int)((uintptr_t)C.vis >> 3 & 1)) == 0 && px1 - px0 + 1 == TW;
+      ulonglong2 v[kStripMax / 64];
 #pragma unroll
-        for (int j = 0; j < kStripMax / 64; j++) {
-          const int i = 64 * j + 2 * lane, cy = i >> lw, x = px0 + (i & (TW - 1)), y = py0 + cy;
-          v[j] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
-          if (C.vis && i < SH * TW && y <= py1) {
-            unsigned long long* q = C.vis + ((uint32_t)y * (uint32_t)C.v.W + (uint32_t)x);
-            if (pairs) {
-              v[j] = *reinterpret_cast<const ulonglong2*>(q);
-            } else {
-              if (x <= px1) v[j].x = q[0];
-              if (x + 1 <= px1) v[j].y = q[1];
-            }
+      for (int j = 0; j < kStripMax / 64; j++) {
+        const int i = 64 * j + 2 * lane, cy = i >> lw, x = px0 + (i & (TW - 1)), y = py0 + cy;
+        v[j] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
+        if (C.vis && i < SH * TW && y <= py1) {
+          unsigned long long* q = C.vis + ((uint32_t)y * (uint32_t)C.v.W + (uint32_t)x);
+          if (pairs) {
+            v[j] = *reinterpret_cast<const ulonglong2*>(q);
+          } else {
+            if (x <= px1) v[j].x = q[0];
+            if (x + 1 <= px1) v[j].y = q[1];
           }
         }
+      }
 #pragma unroll
-        for (int j = 0; j < kStripMax / 64; j++) {
-          const int i = 64 * j + 2 * lane, cy = i >> lw, cx = i & (TW - 1);
-          if (i >= SH * TW) break;
-          if ((v[j].x & v[j].y) != VIS_EMPTY) {
-            drawn = true;
-            unsigned long long* q = C.vis + ((uint32_t)(py0 + cy) * (uint32_t)C.v.W + (uint32_t)(px0 + cx));
-            if (v[j].x != VIS_EMPTY) q[0] = VIS_EMPTY;
-            if (v[j].y != VIS_EMPTY) q[1] = VIS_EMPTY;
-          }
-          *reinterpret_cast<ulonglong2*>(svis + cy * pitch + cx) = v[j];
+      for (int j = 0; j < kStripMax / 64; j++) {
+        const int i = 64 * j + 2 * lane, cy = i >> lw, cx = i & (TW - 1);
+        if (i >= SH * TW) break;
+        if ((v[j].x & v[j].y) != VIS_EMPTY) {
+          drawn = true;
+          unsigned long long* q = C.vis + ((uint32_t)(py0 + cy) * (uint32_t)C.v.W + (uint32_t)(px0 + cx));
+          if (v[j].x != VIS_EMPTY) q[0] = VIS_EMPTY;
+          if (v[j].y != VIS_EMPTY) q[1] = VIS_EMPTY;
         }
+        *reinterpret_cast<ulonglong2*>(svis + cy * pitch + cx) = v[j];
       }
-      __syncwarp();
-      if (ls < le) raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
-      // nothing drawn: the background, four pixels a lane where whole groups
-      // of four lie aligned in every output
-      if (ls >= le && !__any_sync(0xffffffffu, drawn) && px1 - px0 + 1 == TW && (C.v.W & 3) == 0 &&
-          (((uintptr_t)C.depth | (uintptr_t)C.ids) & 15) == 0 && ((uintptr_t)C.rgb8 & 3) == 0) {
-        const uint32_t c = to_byte(C.v.bg[0]) | ((uint32_t)to_byte(C.v.bg[1]) << 8) | ((uint32_t)to_byte(C.v.bg[2]) << 16);
-        for (int i = 4 * lane; i < SH * TW; i += 128) {
-          const int y = py0 + (i >> lw);
-          if (y > py1) break;
-          const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)(px0 + (i & (TW - 1)));
-          if (C.rgb8) {
-            uint32_t* o = reinterpret_cast<uint32_t*>(C.rgb8 + 3 * (size_t)px);
-            o[0] = c | (c << 24);
-            o[1] = (c >> 8) | (c << 16);
-            o[2] = (c >> 16) | (c << 8);
-          }
-          if (C.depth) *reinterpret_cast<float4*>(C.depth + px) = make_float4(1e11f, 1e11f, 1e11f, 1e11f);
-          if (C.ids) *reinterpret_cast<uint4*>(C.ids + px) = make_uint4(MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE);
-        }
-        continue;
-      }
-      const uint32_t id0 = 2u * B.g.tri_base[C.rs_begin];  // ids are reported per scene
-#pragma unroll 1
-      for (int i = lane; i < SH * TW; i += 32) {
-        const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
-        if (x > px1 || y > py1) continue;
-        const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)x;
-        const unsigned long long vw = svis[cy * pitch + cx];
-        V3 value, normal;
-        float depth;
-        const uint32_t id = (uint32_t)vw;
-        if (vw == VIS_EMPTY) {
-          value = v3(C.v.bg[0], C.v.bg[1], C.v.bg[2]);
-          depth = 1e11f;
-        } else {
-          uint32_t gv[3];
-          const DevRenderable& R = B.g.rs[find_triangle<PRE>(B.g, (int)C.rs_begin, (int)C.rs_end, id >> 1, gv)];
-          Winner N;
-          winner<PRE, PRE>(C.v, B.g, R, id, gv, N);
-          Setup S;
-          winner_setup(C.v, N, S);
-          float e1, e2;
-          replay(S, x, y, e1, e2);
-          float k0, k1, k2;
-          depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
-          shade(C.v, R, N.v, k0, k1, k2, value, normal);
-        }
+    }
+    __syncwarp();
+    if (ls < le) raster_strip(B, ls, le, px0, py0, px1, py1, persp, pitch, svis);
+    // nothing drawn: the background, four pixels a lane where whole groups
+    // of four lie aligned in every output
+    if (ls >= le && !__any_sync(0xffffffffu, drawn) && px1 - px0 + 1 == TW && (C.v.W & 3) == 0 &&
+        (((uintptr_t)C.depth | (uintptr_t)C.ids) & 15) == 0 && ((uintptr_t)C.rgb8 & 3) == 0) {
+      const uint32_t c = to_byte(C.v.bg[0]) | ((uint32_t)to_byte(C.v.bg[1]) << 8) | ((uint32_t)to_byte(C.v.bg[2]) << 16);
+      for (int i = 4 * lane; i < SH * TW; i += 128) {
+        const int y = py0 + (i >> lw);
+        if (y > py1) break;
+        const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)(px0 + (i & (TW - 1)));
         if (C.rgb8) {
-          uint8_t* o8 = C.rgb8 + 3 * (size_t)px;
-          o8[0] = to_byte(value.x);
-          o8[1] = to_byte(value.y);
-          o8[2] = to_byte(value.z);
+          uint32_t* o = reinterpret_cast<uint32_t*>(C.rgb8 + 3 * (size_t)px);
+          o[0] = c | (c << 24);
+          o[1] = (c >> 8) | (c << 16);
+          o[2] = (c >> 16) | (c << 8);
         }
-        if (C.depth) C.depth[px] = depth;
-        if (C.ids) C.ids[px] = vw == VIS_EMPTY ? MR_NO_TRIANGLE : id - id0;
+        if (C.depth) *reinterpret_cast<float4*>(C.depth + px) = make_float4(1e11f, 1e11f, 1e11f, 1e11f);
+        if (C.ids) *reinterpret_cast<uint4*>(C.ids + px) = make_uint4(MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE, MR_NO_TRIANGLE);
       }
-      __syncwarp();  // the strip's words may be overwritten
+      continue;
+    }
+    const uint32_t id0 = 2u * B.g.tri_base[C.rs_begin];  // ids are reported per scene
+#pragma unroll 1
+    for (int i = lane; i < SH * TW; i += 32) {
+      const int cy = i >> lw, cx = i & (TW - 1), x = px0 + cx, y = py0 + cy;
+      if (x > px1 || y > py1) continue;
+      const uint32_t px = (uint32_t)y * (uint32_t)C.v.W + (uint32_t)x;
+      const unsigned long long vw = svis[cy * pitch + cx];
+      V3 value, normal;
+      float depth;
+      const uint32_t id = (uint32_t)vw;
+      if (vw == VIS_EMPTY) {
+        value = v3(C.v.bg[0], C.v.bg[1], C.v.bg[2]);
+        depth = 1e11f;
+      } else {
+        uint32_t gv[3];
+        const DevRenderable& R = B.g.rs[find_triangle<PRE>(B.g, (int)C.rs_begin, (int)C.rs_end, id >> 1, gv)];
+        Winner N;
+        winner<PRE, PRE>(C.v, B.g, R, id, gv, N);
+        Setup S;
+        winner_setup(C.v, N, S);
+        float e1, e2;
+        replay(S, x, y, e1, e2);
+        float k0, k1, k2;
+        depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
+        shade(C.v, R, N.v, k0, k1, k2, value, normal);
+      }
+      if (C.rgb8) {
+        uint8_t* o8 = C.rgb8 + 3 * (size_t)px;
+        o8[0] = to_byte(value.x);
+        o8[1] = to_byte(value.y);
+        o8[2] = to_byte(value.z);
+      }
+      if (C.depth) C.depth[px] = depth;
+      if (C.ids) C.ids[px] = vw == VIS_EMPTY ? MR_NO_TRIANGLE : id - id0;
     }
   }
 }
