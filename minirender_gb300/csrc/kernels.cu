@@ -787,6 +787,12 @@ __device__ __forceinline__ void normal(const Geo& G, const DevRenderable& R, uin
   G.vn[g] = make_float4(n.x, n.y, n.z, 0.f);
 }
 
+__device__ __forceinline__ void clear_words(unsigned long long* vis, size_t n, size_t i, size_t stride) {
+  // two words per store (vis is 16-byte aligned)
+  ulonglong2* v2 = reinterpret_cast<ulonglong2*>(vis);
+  for (size_t k = i; k < n / 2; k += stride) v2[k] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
+  if (i == 0 && (n & 1)) vis[n - 1] = VIS_EMPTY;
+}
 // The first kernel of a frame: vis[0..n) = VIS_EMPTY (Renderer::clear), the
 // counters zeroed, and one of
 //   - the staging block of a frame of several renderables copied from mapped
@@ -795,12 +801,8 @@ __device__ __forceinline__ void normal(const Geo& G, const DevRenderable& R, uin
 //   - VERT: the vertex pass of a frame of one renderable, which comes in the
 //     kernel's parameters (one launch less, and the stores of the clear fill
 //     the vertex pass's load latency).
-__device__ __forceinline__ void clear_words(unsigned long long* vis, size_t n, size_t i, size_t stride) {
-  // two words per store (vis is 16-byte aligned)
-  ulonglong2* v2 = reinterpret_cast<ulonglong2*>(vis);
-  for (size_t k = i; k < n / 2; k += stride) v2[k] = make_ulonglong2(VIS_EMPTY, VIS_EMPTY);
-  if (i == 0 && (n & 1)) vis[n - 1] = VIS_EMPTY;
-}
+// Bound by the vertex pass's dependent loads and, in small frames, by the
+// launch: 655,362 vertices and 1920x1080 words 17.6 us between events.
 template <bool VERT>
 __global__ void __launch_bounds__(256) k_begin(FrameParams F) {
   pdl_trigger();
@@ -879,7 +881,10 @@ __global__ void k_validate(DevMesh M, uint32_t* bad, float4* rec) {
 
 // Vertex pass of several renderables: threads [0, n_verts) transform and
 // project positions, threads [n_verts, n_verts + n_nrms) transform normals.
-// BATCH: the view of a vertex is scenes[R.scene].v, else V.
+// BATCH: the view of a vertex is scenes[R.scene].v, else V.  Bound by the
+// search for its renderable and by bytes; normals of meshes whose attributes
+// share one index array go beside the positions (Geo::vc), so most threads of
+// the second range have gone: 256 scenes of 64 primitives 254 -> 88 us.
 template <bool BATCH>
 __global__ void __launch_bounds__(256) k_vertex(Geo G, View V, const SceneRec* scenes) {
   pdl_wait();
@@ -1133,7 +1138,7 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
 // lanes waiting.  Then the spill list: one warp per record, its remaining
 // blocks.  An ordinary launch: with no large record every warp leaves at once.
 // Bound by the serial walk of a row, which is why rows are cut into segments
-// (large_segs): 64 primitives at 1280x720, 30.4 us with whole rows.
+// (large_segs): 64 primitives at 1280x720, 30.4 us with whole rows, 12 so.
 __device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, uint32_t rec, uint32_t k) {
   const BigRec& R = F.recs[rec];
   const Setup S = rec_setup(R);
@@ -1203,7 +1208,12 @@ __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
 // Deferred resolve + shade: one thread per pixel, 128-thread blocks over
 // 32x4-pixel tiles (a block keeps its registers until its slowest warp is
 // done: 1080p mesh 40.9 us with 256 threads, 36.9 with 128, 38.9 with 64; 4K
-// soup 235, 225, 229).
+// soup 235, 225, 229).  Bound by its chain of gathers -- word, triangle,
+// corners, texel -- where neighbouring pixels' triangles lie apart (1080p mesh
+// of 1.31M triangles: 53 % of issue slots used, 36.8 us; 52 with attributes in
+// six arrays and a search for the renderable), by instruction issue where
+// corner records shorten it (10M-triangle soup: 72 %, 219 us; 282).  More
+// blocks per SM spill.
 constexpr int kResolveTileW = 32, kResolveTileH = 4, kResolveThreads = kResolveTileW * kResolveTileH;
 template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_resolve(FrameParams F) {
@@ -1260,8 +1270,42 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
 }
 
 // ---------------------------------------------------------------- batches
+// put(tile, lane) for the tiles of the warp's records, one pair a lane: lane's
+// record covers n tiles, nx to a row, from `first` (pitch: tiles per row of its
+// scene).  With a record per lane, a triangle as large as its frame was one
+// lane's chain of hundreds of atomics that the whole grid waited for: 24 scenes
+// of 256x256 98 us of k_batch, 53 so where such triangles occur, 68 and 59 where
+// hardly; 256 scenes 1811-2006 us, 1777-1820 so.  Called by all lanes.
+template <typename Put>
+__device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, int nx, int n, Put put) {
+  const int lane = (int)(threadIdx.x & 31);
+  int inc = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  const int total = __shfl_sync(0xffffffffu, inc, 31);
+#pragma unroll 1
+  for (int q = 0; q < total; q += 32) {
+    const int j = q + lane;
+    int own = 0;  // the lane whose record pair j belongs to
+#pragma unroll
+    for (int step = 16; step; step >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= j) own += step;
+    const int k = j - __shfl_sync(0xffffffffu, inc - n, own), cols = __shfl_sync(0xffffffffu, nx, own);
+    const int row = k / cols;
+    const uint32_t t = __shfl_sync(0xffffffffu, first, own) + (uint32_t)row * __shfl_sync(0xffffffffu, pitch, own) +
+                       (uint32_t)(k - row * cols);
+    if (j < total) put(t, own);
+  }
+}
+
 // Setup of every triangle of every scene: each sub-triangle with pixels to
 // test becomes a record (warp-compacted), counted into its scene's tiles.
+// Bound by dependent loads (renderable, indices, vertices, view): 49 % of issue
+// slots used; 256 scenes 360 us, 364 and 389 with blocks of 128 and 256
+// threads, 369 and 397 with 40 and 64 registers.
 template <bool PRE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup_batch(BatchParams B) {
   const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -1421,18 +1465,24 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   const uint32_t gw = (blockIdx.x * nt + threadIdx.x) >> 5, share = gw % kShares;
   const uint32_t nrec = min(B.counters->share[share].rec_count, B.rec_share);
   const uint32_t per = (nb * (nt >> 5) + kShares - 1 - share) / kShares;  // warps on this share
-  for (uint32_t r = (gw / kShares) * 32 + lane; r < nrec; r += per * 32) {
-    const uint32_t i = share * B.rec_share + r;
-    const BigRec& R = B.recs[i];
-    const SceneRec& SR = B.scenes[B.rec_scene[i]];
-    int tx0 = R.x0 / TW, tx1 = R.x1 / TW, ty0 = R.y0 / TH, ty1 = R.y1 / TH;
-    for (int ty = ty0; ty <= ty1; ty++)
-      for (int tx = tx0; tx <= tx1; tx++) {
-        uint32_t t = SR.tile_base + ty * SR.tiles_x + tx;
-        uint32_t pos = B.tile_start[t] + atomicAdd(B.tile_fill + t, 1u);
-        if (pos < B.bin_cap) B.bins[pos] = i;
-        else B.counters->bin_overflow = 1;
-      }
+  for (uint32_t r0 = (gw / kShares) * 32; r0 < nrec; r0 += per * 32) {
+    const uint32_t i = share * B.rec_share + r0 + lane;
+    uint32_t first = 0, pitch_t = 0;  // the record's first tile, tiles per row of its scene
+    int nx = 1, n = 0;                // columns and number of its tiles
+    if (r0 + lane < nrec) {
+      const BigRec& R = B.recs[i];
+      const SceneRec& SR = B.scenes[B.rec_scene[i]];
+      const int tx0 = R.x0 / TW, ty0 = R.y0 / TH;
+      nx = R.x1 / TW - tx0 + 1;
+      n = nx * (R.y1 / TH - ty0 + 1);
+      pitch_t = (uint32_t)SR.tiles_x;
+      first = SR.tile_base + (uint32_t)ty0 * pitch_t + (uint32_t)tx0;
+    }
+    each_tile(first, pitch_t, nx, n, [&](uint32_t t, int own) {
+      const uint32_t pos = B.tile_start[t] + atomicAdd(B.tile_fill + t, 1u);
+      if (pos < B.bin_cap) B.bins[pos] = i - lane + own;
+      else B.counters->bin_overflow = 1;
+    });
   }
   grid.sync();
   // 3. strips.  A fetch is one strip, or as many as make half of strip_px where
