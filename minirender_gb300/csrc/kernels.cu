@@ -1275,7 +1275,8 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
 // scene).  With a record per lane, a triangle as large as its frame was one
 // lane's chain of hundreds of atomics that the whole grid waited for: 24 scenes
 // of 256x256 98 us of k_batch, 53 so where such triangles occur, 68 and 59 where
-// hardly; 256 scenes 1811-2006 us, 1777-1820 so.  Called by all lanes.
+// hardly; 256 scenes 1811-2006 us, 1777-1820 so.  (In the setup's counts, whose
+// atomics return nothing: 256 scenes 360 us, 340.)  Called by all lanes.
 template <typename Put>
 __device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, int nx, int n, Put put) {
   const int lane = (int)(threadIdx.x & 31);
@@ -1304,8 +1305,8 @@ __device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, int nx
 // Setup of every triangle of every scene: each sub-triangle with pixels to
 // test becomes a record (warp-compacted), counted into its scene's tiles.
 // Bound by dependent loads (renderable, indices, vertices, view): 49 % of issue
-// slots used; 256 scenes 360 us, 364 and 389 with blocks of 128 and 256
-// threads, 369 and 397 with 40 and 64 registers.
+// slots used; 256 scenes 340 us.  (Blocks of 128 and 256 threads cost 1 % and
+// 8 % more, 40 and 64 registers 2 % and 10 %.)
 template <bool PRE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup_batch(BatchParams B) {
   const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -1338,18 +1339,22 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
     if (lane == 0 && m) base = atomicAdd(&B.counters->share[warp_share()].rec_count, (unsigned)__popc(m));
     base = __shfl_sync(0xffffffffu, base, 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
+    uint32_t first = 0, pitch = 0;
+    int nx = 1, n = 0;
     if (big) {
       const unsigned at = base + __popc(m & lt), slot = warp_share() * B.rec_share + at;
       if (at < B.rec_share) {
         B.recs[slot] = to_rec(S, id);
         B.rec_scene[slot] = scene;
         const SceneRec& SR = B.scenes[scene];
-        const int tx0 = S.x0 / B.tile_w, tx1 = S.x1 / B.tile_w, ty0 = S.y0 / B.tile_h, ty1 = S.y1 / B.tile_h;
-        for (int ty = ty0; ty <= ty1; ty++)
-          for (int tx = tx0; tx <= tx1; tx++)
-            atomicAdd(B.tile_count + SR.tile_base + ty * SR.tiles_x + tx, 1u);
+        const int tx0 = S.x0 / B.tile_w, ty0 = S.y0 / B.tile_h;
+        nx = S.x1 / B.tile_w - tx0 + 1;
+        n = nx * (S.y1 / B.tile_h - ty0 + 1);
+        pitch = (uint32_t)SR.tiles_x;
+        first = SR.tile_base + (uint32_t)ty0 * pitch + (uint32_t)tx0;
       }
     }
+    if (m) each_tile(first, pitch, nx, n, [&](uint32_t t, int) { atomicAdd(B.tile_count + t, 1u); });
     if (B.small_max > 0) raster_small<!PRE>(S, small, id, scene, BatchTarget{B.scenes});
   }
 }
