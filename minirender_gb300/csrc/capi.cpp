@@ -1038,11 +1038,14 @@ static int batch_launch(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling
 // them so (a separate clear of every scene's words was 110 us of a 256-scene
 // batch), unless the buffer is new, a launch failed or the batch is only
 // recorded (into the caller's capture of st, which then clears at each replay).
+// A staged batch without words (small_max 0 when it was staged) tells nothing
+// about them.
 int batch_run(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
+  if (!B.P.vis) return batch_launch(c, B, st, profiling, ev);
   cudaStreamCaptureStatus cap;
   CK(cudaStreamIsCapturing(st, &cap), "capture status");
   const bool runs = cap == cudaStreamCaptureStatusNone;
-  if (B.small_max > 0 && !(B.vis_empty && runs))
+  if (!(B.vis_empty && runs))
     CK(cudaMemsetAsync(B.vis.p, 0xFF, B.vis.cap * sizeof(unsigned long long), st), "visibility clear");
   B.vis_empty = false;
   const int rc = batch_launch(c, B, st, profiling, ev);
