@@ -563,7 +563,7 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   std::lock_guard<std::recursive_mutex> g(c->mu);
   if (!f || (n > 0 && !rs) || n < 0) return fail(c, MR_E_INVALID, "null frame or renderables");
   if (f->width <= 0 || f->height <= 0 || (int64_t)f->width * f->height > (int64_t)1 << 28 ||
-      f->width > (1 << 16) || f->height > (1 << 16))
+      f->width > kMaxSide || f->height > kMaxSide)
     return fail(c, MR_E_INVALID, "frame size out of range");
   cudaSetDevice(c->device);
   if (c->async_read) {  // the last frame's reads complete before it is replaced
@@ -1085,7 +1085,7 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   const int TW = B.tile_w, TH = B.tile_h;
   for (int32_t s = 0; s < n_scenes; s++) {
     const mr_frame* f = &sc[s].frame;
-    if (f->width <= 0 || f->height <= 0 || f->width > (1 << 16) || f->height > (1 << 16))
+    if (f->width <= 0 || f->height <= 0 || f->width > kMaxSide || f->height > kMaxSide)
       return fail(c, MR_E_INVALID, "scene frame size out of range");
     if (sc[s].first_renderable < 0 || sc[s].n_renderables < 0 ||
         (int64_t)sc[s].first_renderable + sc[s].n_renderables > n_rs ||
@@ -1292,6 +1292,8 @@ int batch_settle(mr_ctx* c, BatchSlot& B, cudaStream_t st) {
     CK(cudaStreamSynchronize(st), "batch wait");
     if (!B.h_cnt->bin_overflow)
       return (B.h_cnt->error_flags & 1u) ? fail(c, MR_E_BAD_INDEX, "a mesh index was out of range; those triangles were skipped") : MR_OK;
+    if (B.h_cnt->bin_needed > 0xFFFFFFFFu)
+      return fail(c, MR_E_NOMEM, "more than 2^32-1 (tile, triangle) pairs in one batch");
     size_t want = (size_t)B.h_cnt->bin_needed + B.h_cnt->bin_needed / 4 + 1024;
     CK(B.bins.ensure(want), "batch bins");
     B.P.bins = B.bins.p;

@@ -22,7 +22,7 @@ int batch_grid(int tile_w, int tile_h, int threads, bool pre);
 // Tile shapes k_batch takes: power-of-two sides, 64..4096 pixels (whole warps).
 inline bool batch_tile_ok(int tw, int th) {
   auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
-  return pow2(tw) && pow2(th) && tw >= 4 && tw <= 256 && th >= 2 && th <= 64 && tw * th >= 64 && tw * th <= 4096;
+  return pow2(tw) && pow2(th) && tw >= 4 && tw <= 256 && th >= 2 && th <= 64 && tw * th >= kMinTilePx && tw * th <= 4096;
 }
 }  // namespace mrg
 

@@ -1278,26 +1278,26 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
 // hardly; 256 scenes 1811-2006 us, 1777-1820 so.  (In the setup's counts, whose
 // atomics return nothing: 256 scenes 360 us, 340.)  Called by all lanes.
 template <typename Put>
-__device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, int nx, int n, Put put) {
+__device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, uint32_t nx, PairNo n, Put put) {
   const int lane = (int)(threadIdx.x & 31);
-  int inc = n;
+  PairNo inc = n;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    const PairNo u = __shfl_up_sync(0xffffffffu, inc, o);
     if (lane >= o) inc += u;
   }
-  const int total = __shfl_sync(0xffffffffu, inc, 31);
+  const PairNo total = __shfl_sync(0xffffffffu, inc, 31);
 #pragma unroll 1
-  for (int q = 0; q < total; q += 32) {
-    const int j = q + lane;
+  for (PairNo q = 0; q < total; q += 32) {
+    const PairNo j = q + (PairNo)lane;
     int own = 0;  // the lane whose record pair j belongs to
 #pragma unroll
     for (int step = 16; step; step >>= 1)
       if (__shfl_sync(0xffffffffu, inc, own + step - 1) <= j) own += step;
-    const int k = j - __shfl_sync(0xffffffffu, inc - n, own), cols = __shfl_sync(0xffffffffu, nx, own);
-    const int row = k / cols;
-    const uint32_t t = __shfl_sync(0xffffffffu, first, own) + (uint32_t)row * __shfl_sync(0xffffffffu, pitch, own) +
-                       (uint32_t)(k - row * cols);
+    const PairNo k = j - __shfl_sync(0xffffffffu, inc - n, own);
+    const uint32_t cols = __shfl_sync(0xffffffffu, nx, own);
+    const uint32_t row = k / cols;
+    const uint32_t t = __shfl_sync(0xffffffffu, first, own) + row * __shfl_sync(0xffffffffu, pitch, own) + (k - row * cols);
     if (j < total) put(t, own);
   }
 }
@@ -1339,8 +1339,8 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
     if (lane == 0 && m) base = atomicAdd(&B.counters->share[warp_share()].rec_count, (unsigned)__popc(m));
     base = __shfl_sync(0xffffffffu, base, 0);
     const uint32_t id = 2u * g + (uint32_t)sub;
-    uint32_t first = 0, pitch = 0;
-    int nx = 1, n = 0;
+    uint32_t first = 0, pitch = 0, nx = 1;
+    PairNo n = 0;
     if (big) {
       const unsigned at = base + __popc(m & lt), slot = warp_share() * B.rec_share + at;
       if (at < B.rec_share) {
@@ -1348,8 +1348,8 @@ __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kS
         B.rec_scene[slot] = scene;
         const SceneRec& SR = B.scenes[scene];
         const int tx0 = S.x0 / B.tile_w, ty0 = S.y0 / B.tile_h;
-        nx = S.x1 / B.tile_w - tx0 + 1;
-        n = nx * (S.y1 / B.tile_h - ty0 + 1);
+        nx = (uint32_t)(S.x1 / B.tile_w - tx0 + 1);
+        n = nx * (PairNo)(S.y1 / B.tile_h - ty0 + 1);
         pitch = (uint32_t)SR.tiles_x;
         first = SR.tile_base + (uint32_t)ty0 * pitch + (uint32_t)tx0;
       }
@@ -1454,16 +1454,18 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   // 1. the tiles' ranges, in any order: one atomic per warp of tiles
   for (uint32_t t0 = (blockIdx.x * nt + threadIdx.x) & ~31u; t0 < B.n_tiles; t0 += nb * nt) {
     const uint32_t t = t0 + lane, v = t < B.n_tiles ? B.tile_count[t] : 0u;
-    uint32_t inc = v;
+    unsigned long long inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      const unsigned long long u = __shfl_up_sync(0xffffffffu, inc, o);
       if (lane >= o) inc += u;
     }
-    uint32_t base = 0;
+    unsigned long long base = 0;
     if (lane == 31 && inc) base = atomicAdd(&B.counters->bin_needed, inc);
     base = __shfl_sync(0xffffffffu, base, 31);
-    if (t < B.n_tiles) B.tile_start[t] = base + inc - v;
+    // (a batch of 2^32 pairs and more is refused once it is read: its ranges
+    // may overlap, but every entry below bin_cap is a record's index)
+    if (t < B.n_tiles) B.tile_start[t] = (uint32_t)(base + inc - v);
   }
   grid.sync();
   // 2. scatter
@@ -1472,14 +1474,14 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   const uint32_t per = (nb * (nt >> 5) + kShares - 1 - share) / kShares;  // warps on this share
   for (uint32_t r0 = (gw / kShares) * 32; r0 < nrec; r0 += per * 32) {
     const uint32_t i = share * B.rec_share + r0 + lane;
-    uint32_t first = 0, pitch_t = 0;  // the record's first tile, tiles per row of its scene
-    int nx = 1, n = 0;                // columns and number of its tiles
+    uint32_t first = 0, pitch_t = 0, nx = 1;  // the record's first tile, tiles per row of its scene, columns
+    PairNo n = 0;                             // and number of its tiles
     if (r0 + lane < nrec) {
       const BigRec& R = B.recs[i];
       const SceneRec& SR = B.scenes[B.rec_scene[i]];
       const int tx0 = R.x0 / TW, ty0 = R.y0 / TH;
-      nx = R.x1 / TW - tx0 + 1;
-      n = nx * (R.y1 / TH - ty0 + 1);
+      nx = (uint32_t)(R.x1 / TW - tx0 + 1);
+      n = nx * (PairNo)(R.y1 / TH - ty0 + 1);
       pitch_t = (uint32_t)SR.tiles_x;
       first = SR.tile_base + (uint32_t)ty0 * pitch_t + (uint32_t)tx0;
     }

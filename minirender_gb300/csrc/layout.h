@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <vector_types.h>
 
+#include <limits>
+
 #include "../../include/minirender_gpu.h"
 
 namespace mrg {
@@ -15,6 +17,17 @@ namespace mrg {
 // fragment because real fragments need z < 1e11f (the clear value of the
 // reference z-buffer, src/Renderer.cpp:116) and id < 0xFFFFFFFF.
 static constexpr unsigned long long VIS_EMPTY = ~0ull;
+
+// Limits of a frame's sides and of a batch's tiles.
+constexpr int kMaxSide = 1 << 16;
+constexpr int kMinTilePx = 64;
+
+// Number of a (record, tile) pair among those of a warp's 32 records.  A
+// record as large as the largest scene lies in 2^26 of the smallest tiles:
+// 2^31 pairs, one more than an int holds.
+using PairNo = uint32_t;
+static_assert(32ull * ((unsigned long long)kMaxSide * kMaxSide / kMinTilePx) <= std::numeric_limits<PairNo>::max(),
+              "a warp's (record, tile) pairs need a wider PairNo");
 
 // One resident mesh (TriMesh arrays, include/minirender/Scene.h:73-87).
 struct DevMesh {
@@ -129,8 +142,8 @@ struct alignas(32) ShareSlot {
 struct Counters {
   StatSlot stat[kStatSlots];
   ShareSlot share[kShares];
+  unsigned long long bin_needed;  // total (tile, record) pairs requested
   unsigned int error_flags;
-  unsigned int bin_needed;     // total (tile, record) pairs requested
   unsigned int bin_overflow;
   unsigned int work_next;      // persistent-kernel work counter
   unsigned int spill_count;    // records whose remaining blocks did not fit the block list
