@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import weakref
 from typing import Optional
 
 import numpy as np
@@ -114,6 +115,8 @@ def _ptr(a: Optional[np.ndarray]):
 class Context:
     """One mr_ctx: resident meshes/textures and frame buffers on one GPU."""
 
+    _holders = ()
+
     def __init__(self, device: int = 0):
         h = _P()
         rc = lib().mr_create(device, C.byref(h))
@@ -128,10 +131,25 @@ class Context:
             raise MRError(rc, f"{what}: {lib().mr_last_error(self.h).decode()}")
         return rc
 
+    def hold(self, read_rest) -> None:
+        """Calls the bound method `read_rest` (kept by a weak reference) once,
+        before the last frame's outputs are replaced or released."""
+        self._holders = [*self._holders, weakref.WeakMethod(read_rest)]
+
+    def _release_held(self) -> None:
+        holders, self._holders = self._holders, ()
+        for ref in holders:
+            read_rest = ref()
+            if read_rest is not None:
+                read_rest()
+
     def close(self):
         if self.h:
-            lib().mr_destroy(self.h)
-            self.h = None
+            try:
+                self._release_held()
+            finally:
+                lib().mr_destroy(self.h)
+                self.h = None
 
     def __del__(self):
         try:
@@ -194,11 +212,17 @@ class Context:
         self._tex_layout.pop(handle, None)
 
     def render(self, frame: abi.mr_frame, renderables, n: int, outputs: int = abi.MR_OUT_DEFAULT):
+        if self._holders:
+            self._release_held()
+        rc = lib().mr_render(self.h, C.byref(frame), C.addressof(renderables) if n else None, n, outputs)
+        if rc != 0:
+            error = MRError(rc, f"mr_render: {lib().mr_last_error(self.h).decode()}")
+            # the library's last frame, whose size the reads go by: the one
+            # before, or this one where only its launch failed
+            o = abi.mr_outputs()
+            self._frame_hw = (o.height, o.width) if lib().mr_get_outputs(self.h, C.byref(o)) == 0 else None
+            raise error
         self._frame_hw = (frame.height, frame.width)
-        self._outputs = outputs
-        self._save_normals = bool(frame.save_normals)
-        self._check(lib().mr_render(self.h, C.byref(frame), C.addressof(renderables) if n else None,
-                                    n, outputs), "mr_render")
 
     def _hw(self):
         if self._frame_hw is None:

@@ -204,14 +204,25 @@ class Renderer:
         for key in [k for k in self._textures if k not in textures]:
             self.ctx.free_texture(self._textures.pop(key)[0])
 
+    def _draw(self, frame, rs, n):
+        """Renders a frame.  Outputs not read yet of the one it replaces are
+        let go, unless the call fails."""
+        out, self._out = self._out, None
+        try:
+            self.ctx.render(frame, rs, n, self.outputs)
+        except BaseException:
+            if out is not None:
+                self._out = out
+                self.ctx.hold(self._read_rest)
+            raise
+
     def render(self):
         """Renderer::render (src/Renderer.cpp:311-332)."""
         self._used = (set(), set())
         frame, rs, n = self.prepare()
-        self.ctx.render(frame, rs, n, self.outputs)
+        self._draw(frame, rs, n)
         self._base_used = (set(self._used[0]), set(self._used[1]))
         self._prune()
-        self._out = None
         self._rendered = True
         self._base = (rs, n)
         self._paints = []
@@ -231,11 +242,10 @@ class Renderer:
         for j in range(len(self._paints)):
             rs[base_n + j] = prs[j]
         frame = self._frame_c()
-        self.ctx.render(frame, rs, n, self.outputs)
+        self._draw(frame, rs, n)
         self._prune()
         self._rendered = True
         self._dirty = False
-        self._out = None
 
     def _frame_c(self):
         """mr_frame of a flush: the light, its view and the default switches
@@ -252,22 +262,46 @@ class Renderer:
         return frame
 
     def _read(self, name: Optional[str] = None) -> dict:
-        """The outputs of the last frame read so far, `name` among them: each
-        is copied from the device when it is first asked for."""
+        """The outputs read so far, `name` among them: those of the frame that
+        the context held when the first one was asked for.  Each is copied
+        when it is asked for; the context calls _read_rest before it replaces
+        that frame."""
         if self._dirty:
             self._flush_paints()
         if self._out is None:
             if not self._rendered:
                 return self._cleared()
             self._out = {}
+            self.ctx.hold(self._read_rest)
         want = set() if name is None or name in self._out else {name}
         if not self._out and self.state.save_normals:
             want.add("normals")
         if want:
-            self._out.update(self.ctx.read(rgb8="rgb8" in want, depth="depth" in want, rgb_f32="image" in want,
-                                           tri_id="ids" in want,
-                                           normals="normals" in want and self.state.save_normals))
+            try:
+                self._out.update(self.ctx.read(rgb8="rgb8" in want, depth="depth" in want, rgb_f32="image" in want,
+                                               tri_id="ids" in want,
+                                               normals="normals" in want and self.state.save_normals))
+            except capi.MRError:
+                if not self._out:
+                    self._out = None
+                raise
         return self._out
+
+    def _read_rest(self):
+        """Reads what has not been asked for yet of the frame whose outputs
+        are being read (what the first getter could not read is let go)."""
+        if self._out is None or self._dirty:
+            return
+        try:
+            o = self.ctx.outputs()
+            rest = {arg: bool(ptr) and name not in self._out for arg, name, ptr in (
+                ("rgb8", "rgb8", o.rgb8), ("depth", "depth", o.depth), ("rgb_f32", "image", o.rgb_f32),
+                ("tri_id", "ids", o.tri_id), ("normals", "normals", o.normals if self.state.save_normals else None))}
+            if any(rest.values()):
+                self._out.update(self.ctx.read(**rest))
+        except capi.MRError:
+            if not self._out:
+                self._out = None
 
     def _cleared(self) -> dict:
         H, W = self.state.height, self.state.width
@@ -308,10 +342,5 @@ class Renderer:
         return self.ctx.stats()
 
     def close(self):
-        # outputs of a frame that was being read stay available
-        if self._out and not self._dirty and self.ctx.h:
-            for name, bit in (("rgb8", abi.MR_OUT_RGB8), ("depth", abi.MR_OUT_DEPTH), ("image", abi.MR_OUT_RGB_F32),
-                              ("ids", abi.MR_OUT_TRI_ID)):
-                if self.ctx._outputs & bit:
-                    self._read(name)
+        # (outputs of a frame that was being read stay available)
         self.ctx.close()
