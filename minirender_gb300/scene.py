@@ -96,9 +96,11 @@ class Scene(SceneNode):
 
 
 def _floats(a) -> list:
-    """The numbers of an array as Python floats (one call for an array: a
-    frame of 64 meshes converts some 1600 of them)."""
-    return a.ravel().tolist() if isinstance(a, np.ndarray) else [float(x) for x in a]
+    """The numbers of a row as Python floats (one call for an array of them: a
+    frame of 64 meshes converts some 1600)."""
+    if type(a) is np.ndarray and a.ndim == 1 and a.dtype.kind == "f":
+        return a.tolist()
+    return [float(x) for x in a]
 
 
 def _fill_material(dst: abi.mr_material, m: Material, tex_index: int) -> None:
@@ -121,7 +123,7 @@ class Flat:
         self.textures = textures
 
 
-def _fill_nodes(nodes, order, mesh_of, tex_of) -> None:
+def _fill_fields(nodes, order, mesh_of, tex_of) -> None:
     for i, (node, parent) in enumerate(order):
         nd = nodes[i]
         nd.parent = parent
@@ -134,26 +136,46 @@ def _fill_nodes(nodes, order, mesh_of, tex_of) -> None:
             _fill_material(nd.material, node.material, tex_of[i])
 
 
+_fill_nodes = _fill_fields
+
+
+def _rows(colours):
+    """Colours as the rows of an array, where every one is a row of three
+    floats; None where one is anything else (numpy would spread a number, or a
+    row of one, over all of them)."""
+    try:
+        a = np.array(colours)
+    except ValueError:
+        return None
+    return a if a.shape == (len(colours), 3) and a.dtype in (np.float32, np.float64) else None
+
+
 def _fill_columns(nodes, order, mesh_of, tex_of) -> None:
     """_fill_nodes a column at a time: field by field, ctypes took most of a
     frame's host time (64 meshes: 300 us of the 540 that a render and its
-    reads took; here 90).  Fewer than four nodes are quicker field by field."""
+    reads took; here 90).  Fewer than four nodes are quicker field by field,
+    and colours that are no rows of three floats are left to that."""
+    lit = [i for i, (node, _) in enumerate(order) if mesh_of[i] >= 0 and node.material is not None]
+    mats = [order[i][0].material for i in lit]
+    rows = {name: _rows([getattr(m, name) for m in mats]) for name in ("diffuse", "specular", "emissive")} if lit else {}
+    if any(r is None for r in rows.values()):
+        return _fill_fields(nodes, order, mesh_of, tex_of)
     col = np.frombuffer(nodes, _NODE)
     col["parent"] = [parent for _, parent in order]
     transforms = [node.transform for node, _ in order]
-    col["transform"] = np.array([t if getattr(t, "shape", None) == (4, 4) else np.reshape(t, (4, 4)) for t in transforms],
-                                np.float32).reshape(len(order), 16)
-    col["mesh"] = mesh_of
-    col["opacity"] = 1.0
-    lit = [i for i, (node, _) in enumerate(order) if mesh_of[i] >= 0 and node.material is not None]
-    if lit:
-        mats = [order[i][0].material for i in lit]
-        col["has_material"][lit] = 1
-        col["opacity"][lit] = [m.opacity for m in mats]
-        material = col["material"]
-        for name in ("diffuse", "specular", "emissive", "shininess"):
-            material[name][lit] = np.array([getattr(m, name) for m in mats], np.float32)
-        material["texture"] = tex_of
+    with np.errstate(all="ignore"):  # (overflows as a C cast to float does)
+        col["transform"] = np.array([t if getattr(t, "shape", None) == (4, 4) else np.reshape(t, (4, 4)) for t in transforms],
+                                    np.float32).reshape(len(order), 16)
+        col["mesh"] = mesh_of
+        col["opacity"] = 1.0
+        if lit:
+            col["has_material"][lit] = 1
+            col["opacity"][lit] = [float(m.opacity) for m in mats]
+            material = col["material"]
+            for name, r in rows.items():
+                material[name][lit] = r
+            material["shininess"][lit] = [float(m.shininess) for m in mats]
+            material["texture"] = tex_of
 
 
 def flatten(scene: SceneNode) -> Flat:
