@@ -678,15 +678,13 @@ MR_API int mr_render(mr_ctx* c, const mr_frame* f, const mr_renderable* rs, int3
   CK(c->recs.ensure(share * kShares), "record buffer");
   CK(c->spill.ensure(share * kShares), "spill buffer");
   if (c->items.cap < ((size_t)1 << 19)) CK(c->items.ensure((size_t)1 << 19), "block list");
-  // The per-vertex pass pays off when vertices are shared (each one used by
-  // two or more triangle corners on average); for triangle soups every
-  // corner is its own vertex and the kernels transform corners themselves.
-  const bool vertex_pass = 3 * (uint64_t)total >= 2 * (uint64_t)vbase;
+  const bool vertex_pass = wants_vertex_pass(total, vbase);
   if (vertex_pass) {
-    CK(c->va.ensure(vbase), "vertex buffer");
-    CK(c->vc.ensure(2 * vbase), "vertex buffer");
-    if (n != 1) CK(c->tri.ensure(total), "triangle table");
-    CK(c->vn.ensure(nbase), "normal buffer");
+    const PassBuffers need = pass_buffers((size_t)total, (size_t)vbase, (size_t)nbase);
+    CK(c->va.ensure(need.va), "vertex buffer");
+    CK(c->vc.ensure(need.vc), "vertex buffer");
+    if (n != 1) CK(c->tri.ensure(need.tri), "triangle table");
+    CK(c->vn.ensure(need.vn), "normal buffer");
   }
   FrameParams& F = c->last;
   memset(&F, 0, sizeof(F));
@@ -1138,13 +1136,13 @@ int batch_stage(mr_ctx* c, BatchSlot& B, const mr_batch_scene* sc, int32_t n_sce
   CK(B.rs.ensure((size_t)n_rs), "batch renderables");
   CK(B.bases.ensure((size_t)3 * (n_rs + 1) + n_scenes + 1), "batch bases");
   CK(B.scenes.ensure((size_t)n_scenes), "batch scenes");
-  // per-vertex pass only when vertices are shared (see mr_render)
-  const bool vertex_pass = 3 * tris >= 2 * verts;
+  const PassBuffers need = pass_buffers((size_t)tris, (size_t)verts, (size_t)nrms);
+  const bool vertex_pass = wants_vertex_pass(tris, verts) && need.bytes() <= B.pass_limit;
   if (vertex_pass) {
-    CK(B.va.ensure(verts), "batch vertex buffer");
-    CK(B.vc.ensure(2 * verts), "batch vertex buffer");
-    CK(B.tri.ensure(tris), "batch triangle table");
-    CK(B.vn.ensure(nrms), "batch normal buffer");
+    CK(B.va.ensure(need.va), "batch vertex buffer");
+    CK(B.vc.ensure(need.vc), "batch vertex buffer");
+    CK(B.tri.ensure(need.tri), "batch triangle table");
+    CK(B.vn.ensure(need.vn), "batch normal buffer");
   }
   const size_t share = rec_share_for((size_t)tris);
   CK(B.recs.ensure(share * kShares), "batch records");

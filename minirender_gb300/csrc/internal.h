@@ -94,6 +94,19 @@ inline void set_reads(DevRenderable& R) {
            (R.lit && (R.point || R.shininess != 0) ? kNeedPosition : 0);
 }
 
+// The per-vertex pass pays off when vertices are shared (each one used by two
+// or more triangle corners on average); for triangle soups every corner is its
+// own vertex and the kernels transform corners themselves.
+inline bool wants_vertex_pass(uint64_t tris, uint64_t verts) { return 3 * tris >= 2 * verts; }
+
+// Elements of the vertex pass's buffers (Geo::va, vc, tri, vn) for so many
+// triangles, vertices and normals with a buffer of their own, and their bytes.
+struct PassBuffers {
+  size_t va, vc, tri, vn;
+  size_t bytes() const { return (va + vc + vn) * sizeof(float4) + tri * sizeof(uint4); }
+};
+inline PassBuffers pass_buffers(size_t tris, size_t verts, size_t nrms) { return {verts, 2 * verts, tris, nrms}; }
+
 inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace mrgi
@@ -107,6 +120,7 @@ struct BatchSlot {
   int tile_w = 16, tile_h = 16, threads = 256, chunk = 64;
   int small_max = 64;  // bbox pixels up to which the setup kernel rasterises (0: every triangle binned)
   bool graphs = true;
+  size_t pass_limit = SIZE_MAX;  // bytes the vertex pass may take (more: the kernels transform corners themselves)
   DevBuf<DevRenderable> rs;
   DevBuf<uint32_t> bases;
   DevBuf<SceneRec> scenes;

@@ -36,6 +36,7 @@ struct Request {
   uint64_t ticket = 0;
   mr_request req{};
   size_t cost = 0;      // footprint while queued/running
+  size_t pass = 0;      // of this, for the vertex pass
   size_t scene_px = 0;
   double t_submit = 0, t_launch = 0, t_done = 0;
   int status = 1;       // 1 queued, 2 running, 0 done
@@ -57,6 +58,7 @@ struct Slot {
   BatchSlot b;
   cudaStream_t stream = nullptr;
   std::vector<Request*> reqs;
+  size_t extra = 0;  // committed for the running batch's vertex pass beyond its requests' charges
   bool busy = false;
 };
 
@@ -65,6 +67,16 @@ size_t mesh_footprint(const mr_mesh_desc& d) {
   return (size_t)12 * d.n_vertices + (size_t)12 * d.n_normals + (size_t)8 * d.n_texcoords +
          (size_t)12 * d.n_indices + nt / 8 + 4096 +
          (mesh_wants_records((long long)nt, d.n_vertices) ? kRecBytes * nt : 0);
+}
+
+// Device bytes a request is charged for its batch's vertex pass: what it takes
+// alone.  A soup alone takes none; what it is charged goes towards the pass of
+// a batch that also holds meshes with shared vertices (see launch).
+size_t pass_footprint(const mr_mesh_desc& d) {
+  const size_t nt = (size_t)(d.n_indices / 3), nv = (size_t)d.n_vertices, nn = (size_t)d.n_normals;
+  const bool has_uv = d.n_texcoords > 0 && d.n_texcoordsI > 0;
+  const bool unified = d.normalsI == d.indices && (!has_uv || d.texcoordsI == d.indices);
+  return wants_vertex_pass(nt, nv) ? pass_buffers(nt, nv, unified ? 0 : nn).bytes() : 24 * nv + 16 * nn;
 }
 
 // Device bytes a request occupies while it runs: its outputs and the
@@ -77,8 +89,8 @@ size_t request_footprint(const mr_request& r) {
   if (r.outputs & MR_OUT_RGB8) out += 3 * px;
   if (r.outputs & MR_OUT_DEPTH) out += 4 * px;
   if (r.outputs & MR_OUT_TRI_ID) out += 4 * px;
-  return out + nt * (2 * sizeof(BigRec) + 16) + (size_t)r.mesh.n_vertices * 24 +
-         (size_t)r.mesh.n_normals * 16 + (px / 64 + 16) * 12 + sizeof(DevRenderable) + sizeof(SceneRec);
+  return out + nt * (2 * sizeof(BigRec) + 16) + pass_footprint(r.mesh) + (px / 64 + 16) * 12 +
+         sizeof(DevRenderable) + sizeof(SceneRec);
 }
 
 }  // namespace
@@ -150,6 +162,8 @@ void mr_server::launch(Slot* s, std::vector<Request*>& batch) {
   std::vector<mr_renderable> rs(batch.size());
   int32_t outputs = 0;
   int rc = MR_OK;
+  uint64_t tris = 0, verts = 0, nrms = 0;
+  size_t charged = 0;  // for the batch's vertex pass
   {
     std::lock_guard<std::recursive_mutex> g(c->mu);
     cudaSetDevice(c->device);
@@ -185,7 +199,25 @@ void mr_server::launch(Slot* s, std::vector<Request*>& batch) {
       rs[i].material = r->req.material;
       rs[i].material.texture = th;
       outputs |= r->req.outputs;
+      const DevMesh& M = c->meshes[mh].d;
+      tris += (uint64_t)M.n_tri;
+      verts += (uint64_t)M.n_pos;
+      nrms += mesh_unified(M) ? 0 : (uint64_t)M.n_nrm;
+      charged += r->pass;
     }
+    // Soups among meshes with shared vertices go through the vertex pass, too,
+    // which takes more than they were charged: the budget makes up for it, or
+    // the batch runs without the pass (the same pixels).
+    const size_t need = wants_vertex_pass(tris, verts) ? pass_buffers(tris, verts, nrms).bytes() : 0;
+    if (need > charged) {
+      std::lock_guard<std::mutex> lk(m);
+      if (committed + (need - charged) <= o.budget_bytes) {
+        s->extra = need - charged;
+        committed += s->extra;
+        charged = need;
+      }
+    }
+    s->b.pass_limit = charged;
     rc = batch_stage(c, s->b, scenes.data(), (int32_t)scenes.size(), rs.data(), (int32_t)rs.size(), outputs);
     if (rc == MR_OK) rc = batch_run(c, s->b, s->stream, false, nullptr);
     if (rc == MR_OK) {
@@ -256,6 +288,8 @@ void mr_server::retire(Slot* s) {
     completed++;
     t_last = t;
   }
+  committed -= s->extra;
+  s->extra = 0;
   s->reqs.clear();
   s->busy = false;
   cv_done.notify_all();
@@ -509,6 +543,7 @@ MR_API int mr_server_submit(mr_server* s, const mr_request* q, uint64_t* ticket)
   r->mesh_key = q->mesh_key;
   r->tex_key = q->texture_key;
   r->cost = request_footprint(*q);
+  r->pass = pass_footprint(q->mesh);
   const size_t own = r->cost + mesh_footprint(q->mesh) + (size_t)q->tex_rows * q->tex_cols * 3;
   std::lock_guard<std::mutex> lk(s->m);
   if (own > s->o.budget_bytes) {
