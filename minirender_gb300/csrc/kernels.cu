@@ -516,7 +516,7 @@ __device__ __forceinline__ int large_blocks(int x0, int y0, int x1, int y1) {
 // The counters' slots of a warp: its statistics, and its share of the record
 // store and block list.
 __device__ __forceinline__ uint32_t warp_slot() { return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kStatSlots; }
-__device__ __forceinline__ uint32_t warp_share() { return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kShares; }
+__device__ __forceinline__ uint32_t warp_share() { return share_of_warp((blockIdx.x * blockDim.x + threadIdx.x) >> 5); }
 
 // Adds a warp's sub-triangles (small: rasterised by the setup kernel) and
 // cut triangles to its statistics slot.  Called by all lanes of the warp.

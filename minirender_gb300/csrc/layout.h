@@ -133,6 +133,20 @@ struct alignas(32) StatSlot {
 // update takes some 2 ns, 10 us of the setup of 327,680 triangles of 18
 // pixels.  (64 shares cost the large raster 2 us to add up, 16 cost none.)
 constexpr int kShares = 16;
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+// The share of setup warp w: one warp of each sixteen in a row to a share, in
+// an order that differs from sixteen to sixteen, so that large triangles that
+// recur every so many warps do not all meet in one.  (400,000 triangles at
+// 1080p, the 32 of every sixteenth warp large, in the fixed store of the
+// allocation-free entry: 388 us with w % 16, where five of six found their
+// share full, 215 so.)
+inline uint32_t share_of_warp(uint32_t w) {
+  uint32_t h = (w / kShares) * 0x9E3779B1u;  // (two odd multipliers; any that mix would do)
+  h = (h ^ (h >> 15)) * 0x2C1B3C6Du;
+  return (w ^ (h >> 28)) % kShares;
+}
 struct alignas(32) ShareSlot {
   unsigned long long item_count;  // large-triangle blocks requested (single frames; 64 bits: a frame
                                   // of many screen-sized triangles passes 2^32)
@@ -165,8 +179,8 @@ constexpr int kLargeRows = 32;
 constexpr int kLargeCols = 16, kLargeSegs = 16;
 
 // Records per share in which T triangles always find room: a share's warps hold
-// at most T / kShares + 64 of them (setup warps, 2 to 32 triangles each, take
-// shares in turn), two sub-triangles each.
+// at most T / kShares + 64 of them (of each sixteen setup warps, 2 to 32
+// triangles each, one), two sub-triangles each.
 inline size_t rec_share_for(size_t T) { return T / (kShares / 2) + 128; }
 
 struct FrameParams {

@@ -194,3 +194,53 @@ def test_batches_of_growing_and_shrinking_frames(product_lib):
                 _same(br.read(k), ref, f"{w}x{h} scene {k}")
     finally:
         br.close()
+
+
+def _share_of_warp(w):
+    """layout.h's share_of_warp."""
+    h = (w // 16 * 0x9E3779B1) & 0xFFFFFFFF
+    h = ((h ^ (h >> 15)) * 0x2C1B3C6D) & 0xFFFFFFFF
+    return (w ^ (h >> 28)) % 16
+
+
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_overfull_record_shares(product_lib, noalloc):
+    """Warps of 32 triangles, 29 of them large, in three shares of sixteen: each
+    of these holds more than the fixed store has room for in a share, the last
+    warp that finds room not for all of its own; the others hold one each.  In
+    the growing store every large triangle has a record."""
+    import test_zz_no_alloc as N
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    warps = max(16 * sms, 16 * 150)
+    t = np.arange(32 * warps)
+    share = np.array([_share_of_warp(w) for w in range(warps)])[t // 32]
+    large = np.where(share < 3, t % 32 < 29, t % (32 * 97) == 5)
+    per_share = np.bincount(share[large], minlength=16)
+    cap = 32768 // 16  # of the fixed store
+    assert per_share[:3].min() > cap and 0 < per_share[3:].max() < cap and cap % 29
+    rng = np.random.default_rng(5)
+    w, h = 320, 240
+    size = np.where(large, 12.0, 1.6)[:, None]  # boxes of 13x13 and 2x2 or 3x3 pixels
+    c = np.stack([rng.uniform(-w / 2, w / 2 - 13, t.size), rng.uniform(-h / 2, h / 2 - 13, t.size)], 1)
+    z = -rng.uniform(2, 50, (t.size, 3, 1))
+    v = np.concatenate([np.stack([c, c + size * [1, 0], c + size * [0.5, 1]], 1), z], 2).astype(np.float32)
+    idx = np.arange(3 * t.size, dtype=np.int32)
+    nrm = np.tile(np.array([[0.2, 0.3, 1]], np.float32), (3 * t.size, 1))
+    sc = S.Scene()
+    sc.add(S.TriMesh(v.reshape(-1, 3), nrm, idx, normalsI=idx, material=S.Material()))
+    st = FrameState(width=w, height=h, projection=pj.projection_ortho(-w / 2, w / 2, -h / 2, h / 2, 1, 60),
+                    light=np.array([0.3, 0.4, 1], np.float32))
+    ref = O.render(st, sc)
+    if noalloc:
+        _same(N._noalloc(st, sc, calls=2)[1], ref, "fixed store")
+        return
+    r = Renderer(0)
+    try:
+        r.state = st
+        r.setScene(sc)
+        r.render()
+        _same({"rgb8": r.getImageRGB8(), "depth": r.getDepth(), "ids": r.getTriangleIds()}, ref, "growing store")
+        assert r.stats().binned == large.sum()
+    finally:
+        r.close()

@@ -29,3 +29,26 @@ def test_pair_numbers_hold_a_warp_of_frame_sized_records(tmp_path):
       printf("%llu %llu", most, (unsigned long long)std::numeric_limits<mrg::PairNo>::max());""")
     assert int(most) == 1 << 31
     assert int(held) >= int(most)
+
+
+def test_warps_are_spread_over_the_record_shares(tmp_path):
+    """Of each sixteen warps in a row one goes to each share (what the stores'
+    sizes count on), and warps that recur at any regular distance meet in no
+    share more than twice as often as in the mean."""
+    bad_rows, worst = _run(tmp_path, """
+      int bad = 0;
+      double worst = 0;
+      for (uint32_t g = 0; g < 70000; g++) {
+        unsigned seen = 0;
+        for (uint32_t k = 0; k < 16; k++) seen |= 1u << mrg::share_of_warp(16 * g + k);
+        bad += seen != 0xffffu;
+      }
+      for (uint32_t step = 1; step <= 1024; step++)
+        for (uint32_t first = 0; first < 16; first++) {
+          int n[mrg::kShares] = {};
+          for (uint32_t k = 0; k < 1024; k++) n[mrg::share_of_warp(first + k * step)]++;
+          for (int c : n) worst = c > worst ? c : worst;
+        }
+      printf("%d %g", bad, worst / (1024 / mrg::kShares));""")
+    assert int(bad_rows) == 0
+    assert float(worst) <= 2
