@@ -128,25 +128,26 @@ struct alignas(32) StatSlot {
   unsigned long long clipped;  // triangles cut by the near plane
 };
 
-// Counters of one share of the record store and of the block list.  Every warp
-// of the setup waits for these, so they are spread, too: on one address an
-// update takes some 2 ns, 10 us of the setup of 327,680 triangles of 18
-// pixels.  (64 shares cost the large raster 2 us to add up, 16 cost none.)
 constexpr int kShares = 16;
+// The share of the record store and of the block list that setup warp w uses:
+// one warp of each sixteen in a row to a share, in an order that differs from
+// sixteen to sixteen, so that large triangles that recur every so many warps
+// do not all meet in one.  (400,000 triangles at 1080p, the 32 of every
+// sixteenth warp large, in the fixed store of the allocation-free entry: 388
+// us with w % 16, where five of six found their share full, 215 so.)
 #ifdef __CUDACC__
 __host__ __device__
 #endif
-// The share of setup warp w: one warp of each sixteen in a row to a share, in
-// an order that differs from sixteen to sixteen, so that large triangles that
-// recur every so many warps do not all meet in one.  (400,000 triangles at
-// 1080p, the 32 of every sixteenth warp large, in the fixed store of the
-// allocation-free entry: 388 us with w % 16, where five of six found their
-// share full, 215 so.)
 inline uint32_t share_of_warp(uint32_t w) {
   uint32_t h = (w / kShares) * 0x9E3779B1u;  // (two odd multipliers; any that mix would do)
   h = (h ^ (h >> 15)) * 0x2C1B3C6Du;
   return (w ^ (h >> 28)) % kShares;
 }
+
+// Counters of one share of the record store and of the block list.  Every warp
+// of the setup waits for these, so they are spread, too: on one address an
+// update takes some 2 ns, 10 us of the setup of 327,680 triangles of 18
+// pixels.  (64 shares cost the large raster 2 us to add up, 16 cost none.)
 struct alignas(32) ShareSlot {
   unsigned long long item_count;  // large-triangle blocks requested (single frames; 64 bits: a frame
                                   // of many screen-sized triangles passes 2^32)

@@ -18,6 +18,7 @@
 // records and blocks in the array as in mr_render, up to kRecCap / kShares in
 // each share; any further ones are rasterised by the setup kernel itself.  Calls whose GPU work overlaps race on the array.
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <string.h>
 
 #include <mutex>
@@ -156,9 +157,10 @@ extern "C" MR_API int mr_render_noalloc(const mr_frame* f, const mr_mesh_desc* d
 
   cudaError_t e = launch_validate(M, (uint32_t*)(S + kBadOff), st);
   if (e == cudaSuccess) e = launch_frame(F, st, nullptr);
-  Counters c;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&c, S + kCntOff, sizeof(c), cudaMemcpyDeviceToHost, st);
+  unsigned int flags = 0;
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&flags, S + kCntOff + offsetof(Counters, error_flags), sizeof(flags), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return MR_E_CUDA;
-  return (c.error_flags & 1u) ? MR_E_BAD_INDEX : MR_OK;
+  return (flags & 1u) ? MR_E_BAD_INDEX : MR_OK;
 }
