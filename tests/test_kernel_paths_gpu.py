@@ -244,3 +244,34 @@ def test_overfull_record_shares(product_lib, noalloc):
         assert r.stats().binned == large.sum()
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("n,box,frame", [(600, 900, 1000), (900, 500, 600), (2500, 250, 300), (30000, 100, 400)])
+def test_spilled_blocks(product_lib, n, box, frame):
+    """Large triangles whose blocks pass the fixed store's list, from a few
+    hundred spilled records (many warps on each) to more than there are warps,
+    and with records whose first blocks found room."""
+    import test_zz_no_alloc as N
+    rng = np.random.default_rng(n)
+    side = box * rng.uniform(0.6, 1, (n, 1))
+    at = np.stack([rng.uniform(-frame / 2, frame / 2 - 0.6 * box, n), rng.uniform(-frame / 2, frame / 2 - 0.6 * box, n)], 1)
+    third = rng.uniform(0, 1, (n, 1))
+    z = -rng.uniform(2, 50, (n, 3, 1))
+    v = np.concatenate([np.stack([at, at + side * [1, 0.02], at + side * np.concatenate([third, np.ones((n, 1))], 1)], 1), z], 2)
+    idx = np.arange(3 * n, dtype=np.int32)
+    nrm = np.tile(np.array([[0.2, 0.3, 1]], np.float32), (3 * n, 1))
+    sc = S.Scene()
+    sc.add(S.TriMesh(v.astype(np.float32).reshape(-1, 3), nrm, idx, normalsI=idx, material=S.Material()))
+    st = FrameState(width=frame, height=frame, projection=pj.projection_ortho(-frame / 2, frame / 2, -frame / 2, frame / 2, 1, 60),
+                    light=np.array([0.3, 0.4, 1], np.float32))
+    ref = O.render(st, sc)
+    _same(N._noalloc(st, sc, calls=2)[1], ref, "fixed store")
+    r = Renderer(0)
+    try:
+        r.state = st
+        r.setScene(sc)
+        r.render()
+        assert r.stats().bin_entries > 1 << 17  # blocks the fixed store lists
+        _same({"rgb8": r.getImageRGB8(), "depth": r.getDepth(), "ids": r.getTriangleIds()}, ref, "growing store")
+    finally:
+        r.close()
