@@ -112,6 +112,7 @@ def _fill_material(dst: abi.mr_material, m: Material, tex_index: int) -> None:
 
 
 _NODE = np.dtype(abi.mr_node)
+_FLOATS = (np.dtype(np.float32), np.dtype(np.float64))
 
 
 class Flat:
@@ -141,13 +142,13 @@ _fill_nodes = _fill_fields
 
 def _rows(colours):
     """Colours as the rows of an array, where every one is a row of three
-    floats; None where one is anything else (numpy would spread a number, or a
-    row of one, over all of them)."""
+    floats; None where one is anything else (as a column numpy would spread a
+    number, or a row of one, over all of them)."""
     try:
         a = np.array(colours)
     except ValueError:
         return None
-    return a if a.shape == (len(colours), 3) and a.dtype in (np.float32, np.float64) else None
+    return a if a.shape == (len(colours), 3) and a.dtype in _FLOATS else None
 
 
 def _fill_columns(nodes, order, mesh_of, tex_of) -> None:
@@ -157,24 +158,27 @@ def _fill_columns(nodes, order, mesh_of, tex_of) -> None:
     and colours that are no rows of three floats are left to that."""
     lit = [i for i, (node, _) in enumerate(order) if mesh_of[i] >= 0 and node.material is not None]
     mats = [order[i][0].material for i in lit]
-    rows = {name: _rows([getattr(m, name) for m in mats]) for name in ("diffuse", "specular", "emissive")} if lit else {}
-    if any(r is None for r in rows.values()):
-        return _fill_fields(nodes, order, mesh_of, tex_of)
+    n = len(mats)
+    if n:
+        rows = _rows([m.diffuse for m in mats] + [m.specular for m in mats] + [m.emissive for m in mats])
+        if rows is None:
+            return _fill_fields(nodes, order, mesh_of, tex_of)
     col = np.frombuffer(nodes, _NODE)
     col["parent"] = [parent for _, parent in order]
-    transforms = [node.transform for node, _ in order]
-    with np.errstate(all="ignore"):  # (overflows as a C cast to float does)
-        col["transform"] = np.array([t if getattr(t, "shape", None) == (4, 4) else np.reshape(t, (4, 4)) for t in transforms],
-                                    np.float32).reshape(len(order), 16)
+    transforms = [t if getattr(t, "shape", None) == (4, 4) else np.reshape(t, (4, 4)) for t in [node.transform for node, _ in order]]
+    with np.errstate(over="ignore"):  # (as a C cast to float)
+        col["transform"] = np.concatenate(transforms).reshape(len(order), 16)
         col["mesh"] = mesh_of
         col["opacity"] = 1.0
-        if lit:
-            col["has_material"][lit] = 1
-            col["opacity"][lit] = [float(m.opacity) for m in mats]
+        if n:
+            at = np.array(lit)
+            col["has_material"][at] = 1
+            col["opacity"][at] = [float(m.opacity) for m in mats]
             material = col["material"]
-            for name, r in rows.items():
-                material[name][lit] = r
-            material["shininess"][lit] = [float(m.shininess) for m in mats]
+            material["diffuse"][at] = rows[:n]
+            material["specular"][at] = rows[n:2 * n]
+            material["emissive"][at] = rows[2 * n:]
+            material["shininess"][at] = [float(m.shininess) for m in mats]
             material["texture"] = tex_of
 
 
