@@ -132,13 +132,12 @@ class Context:
         return rc
 
     def hold(self, read_rest) -> None:
-        """Calls the bound method `read_rest` (kept by a weak reference) once,
-        before the last frame's outputs are replaced or released."""
-        self._holders = [*self._holders, weakref.WeakMethod(read_rest)]
+        """Calls the bound method `read_rest` (kept by a weak reference) before
+        each time that the last frame's outputs are replaced or released."""
+        self._holders = [*(ref for ref in self._holders if ref() is not None), weakref.WeakMethod(read_rest)]
 
-    def _release_held(self) -> None:
-        holders, self._holders = self._holders, ()
-        for ref in holders:
+    def _read_held(self) -> None:
+        for ref in self._holders:
             read_rest = ref()
             if read_rest is not None:
                 read_rest()
@@ -146,7 +145,7 @@ class Context:
     def close(self):
         if self.h:
             try:
-                self._release_held()
+                self._read_held()
             finally:
                 lib().mr_destroy(self.h)
                 self.h = None
@@ -212,8 +211,7 @@ class Context:
         self._tex_layout.pop(handle, None)
 
     def render(self, frame: abi.mr_frame, renderables, n: int, outputs: int = abi.MR_OUT_DEFAULT):
-        if self._holders:
-            self._release_held()
+        self._read_held()
         rc = lib().mr_render(self.h, C.byref(frame), C.addressof(renderables) if n else None, n, outputs)
         if rc != 0:
             error = MRError(rc, f"mr_render: {lib().mr_last_error(self.h).decode()}")

@@ -42,6 +42,8 @@ class Renderer:
         self._meshes: Dict[tuple, tuple] = {}   # geometry key -> (handle, version, vertices)
         self._textures: Dict[int, tuple] = {}   # id(array) -> (handle, array)
         self._out: Optional[dict] = None
+        self._whole = False                    # whether _out holds all that its frame has
+        self._held_by: Optional[capi.Context] = None  # calls _read_rest before it replaces the outputs
         self._rendered = False
         self._base = None                      # (renderables, count) of the last render()
         self._paints: list = []                # paintMesh / paintTriangle since then
@@ -211,9 +213,7 @@ class Renderer:
         try:
             self.ctx.render(frame, rs, n, self.outputs)
         except BaseException:
-            if out is not None:
-                self._out = out
-                self.ctx.hold(self._read_rest)
+            self._out = out
             raise
 
     def render(self):
@@ -272,7 +272,12 @@ class Renderer:
             if not self._rendered:
                 return self._cleared()
             self._out = {}
-            self.ctx.hold(self._read_rest)
+            self._whole = False
+            if self._held_by is not self.ctx:
+                self.ctx.hold(self._read_rest)
+                self._held_by = self.ctx
+        if self._whole:  # (the context's frame may be another by now)
+            return self._out
         want = set() if name is None or name in self._out else {name}
         if not self._out and self.state.save_normals:
             want.add("normals")
@@ -290,8 +295,9 @@ class Renderer:
     def _read_rest(self):
         """Reads what has not been asked for yet of the frame whose outputs
         are being read (what the first getter could not read is let go)."""
-        if self._out is None or self._dirty:
+        if self._out is None or self._whole or self._dirty:
             return
+        self._whole = True
         try:
             o = self.ctx.outputs()
             rest = {arg: bool(ptr) and name not in self._out for arg, name, ptr in (

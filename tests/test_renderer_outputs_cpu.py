@@ -107,6 +107,22 @@ def test_outputs_are_the_contexts_frame_when_first_asked_for(fake):
     assert _frames(r) == dict.fromkeys(GETTERS, 2)
 
 
+def test_what_could_not_be_read_is_of_no_other_frame(fake):
+    """After a read of the rest that fails, the outputs not read are gone, not
+    the next frame's."""
+    r = _renderer()
+    r.render()
+    r.getDepth()
+    fake.fail["mr_read"] = abi.MR_E_CUDA
+    r.ctx.render(*r.prepare(), abi.MR_OUT_DEFAULT)
+    del fake.fail["mr_read"]
+    assert int(np.unique(r.getDepth()).item()) == 1
+    with pytest.raises(KeyError):
+        r.getImage()
+    r.render()
+    assert _frames(r) == dict.fromkeys(GETTERS, 3)
+
+
 def test_a_render_reads_nothing_of_the_frame_it_replaces(fake):
     r = _renderer()
     for _ in range(3):
