@@ -275,3 +275,43 @@ def test_spilled_blocks(product_lib, n, box, frame):
         _same({"rgb8": r.getImageRGB8(), "depth": r.getDepth(), "ids": r.getTriangleIds()}, ref, "growing store")
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("meshes", [1, 3])
+@pytest.mark.parametrize("shared", [False, True], ids=["soup", "shared"])
+@pytest.mark.parametrize("w,h", [(65536, 20), (20, 65536), (40000, 33)])
+def test_frames_of_the_largest_sides(product_lib, w, h, shared, meshes):
+    """Coordinates past 32767 (the small raster packs two into 32 bits) and
+    triangles as long as the frame (column segments of thousands of columns)."""
+    rng = np.random.default_rng(w + shared)
+    n = 600
+    small = np.arange(n) % 20 > 0
+    size = np.stack([np.where(small, rng.uniform(1, 11, n), rng.uniform(0.1, 1, n) * w),
+                     np.where(small, rng.uniform(1, 11, n), rng.uniform(0.1, 1, n) * h)], 1)
+    at = np.stack([rng.uniform(-w / 2, w / 2, n), rng.uniform(-h / 2, h / 2, n)], 1)
+    at[::3] = [w / 2, h / 2] - at[::3] % 12  # many in the last columns and rows
+    at = np.where(small[:, None], at, np.minimum(at, [w / 2, h / 2] - size))
+    z = -rng.uniform(2, 50, (n, 3, 1))
+    v = np.concatenate([np.stack([at, at + size * [1, 0.1], at + size * [0.4, 1]], 1), z], 2).astype(np.float32)
+    sc = S.Scene()
+    for part in np.array_split(v, meshes):
+        k = 3 * len(part)
+        idx = np.arange(k, dtype=np.int32)
+        if shared:
+            idx = np.concatenate([idx, idx])
+        nrm = np.tile(np.array([[0.2, 0.3, 1]], np.float32), (k, 1))
+        sc.add(S.TriMesh(part.reshape(-1, 3), nrm, idx, normalsI=idx, material=S.Material()))
+    st = FrameState(width=w, height=h, projection=pj.projection_ortho(-w / 2, w / 2, -h / 2, h / 2, 1, 60),
+                    light=np.array([0.3, 0.4, 1], np.float32))
+    ref = O.render(st, sc)
+    drawn = np.nonzero(ref["ids"] != 0xFFFFFFFF)
+    assert drawn[1 if w > h else 0].max() > 0.99 * max(w, h)
+    _same(_render(st, sc), ref, "frame")
+    from minirender_gb300.batch import BatchRenderer
+    br = BatchRenderer(0)
+    try:
+        br.render([(st, sc), (st, sc)])
+        for k in range(2):
+            _same(br.read(k), ref, f"batch scene {k}")
+    finally:
+        br.close()
