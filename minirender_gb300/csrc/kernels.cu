@@ -754,8 +754,24 @@ __device__ __forceinline__ void winner_setup(const View& V, const Winner& N, Set
 
 // The running edge values at pixel (x, y): row start, then column by column
 // from the bounding-box edge (src/Renderer.cpp:240-243).
+// Long replays, of triangles as wide as the frame, are bound by issue: LONG
+// takes 32 sums a turn of the loop (20 such triangles at 16384x16384: resolve
+// 134.9 ms with 8 a turn, 116.8 with 32; 16 at 1920x1080 147 and 135 us).  The
+// batch kernel, whose warps wait for instructions as it is, does without (256
+// scenes 2208 us, 2218 with it).
+template <bool LONG>
 __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, float& e2) {
-  unpack2(advance2(row_start2(S, y), pack2(S.n1.x, S.n2.x), x - S.x0), e1, e2);
+  const unsigned long long d = pack2(S.n1.x, S.n2.x);
+  unsigned long long e = row_start2(S, y);
+  int n = x - S.x0;
+  if (LONG) {
+#pragma unroll 1
+    for (; n >= 32; n -= 32) {
+#pragma unroll
+      for (int k = 0; k < 32; k++) e = add2(e, d);
+    }
+  }
+  unpack2(advance2(e, d, n), e1, e2);
 }
 
 // savePPM conversion, src/io.cpp:358-362.
@@ -1261,7 +1277,7 @@ __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_res
     Setup S;
     winner_setup(F.v, N, S);
     float e1, e2, k0, k1, k2;
-    replay(S, x, y, e1, e2);
+    replay<true>(S, x, y, e1, e2);
     depth = frag_depth(S, F.v.persp != 0, e1, e2, k0, k1, k2);
     shade(F.v, R, N.v, k0, k1, k2, value, normal);
   }
@@ -1629,7 +1645,7 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
         Setup S;
         winner_setup(C.v, N, S);
         float e1, e2;
-        replay(S, x, y, e1, e2);
+        replay<false>(S, x, y, e1, e2);
         float k0, k1, k2;
         depth = frag_depth(S, persp, e1, e2, k0, k1, k2);
         shade(C.v, R, N.v, k0, k1, k2, value, normal);
