@@ -73,7 +73,9 @@ __device__ __forceinline__ int find_base(const uint32_t* base, int lo, int hi, u
 // find_base for the warp's consecutive g (lane 0 holds the smallest; every
 // lane calls): 32 candidates a round find lane 0's entry -- three dependent
 // loads for 16384 renderables instead of fourteen -- and the other lanes step
-// on from there.  n entries; base[n] is the end.
+// on from there: over 31 renderables with triangles at most, but over any
+// number of empty ones, so a longer way is searched again.  n entries; base[n]
+// is the end.
 __device__ __forceinline__ int find_base_warp(const uint32_t* base, int n, uint32_t g) {
   const int lane = (int)(threadIdx.x & 31);
   const uint32_t g0 = __shfl_sync(0xffffffffu, g, 0);
@@ -85,7 +87,8 @@ __device__ __forceinline__ int find_base_warp(const uint32_t* base, int n, uint3
     lo += at;
     m = min(step, m - at);
   }
-  while (lo + 1 < n && base[lo + 1] <= g) lo++;
+  for (int last = lo + 32; lo + 1 < n && base[lo + 1] <= g; lo++)
+    if (lo == last) return find_base(base, lo, n, g);
   return lo;
 }
 

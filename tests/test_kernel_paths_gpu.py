@@ -315,3 +315,36 @@ def test_frames_of_the_largest_sides(product_lib, w, h, shared, meshes):
             _same(br.read(k), ref, f"batch scene {k}")
     finally:
         br.close()
+
+
+@pytest.mark.parametrize("shared", [False, True], ids=["soup", "shared"])
+@pytest.mark.parametrize("hollow", [False, True], ids=["empty", "vertices_only"])
+def test_runs_of_empty_renderables(product_lib, shared, hollow):
+    """Renderables without triangles (with and without vertices) between others
+    of 1 to 40: the search for a triangle's or vertex's renderable steps over
+    32 of them and searches past more."""
+    rng = np.random.default_rng(9 + shared)
+    nothing = np.zeros((5 if hollow else 0, 3), np.float32)
+    sc = S.Scene()
+    for run in (0, 1, 30, 31, 32, 33, 64, 500, 0, 0, 2):
+        for _ in range(run):
+            sc.add(S.TriMesh(nothing, nothing, np.zeros(0, np.int32), material=S.Material()))
+        for n in (1, 2, 40, 1):
+            c = np.concatenate([rng.uniform(-70, 60, (n, 1, 2)), -rng.uniform(2, 50, (n, 1, 1))], 2)
+            v = (c + [[0, 0, 0], [9, 1, 0], [3, 8, 0]]).astype(np.float32).reshape(-1, 3)
+            idx = np.arange(3 * n, dtype=np.int32)
+            idx = np.concatenate([idx] * (3 if shared else 1))
+            nrm = rng.normal(size=(3 * n, 3)).astype(np.float32)
+            sc.add(S.TriMesh(v, nrm, idx, normalsI=idx, material=S.Material(diffuse=rng.uniform(0.2, 1, 3))))
+    st = FrameState(width=160, height=120, projection=pj.projection_ortho(-80, 80, -60, 60, 1, 60),
+                    light=np.array([0.3, 0.4, 1], np.float32))
+    ref = O.render(st, sc)
+    _same(_render(st, sc), ref, "frame")
+    from minirender_gb300.batch import BatchRenderer
+    br = BatchRenderer(0)
+    try:
+        br.render([(st, sc), (st, sc)])
+        for k in range(2):
+            _same(br.read(k), ref, f"batch scene {k}")
+    finally:
+        br.close()
