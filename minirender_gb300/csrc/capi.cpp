@@ -547,7 +547,7 @@ MR_API int mr_texture_free(mr_ctx* c, int32_t h) {
   return texture_destroy(c, h, nullptr);
 }
 
-static int settle(mr_ctx* c);
+static int settle(mr_ctx* c, const ReadTargets* r = nullptr);
 
 // Launches the kernels of c->last after resetting the per-frame counters.
 static int launch_last(mr_ctx* c) {
@@ -754,21 +754,10 @@ static int queue_reads(mr_ctx* c, const ReadTargets& r) {
 // rasterises the rest through the spill list.
 constexpr size_t kMaxItems = (size_t)1 << 26;
 
-// Waits for the last frame and reads its counters.  An outstanding
-// mr_read_async completes here: its counter copy was queued behind the frame
-// and its output copies before the read_done event (work queued on the
-// stream after them, such as the next frame's mesh upload, is not waited
-// for).  A frame whose blocks overflowed the list was still rasterised
-// completely (through the spill list); the list grows for the next frames.
-static int settle(mr_ctx* c) {
-  if (!c->have_frame) return fail(c, MR_E_INVALID, "no frame rendered yet");
-  if (c->async_read) {
-    CK(cudaEventSynchronize(c->read_done), "read wait");
-    c->async_read = false;
-  } else {
-    CK(cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "counter read");
-    CK(cudaStreamSynchronize(c->stream), "frame wait");
-  }
+// What the last frame's counters, which have been read, tell.  A frame whose
+// blocks overflowed the list was still rasterised completely (through the
+// spill list); the list grows for the next frames.
+static int frame_counters(mr_ctx* c) {
   c->pending = false;
   const Counters& k = *c->h_cnt;
   unsigned long long most = 0;  // of any share
@@ -778,6 +767,28 @@ static int settle(mr_ctx* c) {
     CK(c->items.ensure(want), "block list");
   }
   return (k.error_flags & 1u) ? fail(c, MR_E_BAD_INDEX, "a mesh index was out of range; those triangles were skipped") : MR_OK;
+}
+
+// Waits for the last frame and reads its counters, and with it the outputs
+// asked for.  An outstanding mr_read_async completes here: its counter copy
+// was queued behind the frame and its output copies before the read_done event
+// (work queued on the stream after them, such as the next frame's mesh upload,
+// is not waited for).
+static int settle(mr_ctx* c, const ReadTargets* r) {
+  if (!c->have_frame) return fail(c, MR_E_INVALID, "no frame rendered yet");
+  if (c->async_read) {
+    CK(cudaEventSynchronize(c->read_done), "read wait");
+    c->async_read = false;
+    if (!r) return frame_counters(c);
+  } else {
+    CK(cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream), "counter read");
+  }
+  if (r) {
+    int q = queue_reads(c, *r);
+    if (q) return q;
+  }
+  CK(cudaStreamSynchronize(c->stream), "frame wait");
+  return frame_counters(c);
 }
 
 static int check_reads(mr_ctx* c, const ReadTargets& r) {
@@ -797,12 +808,7 @@ MR_API int mr_read(mr_ctx* c, uint8_t* rgb8, float* depth, float* rgb_f32, uint3
   const ReadTargets r{rgb8, depth, rgb_f32, tri_id, normals};
   int rc = check_reads(c, r);
   if (rc) return rc;
-  rc = settle(c);
-  if (rc && rc != MR_E_BAD_INDEX) return rc;
-  int q = queue_reads(c, r);
-  if (q) return q;
-  CK(cudaStreamSynchronize(c->stream), "read wait");
-  return rc;
+  return settle(c, &r);
 }
 
 MR_API int mr_read_async(mr_ctx* c, uint8_t* rgb8, float* depth, float* rgb_f32, uint32_t* tri_id, float* normals) {
