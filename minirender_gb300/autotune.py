@@ -1,12 +1,11 @@
 """Autotuner for the batched launch: picks the screen-tile shape (width x
-height), the threads per tile block and the number of records staged per
-shared-memory pass of the persistent fused kernel by timing every candidate
-on the caller's own batch (device time of the vertex, setup and fused
-stages, CUDA-graph replay), then, for the best of those, the bounding-box
-size up to which triangles are rasterised by the setup kernel instead of
-being binned; and caches the winner in a JSON file keyed by GPU name and a
-coarse class of the batch (scene count, triangle count and pixel count, each
-bucketed by powers of two).
+height) and the threads per block of the persistent fused kernel by timing
+every candidate on the caller's own batch (device time of the vertex, setup
+and fused stages, CUDA-graph replay), then, for the best of those, the
+bounding-box size up to which triangles are rasterised by the setup kernel
+instead of being binned; and caches the winner in a JSON file keyed by GPU
+name and a coarse class of the batch (scene count, triangle count and pixel
+count, each bucketed by powers of two).
 
 Every candidate produces the same pixels; only the work split changes."""
 from __future__ import annotations
@@ -21,9 +20,8 @@ from . import capi
 # (tile width, tile height): square tiles plus wide ones, which shorten the
 # per-row edge replay of triangles crossing several tiles.
 SHAPES: List[Tuple[int, int]] = [(8, 8), (16, 16), (32, 16), (32, 32), (64, 16), (128, 8), (64, 32), (64, 64)]
-CANDIDATES: List[Tuple[int, int, int, int]] = [(tw, th, t, ch) for tw, th in SHAPES for t in (64, 128, 256)
-                                               for ch in (32, 64, 128)]
-
+# (tile width, tile height, threads, chunk); no kernel reads chunk, so one value is timed
+CANDIDATES: List[Tuple[int, int, int, int]] = [(tw, th, t, 64) for tw, th in SHAPES for t in (64, 128, 256)]
 
 # bounding-box pixels up to which the setup kernel rasterises (0: bin all)
 SMALL_MAX: List[int] = [0, 16, 64, 256]

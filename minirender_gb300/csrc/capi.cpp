@@ -940,7 +940,6 @@ MR_API int mr_set_batch_tiling(mr_ctx* c, int tile_w, int tile_h, int threads, i
   c->b.tile_w = tile_w;
   c->b.tile_h = tile_h;
   c->b.threads = threads;
-  c->b.chunk = chunk;
   return MR_OK;
 }
 
@@ -991,7 +990,7 @@ static int enqueue_batch(mr_ctx* c, BatchSlot& B, cudaStream_t st, cudaEvent_t* 
 // the whole batch and (outside graphs) ev[0..3] its stages.
 static int batch_launch(mr_ctx* c, BatchSlot& B, cudaStream_t st, bool profiling, cudaEvent_t* ev) {
   std::vector<uint64_t> key = {(uint64_t)B.n_scenes, (uint64_t)B.n_rs, B.P.g.n_tris, B.P.g.n_verts, B.P.g.n_nrms,
-                               (uint64_t)B.tile_w, (uint64_t)B.tile_h, (uint64_t)B.threads, (uint64_t)B.chunk,
+                               (uint64_t)B.tile_w, (uint64_t)B.tile_h, (uint64_t)B.threads,
                                (uint64_t)B.grid, (uint64_t)B.P.small_max, (uint64_t)(uintptr_t)B.P.vis,
                                (uint64_t)profiling, (uint64_t)(uintptr_t)st,
                                (uint64_t)(uintptr_t)B.h_rs, (uint64_t)(uintptr_t)B.h_u32,

@@ -117,7 +117,7 @@ using namespace mrgi;
 // and (optionally) the CUDA graph of its launch sequence.  The context owns
 // one for mr_render_batch; a render server owns several.
 struct BatchSlot {
-  int tile_w = 16, tile_h = 16, threads = 256, chunk = 64;
+  int tile_w = 16, tile_h = 16, threads = 256;
   int small_max = 64;  // bbox pixels up to which the setup kernel rasterises (0: every triangle binned)
   bool graphs = true;
   size_t pass_limit = SIZE_MAX;  // bytes the vertex pass may take (more: the kernels transform corners themselves)

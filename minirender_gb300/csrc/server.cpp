@@ -483,7 +483,6 @@ MR_API int mr_server_create(mr_ctx* c, const mr_server_opts* o, mr_server** out)
     sl->b.tile_w = tw;
     sl->b.tile_h = th;
     sl->b.threads = threads;
-    sl->b.chunk = chunk;
     sl->b.small_max = small_max;
     sl->b.graphs = false;  // shapes change from batch to batch
     if (cudaStreamCreateWithFlags(&sl->stream, cudaStreamNonBlocking) != cudaSuccess) {

@@ -17,8 +17,8 @@ from .scene import Material, TriMesh
 class RenderServer:
     def __init__(self, ctx: capi.Context, budget_bytes: int = 40 << 30, slots: int = 2, max_batch: int = 32,
                  tile: int = 16, threads: int = 64, chunk: int = 64, tile_h: int = 0, small_max: int = -1):
-        """tile x tile_h screen tiles (tile_h 0: square), threads per tile
-        block and records per shared-memory pass of the fused batch kernel;
+        """tile x tile_h screen tiles (tile_h 0: square) and threads per block
+        of the fused batch kernel (chunk is checked and read by nothing);
         small_max: bbox pixels up to which the setup kernel rasterises
         (negative: the library default)."""
         self.ctx = ctx

@@ -99,3 +99,8 @@ def test_batch_class_buckets():
     b = A.batch_class(300, 9_000_000, 256 * 640 * 480)
     c = A.batch_class(8, 8_850_000, 256 * 640 * 480)
     assert a == b and a != c
+
+
+def test_candidates_differ_in_what_kernels_read():
+    """No candidate repeats another: chunk, which no kernel reads, is not timed."""
+    assert len({c[:3] for c in A.CANDIDATES}) == len(A.CANDIDATES)
