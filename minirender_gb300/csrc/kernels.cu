@@ -392,21 +392,19 @@ __device__ __forceinline__ unsigned long long advance2(unsigned long long e, uns
   return e;
 }
 
-// Walks columns xs..xe of row y (replaying the running sums from x0) and
-// calls emit(x, packed, e1, e2) for every fragment that would pass z < 1e11f
-// (e1, e2: the running edge values at column x).
+// Walks row y from the bounding-box edge S.x0 to column xe and calls
+// emit(x, packed) for every fragment that would pass z < 1e11f.
 template <typename Emit>
-__device__ __forceinline__ void walk_row(const Setup& S, bool persp, uint32_t id, int y, int xs,
-                                         int xe, Emit emit) {
-  float e1, e2;
+__device__ __forceinline__ void walk_row(const Setup& S, bool persp, uint32_t id, int y, int xe, Emit emit) {
   const unsigned long long d = pack2(S.n1.x, S.n2.x);
-  unsigned long long e = advance2(row_start2(S, y), d, xs - S.x0);
-  for (int x = xs; x <= xe; x++) {
+  unsigned long long e = row_start2(S, y);
+  for (int x = S.x0; x <= xe; x++) {
+    float e1, e2;
     unpack2(e, e1, e2);
     if (covered(e1, e2)) {
       float k0, k1, k2;
-      float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
-      if (z < 1e11f) emit(x, ((unsigned long long)depth_key(z) << 32) | id, e1, e2);
+      const float z = frag_depth(S, persp, e1, e2, k0, k1, k2);
+      if (z < 1e11f) emit(x, ((unsigned long long)depth_key(z) << 32) | id);
     }
     e = add2(e, d);
   }
@@ -1051,8 +1049,8 @@ __device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t i
     if (i < total) {
       const int y = (int)(at >> 16) + k;
       unsigned long long* row = T.row(tg, y);
-      walk_row(U, T.perspective(tg), id + 2u * (uint32_t)(own - (int)lane), y, U.x0, U.x1,
-               [&](int x, unsigned long long v, float, float) { atomicMin(row + x, v); });
+      walk_row(U, T.perspective(tg), id + 2u * (uint32_t)(own - (int)lane), y, U.x1,
+               [&](int x, unsigned long long v) { atomicMin(row + x, v); });
     }
   }
 }
