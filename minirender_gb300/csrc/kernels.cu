@@ -756,10 +756,12 @@ __device__ __forceinline__ void winner_setup(const View& V, const Winner& N, Set
 // The running edge values at pixel (x, y): row start, then column by column
 // from the bounding-box edge (src/Renderer.cpp:240-243).
 // Long replays, of triangles as wide as the frame, are bound by issue: LONG
-// takes 32 sums a turn of the loop (20 such triangles at 16384x16384: resolve
-// 134.9 ms with 8 a turn, 116.8 with 32; 16 at 1920x1080 147 and 135 us).  The
-// batch kernel, whose warps wait for instructions as it is, does without (256
-// scenes 2208 us, 2218 with it).
+// takes 16 sums a turn of the loop, advance2 takes 8 (20 such triangles at
+// 16384x16384 resolve in 122.7 ms, 134.8 with 8, 116.8 with 32; but with 32 a
+// warp whose pixels lie on either side of a multiple takes both ways: 20,000
+// of 38x22 pixels at 1920x1080 57.2 us, 55.2 with 16 and with 8).  The batch
+// kernel, whose warps wait for instructions as it is, does without (256 scenes
+// 2208 us, 2218 with 32).
 template <bool LONG>
 __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, float& e2) {
   const unsigned long long d = pack2(S.n1.x, S.n2.x);
@@ -767,10 +769,15 @@ __device__ __forceinline__ void replay(const Setup& S, int x, int y, float& e1, 
   int n = x - S.x0;
   if (LONG) {
 #pragma unroll 1
-    for (; n >= 32; n -= 32) {
+    for (; n >= 16; n -= 16) {
 #pragma unroll
-      for (int k = 0; k < 32; k++) e = add2(e, d);
+      for (int k = 0; k < 16; k++) e = add2(e, d);
     }
+    if (n & 8) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) e = add2(e, d);
+    }
+    n &= 7;
   }
   unpack2(advance2(e, d, n), e1, e2);
 }
