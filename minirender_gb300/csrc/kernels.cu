@@ -1181,7 +1181,7 @@ __device__ __forceinline__ void raster_block(const FrameParams& F, bool persp, u
   // frame, whose segments are of 4096 columns, 20.7 ms, 6.2 so.)
   const unsigned longest = __reduce_max_sync(0xffffffffu, (unsigned)len);
   const unsigned pieces = __reduce_add_sync(0xffffffffu, (unsigned)(len + kPiece - 1) / kPiece);
-  if ((pieces + 31) / 32 * (104 + longest) < 40 * longest) {
+  if ((pieces + 31) / 32 * (104 + max(longest, 16u)) < 40 * longest) {
     raster_runs(S, persp, id, e, len, at, put);
   } else {
     const unsigned long long d = pack2(S.n1.x, S.n2.x);
