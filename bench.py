@@ -820,7 +820,9 @@ def gpu_arm(args, ws, rank, local):
     # (3T >= 2V); otherwise the setup reads and transforms corners itself
     vertex_pass = 3 * T >= 2 * V
     alg = {
-        "clear+vertex": 8 * P + (12 * V + 24 * V + 16 * V if vertex_pass else 0),
+        # a position in and (x, y, z term, view z, view x, view y, normal,
+        # texcoord) out per vertex, with the normal and texcoord it copies
+        "clear+vertex": 8 * P + (12 * V + 20 * V + 48 * V if vertex_pass else 0),
         "setup": 12 * T + 12 * V + 64 * n_big,
         # blocks (8 B each) and their records; the vis words it updates
         # are the clear's, resident in L2

@@ -549,11 +549,11 @@ MR_API int mr_texture_free(mr_ctx* c, int32_t h) {
 
 static int settle(mr_ctx* c, const ReadTargets* r = nullptr);
 
-// Launches the kernels of c->last after resetting the per-frame counters.
+// Launches the kernels of c->last.
 static int launch_last(mr_ctx* c) {
   FrameParams& F = c->last;
   cudaStream_t st = c->stream;
-  // (the clear kernel also zeroes the counters and the tile tables)
+  // (the first kernel also zeroes the counters)
   CK(launch_frame(F, st, c->profiling ? c->ev : nullptr, c->staged), "frame launch");
   return MR_OK;
 }

@@ -20,17 +20,16 @@
 //                  barycentrics exactly, shades once per visible pixel and
 //                  writes RGB8/depth/ids            (src/Renderer.cpp:271-305, src/io.cpp:358-362)
 // Many frames per call (launch_batch):
-//   k_vertex (when vertices are shared), a clear of the batch's visibility
-//   words (when small triangles are rasterised in the setup), then
-//   k_setup_batch (sub-triangles with a bounding box of at most small_max
-//   pixels rasterised into their scene's visibility words, larger ones
+//   k_vertex (when vertices are shared), then k_setup_batch (sub-triangles
+//   with a bounding box of at most small_max pixels rasterised into their
+//   scene's visibility words, which the batch before left empty, larger ones
 //   become records counted into the scene's tiles), then k_batch: one
 //   cooperative, persistent launch -- list ranges, scatter, and a dynamically
 //   scheduled loop over strips of all tiles of all scenes, one warp each, that
 //   rasterises the tile's records into shared memory (seeded with the small
-//   triangles' words) and resolves + shades the strip's pixels in place.  The
-//   PRE template flag is false for triangle soups: no vertex pass, kernels
-//   transform corners themselves.
+//   triangles' words, which it empties) and resolves + shades the strip's
+//   pixels in place.  The PRE template flag is false for triangle soups: no
+//   vertex pass, kernels transform corners themselves.
 // Also: k_validate (index checks at upload), k_range (getRangeImage,
 // src/Renderer.cpp:388-415).
 //
@@ -455,9 +454,9 @@ __device__ __forceinline__ int row_run(const Setup& S, int y, int& xs, int xe, u
 // values e0, its first pixel at `at`), cut into pieces of kPiece columns and
 // dealt one per lane: depth and put(pixel, word) of every fragment that passes
 // z < 1e11f (src/Renderer.cpp:243-269).  A lane that walked its own row to the
-// end waited for the warp's longest: 256 scenes' fused stage 2266 us so, 1975
-// with pieces of 4, 1955 with 2, 2014 with 1, 2018 with 8.  Called by all
-// lanes of the warp.
+// end would wait for the warp's longest.  256 scenes' fused stage 1826 us with
+// pieces of 2, 1879 with 1, 1855 with 4, 2104 with 8.  Called by all lanes of
+// the warp.
 constexpr int kPiece = 2;
 template <typename Cell, typename Put>
 __device__ __forceinline__ void raster_runs(const Setup& S, bool persp, uint32_t id, unsigned long long e0, int len,
@@ -930,10 +929,10 @@ __global__ void __launch_bounds__(256) k_vertex(Geo G, View V, const SceneRec* s
 }
 
 // Threads per block of the setup kernels.  Their warps share nothing
-// (statistics go to slots, records are reserved by a warp at a time), and a block keeps its place until its slowest warp is done:
-// 1080p mesh setup 48.8 us with 256 threads, 46.6 with 128, 44.6 with 64; 10M-
-// triangle soup 378, 368, 366 us; 256 scenes 387 us with 128 threads and
-// records reserved by the block, 379 so.
+// (statistics go to slots, records are reserved by a warp at a time), and a
+// block keeps its place until its slowest warp is done: 1080p mesh setup 38.6
+// us with 64 threads, 40.6 with 128, 42.6 with 256; 10M-triangle soup 323, 325
+// and 338; 256 scenes 334, 340 and 371.
 constexpr int kSetupThreads = 64;
 
 // Where small triangles' fragments go: the frame's visibility buffer...
@@ -963,10 +962,9 @@ struct BatchTarget {
 // LIST: the covered cells first (bit 4 * row + column), then one covered pixel
 // per turn of a loop, whose depth and atomic a warp issues as often as its
 // fullest lane has pixels (5-6 for triangles of 1-4 square pixels) instead of
-// once for each of the 16 cells that any lane covers: 10M-triangle soup setup
-// 348 -> 329 us, 16 soups 100 -> 92 us.  The vertex-pass kernels take the
-// plain walk: the list's registers are spilled there (1080p mesh 46.7 ->
-// 50.8 us).
+// once for each of the 16 cells that any lane covers: 5 % less of a
+// 10M-triangle soup's setup, 8 % of 16 soups'.  The vertex-pass kernels take
+// the plain walk: the list's registers are spilled there (1080p mesh 9 % more).
 template <bool LIST, typename RowFn>
 __device__ __forceinline__ void raster_tiny(const Setup& Q, bool persp, uint32_t id, RowFn row_of) {
   const unsigned long long d = pack2(Q.n1.x, Q.n2.x);
@@ -1013,8 +1011,8 @@ __device__ __forceinline__ void raster_tiny(const Setup& Q, bool persp, uint32_t
 // most 4x4 pixels the lanes rasterise their own (LIST: see raster_tiny);
 // otherwise their rows are numbered by a prefix sum and taken one per lane,
 // each lane fetching its row's setup from the lane that holds it.  (Staged in
-// shared memory, the setups cost the vertex gathers 4 KB of L1 a block: 1080p
-// mesh 42.5 us, 40.1 so; 256 scenes 375 and 366.)  Called by all lanes.
+// shared memory, the setups cost the vertex gathers 4 KB of L1 a block: 6 %
+// more of the 1080p mesh's setup.)  Called by all lanes.
 template <bool LIST, class Target>
 __device__ __forceinline__ void raster_small(const Setup& S, bool on, uint32_t id, uint32_t tag, const Target& T) {
   const unsigned lane = threadIdx.x & 31;
@@ -1246,13 +1244,13 @@ __global__ void __launch_bounds__(256) k_raster_large(FrameParams F) {
 
 // Deferred resolve + shade: one thread per pixel, 128-thread blocks over
 // 32x4-pixel tiles (a block keeps its registers until its slowest warp is
-// done: 1080p mesh 40.9 us with 256 threads, 36.9 with 128, 38.9 with 64; 4K
-// soup 235, 225, 229).  Bound by its chain of gathers -- word, triangle,
-// corners, texel -- where neighbouring pixels' triangles lie apart (1080p mesh
-// of 1.31M triangles: 53 % of issue slots used, 36.8 us; 52 with attributes in
-// six arrays and a search for the renderable), by instruction issue where
-// corner records shorten it (10M-triangle soup: 72 %, 219 us; 282).  More
-// blocks per SM spill.
+// done: 1080p mesh 36.8 us, 38.9 with 64 threads and with 256; 4K soup 219, 221
+// and 227).  Bound by its chain of gathers -- word, triangle, corners, texel --
+// where neighbouring pixels' triangles lie apart (1080p mesh of 1.31M
+// triangles: 53 % of issue slots used, 36.8 us; 52 with attributes in six
+// arrays and a search for the renderable), by instruction issue where corner
+// records shorten it (10M-triangle soup: 72 %, 219 us; 282).  More blocks per
+// SM spill.
 constexpr int kResolveTileW = 32, kResolveTileH = 4, kResolveThreads = kResolveTileW * kResolveTileH;
 template <bool PRE, bool ONE>
 __global__ void __launch_bounds__(kResolveThreads, 1024 / kResolveThreads) k_resolve(FrameParams F) {
@@ -1341,11 +1339,11 @@ __device__ __forceinline__ void each_tile(uint32_t first, uint32_t pitch, uint32
   }
 }
 
-// Setup of every triangle of every scene: each sub-triangle with pixels to
-// test becomes a record (warp-compacted), counted into its scene's tiles.
-// Bound by dependent loads (renderable, indices, vertices, view): 49 % of issue
-// slots used; 256 scenes 340 us.  (Blocks of 128 and 256 threads cost 1 % and
-// 8 % more, 40 and 64 registers 2 % and 10 %.)
+// Setup of every triangle of every scene: sub-triangles of at most small_max
+// pixels of bounding box are rasterised into their scene's words, the others
+// become records (warp-compacted), counted into their scene's tiles.  Bound by
+// dependent loads (renderable, indices, vertices, view): 49 % of issue slots
+// used; 256 scenes 334 us.
 template <bool PRE>
 __global__ void __launch_bounds__(kSetupThreads, kSetupMinBlocks<PRE> * 256 / kSetupThreads) k_setup_batch(BatchParams B) {
   const unsigned lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
@@ -1470,16 +1468,12 @@ __device__ __forceinline__ void raster_strip(const BatchParams& B, uint32_t s, u
 //   memory, then every pixel is resolved, shaded and written to its scene's
 //   outputs.
 // A strip is one warp's alone and each warp takes its own from a work counter,
-// so no warp waits for another once the lists stand.  With a block per tile,
-// barriers between the phases were 38 % of the warps' time (256 scenes 2934 us,
-// 16 soups 260, eight 3840x2160 scenes in 16x16 tiles 5037); with strips handed
-// to a block two a warp at a time, the barrier around the hand-over was still
-// a fifth (1945, 207); now 1807 and 198, and 24 scenes of 256x256 74 -> 65.
-// (Groups a block's warps share and refill without a barrier: 1830 and 211.)
-// (The old form also captured the winners' edge values where a replay could
-// pass 256 columns; with packed adds the replay is the cheaper.)
-// 64 registers: with 80 the 256 scenes take 2565 us (2270) and 16 soups 221
-// (205), with up to 128, which blocks of 64 threads had, the soups 252.
+// so no warp waits for another once the lists stand (with a block per tile the
+// barriers between the phases were 38 % of the warps' time, with strips handed
+// to a block in groups a fifth).  256 scenes 1826 us at 71 % of issue slots, 16
+// soups 197, 24 scenes of 256x256 54.
+// 64 registers: with 80, three blocks of 256 threads an SM, the 256 scenes take
+// 2068 us and the soups 199.
 template <bool PRE>
 __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1533,9 +1527,9 @@ __global__ void __launch_bounds__(256, 4) k_batch(BatchParams B) {
   grid.sync();
   // 3. strips.  A fetch is one strip, or as many as make half of strip_px where
   // tiles are smaller (the counter takes one atomic at a time: 64 scenes of
-  // 512x512 in 4x16 tiles 1381 us with groups of four for two warps, 1399 with
-  // all of strip_px, 1364 so).  A warp's place is kept in shared memory: in
-  // registers it spills what the shading needs (256 scenes 1832 us, 1807).
+  // 512x512 in 4x16 tiles 2.5 % more with all of strip_px).  A warp's place is
+  // kept in shared memory: in registers it spills what the shading needs (256
+  // scenes 1.4 % more).
   const int ls2 = __ffs(TH / SH) - 1;  // strips per tile, a power of two
   const uint32_t run = max(1u, (uint32_t)B.strip_px / (uint32_t)(2 * TW * SH));  // strips per fetch, likewise
   if (lane == 0) s_at[w] = ~0ull;
